@@ -75,11 +75,12 @@ struct LaunchConfig {
     int track;             /* 1: some view's image asks for contributor counts or last-visited
                               offsets (the compositor then keeps them); set by the host */
 };
-/* measured on B200 at 1080p with 1 M Gaussians: 512-instance compositor
- * chunks (0.233 against 0.238 ms for 256, 0.259 for 128); 4096-key tiles
+/* measured on B200 at 1080p with 1 M Gaussians: 256-instance compositor
+ * chunks (0.156 against 0.157 ms for 128 and 0.175 for 512, which stages more
+ * instances behind the pixels' last splat); 4096-key tiles
  * for both sorts (sort stage 0.1955 ms, against 0.1978 with 2048-key depth
  * tiles, 0.2002 with 6144-key and 0.2232 with 2048-key tile-sort tiles) */
-constexpr LaunchConfig kDefaultLaunch = {512, 16, 16, 1};
+constexpr LaunchConfig kDefaultLaunch = {256, 16, 16, 1};
 
 __host__ __device__ constexpr inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -234,6 +235,22 @@ __device__ __forceinline__ int find_view_by_tile(const ViewTable* vt, int n_view
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (vt->view[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+/* find_view_by_tile by a whole warp: 32 views per step instead of one (a
+ * binary search is a chain of dependent loads). */
+__device__ __forceinline__ int find_view_by_tile_warp(const ViewTable* vt, int n_views, long long tile) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0;   /* the view is in [lo, lo + n) */
+    for (int n = n_views; n > 1;) {
+        const int step = (n + 31) / 32;
+        const int v = lo + lane * step;
+        const bool before = lane * step < n && vt->view[v].tile_begin <= tile;
+        const int k = 31 - __clz(__ballot_sync(0xffffffffu, before) | 1u);   /* the last such lane: begins ascend */
+        lo += k * step;
+        n = n - k * step < step ? n - k * step : step;
     }
     return lo;
 }
