@@ -518,6 +518,7 @@ __device__ __forceinline__ LumenRayHit cast_ray(const CastArgs& A, const CastLev
         best.distance = (float)1e9;
         return best;
     }
+    in_order = in_order || A.root != A.node_count - 1;   /* a cast from another node follows the links */
     RayState r;
     float ainv[3], far = 0.0f;
 #pragma unroll
