@@ -41,6 +41,7 @@ class _RenderFunction(torch.autograd.Function):
         ctx.save_for_backward(tensors[0], tensors[1], tensors[2], tensors[3].reshape(n), sh_flat, res.rgb, res.depth,
                               res.alpha, res.last_idx)
         ctx.mark_non_differentiable(res.last_idx)
+        ctx.set_materialize_grads(False)   # an output without a gradient passes None, not zeros to read
         return res.rgb, res.depth, res.alpha
 
     @staticmethod
