@@ -440,7 +440,7 @@ composite_backward_kernel(const LumenSplatRecord* __restrict__ records, LumenGpu
         return;
     }
     const unsigned int n_visible = ctrl->n_visible;
-    const unsigned int* __restrict__ vals = ctrl->tile_sort.sorted_buffer ? f.vals[1] : f.vals[0];
+    const unsigned int* __restrict__ vals = ctrl->list_buffer ? f.vals[1] : f.vals[0];
     const float tile_x0 = (float)(tx * kTile), tile_y0 = (float)(ty * kTile);
 
     if (tid == 0) {

@@ -330,7 +330,7 @@ __device__ __forceinline__ void composite_tile(CompositeSmem<kChunk>& s, const V
     int rs = f.ranges[2 * gtile], re = f.ranges[2 * gtile + 1];
     const long long n_instances = (long long)ctrl->n_instances;
     const unsigned int n_visible = ctrl->n_visible;
-    const unsigned int* __restrict__ vals = ctrl->tile_sort.sorted_buffer ? f.vals[1] : f.vals[0];
+    const unsigned int* __restrict__ vals = ctrl->list_buffer ? f.vals[1] : f.vals[0];
     const long long K = n_instances < capacity ? n_instances : capacity;
     bool listed = rs != -1 && rs < re;
     if (listed && (rs < 0 || (long long)re > K)) {

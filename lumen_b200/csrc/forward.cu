@@ -10,13 +10,12 @@
  *   batch_project      K1c: projection, cull, SH, records and depth keys at those offsets
  *   histogram<u32>     depth-key digits of the visible splats
  *   onesweep_pass x4   stable sort of visible splats by depth key
- *   emit               K2: (tile id, visible index) per covered tile, in depth order;
- *                      also the tile sort's digit counts, look-back tiles and ranges = -1
- *   onesweep_pass xb   stable sort of instances by tile id (b: the bytes a tile id
- *                      can vary in; with no Gaussians a histogram launch comes first);
- *                      the pass over the highest varying byte writes the tile ranges
- *   tile_ranges        K4: touched tiles and each view's first instance from the
- *                      ranges (the ranges themselves when no tile-id byte varies)
+ *   emit               K2: (cell and tile mask, visible index) per touched cell of 4x4
+ *                      tiles, in depth order; also the cell sort's digit counts and
+ *                      look-back tiles
+ *   onesweep_pass xb   stable sort of the pairs by cell (b: the bytes a cell id can vary in)
+ *   list_count, list_scan, list_write   K4: each cell's list split over its tiles: counts,
+ *                      ranges with touched tiles and each view's first instance, lists
  *   composite          K5
  * Passes whose digit is constant exit at once (decided on the device).
  */
@@ -40,17 +39,17 @@ void launch_project(const ViewTable* vt, int n_views, const LumenRenderOptions& 
 void launch_emit(const ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned long long* lb,
                  unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys, long long n_blocks,
                  bool persistent, int num_sms, cudaStream_t st);
-void launch_tile_sort_counted(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1,
-                              long long capacity, Control* ctrl, ViewTable* vt, int* ranges, unsigned int* lb,
-                              long long lb_tiles_cap, int items, int key_bytes, int num_sms, cudaStream_t st);
 void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1, long long capacity,
-                   SortControl* sc, unsigned int* lb, long long lb_tiles_cap, int* ranges,
-                   const long long* n_range_tiles, unsigned int* err, int items, int key_bytes, int num_sms,
-                   cudaStream_t st);
+                   SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int items,
+                   int key_bytes, int num_sms, cudaStream_t st);
+void launch_cell_sort(const LumenGpuFrame& f, Control* ctrl, const ViewTable* vt, unsigned int* lb,
+                      long long lb_tiles_cap, int items, int key_bytes, int num_sms, cudaStream_t st);
+void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, void* room, long long room_bytes,
+                  long long n_cells, long long n_tiles,
+                  int num_sms, cudaStream_t st);
 void launch_sort64(unsigned long long* k0, unsigned int* v0, unsigned long long* k1, unsigned int* v1,
                    long long capacity, SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err,
                    int num_sms, cudaStream_t st);
-void launch_ranges(const LumenGpuFrame& f, Control* ctrl, ViewTable* vt, int num_sms, cudaStream_t st);
 void launch_key_stats64(const unsigned long long* keys, long long n, SortControl* sc, int num_sms, cudaStream_t st);
 void launch_sorted_keys64(const LumenGpuFrame& f, const Control* ctrl, int key_mode, unsigned long long* out,
                           int num_sms, cudaStream_t st);
@@ -173,8 +172,8 @@ __global__ void frame_init_kernel(unsigned long long* zero, long long n_words, V
     }
 }
 
-/* The frame's kernels after the view table is in place. n_slots and
- * n_tiles are the batch's (plain launches) or upper bounds (persistent
+/* The frame's kernels after the view table is in place. n_slots, n_tiles and
+ * n_cells are the batch's (plain launches) or upper bounds (persistent
  * launches, whose kernels read the batch's sizes from the table); n_views
  * is the batch's view count, or 0 when only the table knows it; n_units
  * the projection units (plain launches). Projection is a visibility count,
@@ -182,15 +181,15 @@ __global__ void frame_init_kernel(unsigned long long* zero, long long n_words, V
  * scene read once); with n_units 0 a single view instead runs the one-pass
  * kernel with its compacting scan fused in (project_kernel). */
 void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRenderOptions& opt,
-                     const LumenGpuFrame& f, long long n_slots, long long n_tiles, int n_views, bool persistent,
-                     const LaunchConfig& lc, cudaEvent_t* ev, cudaStream_t s, bool with_composite,
+                     const LumenGpuFrame& f, long long n_slots, long long n_tiles, long long n_cells, int n_views,
+                     bool persistent, const LaunchConfig& lc, cudaEvent_t* ev, cudaStream_t s, bool with_composite,
                      long long n_units) {
     Control* ctrl = (Control*)(base + L.control_off);
     ViewTable* vt = (ViewTable*)(base + L.table_off);
     unsigned long long* proj_lb = (unsigned long long*)(base + L.proj_lb_off);
     unsigned long long* emit_lb = (unsigned long long*)(base + L.emit_lb_off);
     unsigned int* depth_lb = (unsigned int*)(base + L.depth_lb_off);
-    unsigned int* tile_lb = (unsigned int*)(base + L.tile_lb_off);
+    unsigned int* cell_lb = (unsigned int*)(base + L.tile_lb_off);
     const int sms = device_sm_count();
     if (n_slots > 0) {
         if (n_views == 1 && n_units == 0)
@@ -199,29 +198,21 @@ void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRen
             launch_batch_project(vt, opt, f, ctrl, proj_lb, n_units, L.proj_blocks, persistent, sms, s);
         if (ev) cudaEventRecord(ev[1], s);
         launch_sort32(f.depth_keys[0], f.depth_order[0], f.depth_keys[1], f.depth_order[1], n_slots,
-                      &ctrl->depth_sort, depth_lb, L.depth_tiles, nullptr, nullptr, &ctrl->error_flags,
-                      lc.depth_sort_items, 4, sms, s);
-        launch_emit(vt, f, ctrl, emit_lb, tile_lb, 2 * L.sort_tiles, kSortThreads * lc.tile_sort_items,
+                      &ctrl->depth_sort, depth_lb, L.depth_tiles, &ctrl->error_flags, lc.depth_sort_items, 4, sms,
+                      s);
+        launch_emit(vt, f, ctrl, emit_lb, cell_lb, 2 * L.sort_tiles, kSortThreads * lc.tile_sort_items,
                     L.proj_blocks, persistent, sms, s);
+        /* the cell-sort region holds 4 passes of 2048-key tiles; cell ids
+         * below n_cells (the batch's, or the bound a persistent launch is
+         * sized for) vary in their low ceil(log2(n_cells) / 8) bytes only */
+        int cell_bytes = 0;
+        for (long long t = n_cells - 1; t > 0; t >>= 8) ++cell_bytes;
+        launch_cell_sort(f, ctrl, vt, cell_lb, 2 * L.sort_tiles, lc.tile_sort_items, cell_bytes, sms, s);
     } else if (ev) {
         cudaEventRecord(ev[1], s);
     }
-    /* the tile-sort region holds 4 passes of 2048-key tiles; tile ids below
-     * n_tiles (the batch's, or the bound a persistent launch is sized for)
-     * vary in their low ceil(log2(n_tiles) / 8) bytes only. After an
-     * emission the digit counts, look-back tiles and ranges are ready;
-     * without one (no Gaussians) the sort's histogram kernel does that. */
-    int tile_bytes = 0;
-    for (long long t = n_tiles - 1; t > 0; t >>= 8) ++tile_bytes;
-    if (n_slots > 0)
-        launch_tile_sort_counted(f.keys[0], f.vals[0], f.keys[1], f.vals[1], f.instance_capacity, ctrl, vt,
-                                 f.ranges, tile_lb, 2 * L.sort_tiles, lc.tile_sort_items, tile_bytes, sms, s);
-    else
-        launch_sort32(f.keys[0], f.vals[0], f.keys[1], f.vals[1], f.instance_capacity, &ctrl->tile_sort, tile_lb,
-                      2 * L.sort_tiles, f.ranges, &vt->hdr.total_tiles, &ctrl->error_flags, lc.tile_sort_items,
-                      tile_bytes, sms, s);
     if (ev) cudaEventRecord(ev[2], s);
-    launch_ranges(f, ctrl, vt, sms, s);
+    launch_lists(vt, f, ctrl, cell_lb, (long long)(L.total - L.tile_lb_off), n_cells, n_tiles, sms, s);
     if (ev) cudaEventRecord(ev[3], s);
     if (!with_composite) return;
     launch_composite(vt, n_views, f, ctrl, opt, 0, n_tiles, persistent, lc.composite_chunk, lc.track != 0, sms, s);
@@ -261,6 +252,8 @@ static void single_view_table(const LumenGpuGaussians* g, const LumenViewCamera*
     v->g = *g;
     v->cam = *cam;
     v->tiles_x = (cam->width + kTile - 1) / kTile;
+    v->cells_x = cells_along(v->tiles_x);
+    hdr->total_cells = (long long)v->cells_x * cells_along((cam->height + kTile - 1) / kTile);
     v->img = *img;
     v->inst_begin = -1;
     v->unit_begin = 0;
@@ -288,7 +281,7 @@ static LumenStatus forward_impl(const LumenGpuGaussians* g, const LumenViewCamer
     single_view_table(g, cam, img, L, tiles, &hdr, &v);
     if (ev) cudaEventRecord(ev[0], s);
     launch_init(L, base, &hdr, &v, s);
-    launch_pipeline(L, base, *opt, *f, g->count, tiles, 1, false, lc, ev, s, true, hdr.total_units);
+    launch_pipeline(L, base, *opt, *f, g->count, tiles, hdr.total_cells, 1, false, lc, ev, s, true, hdr.total_units);
     return map_cuda(cudaGetLastError());
 }
 
@@ -314,7 +307,7 @@ LumenStatus forward_banded(const LumenGpuGaussians* g, const LumenViewCamera* ca
     ViewDesc v{};
     single_view_table(g, cam, img, L, tiles, &hdr, &v);
     launch_init(L, base, &hdr, &v, s);
-    launch_pipeline(L, base, *opt, *f, g->count, tiles, 1, false, kDefaultLaunch, nullptr, s, false,
+    launch_pipeline(L, base, *opt, *f, g->count, tiles, hdr.total_cells, 1, false, kDefaultLaunch, nullptr, s, false,
                     hdr.total_units);
     Control* ctrl = (Control*)(base + L.control_off);
     const ViewTable* vt = (const ViewTable*)(base + L.table_off);
@@ -335,7 +328,7 @@ static LumenStatus plan_batch(const LumenGpuBatchView* views, int n_views, const
                               std::vector<ViewDesc>* out, BatchHeader* hdr) {
     if (!views || n_views <= 0 || n_views > kMaxViews) return LUMEN_ERROR_INVALID_ARGUMENT;
     if (opt && check_options(opt) != LUMEN_SUCCESS) return LUMEN_ERROR_INVALID_ARGUMENT;
-    long long blocks = 0, tiles = 0;
+    long long blocks = 0, tiles = 0, cells = 0;
     if (out) out->resize((size_t)n_views);
     for (int v = 0; v < n_views; ++v) {
         const LumenGpuBatchView& bv = views[v];
@@ -343,7 +336,8 @@ static LumenStatus plan_batch(const LumenGpuBatchView* views, int n_views, const
             return LUMEN_ERROR_INVALID_ARGUMENT;
         if (out && !bv.image.rgb && !bv.image.rgb8) return LUMEN_ERROR_INVALID_ARGUMENT;
         const int tiles_x = (bv.camera.width + kTile - 1) / kTile;
-        const long long vt = (long long)tiles_x * ((bv.camera.height + kTile - 1) / kTile);
+        const int tiles_y = (bv.camera.height + kTile - 1) / kTile;
+        const long long vt = (long long)tiles_x * tiles_y;
         if (out) {
             ViewDesc& d = (*out)[(size_t)v];
             std::memset(&d, 0, sizeof(d));
@@ -353,8 +347,11 @@ static LumenStatus plan_batch(const LumenGpuBatchView* views, int n_views, const
             d.img = bv.image;
             d.block_begin = blocks;
             d.tile_begin = tiles;
+            d.cells_x = cells_along(tiles_x);
+            d.cell_begin = cells;
             d.inst_begin = -1;
         }
+        cells += (long long)cells_along(tiles_x) * cells_along(tiles_y);
         blocks += (bv.gaussians.count + kProjThreads - 1) / kProjThreads;
         tiles += vt;
     }
@@ -364,6 +361,7 @@ static LumenStatus plan_batch(const LumenGpuBatchView* views, int n_views, const
     hdr->n_views = n_views;
     hdr->total_blocks = blocks;
     hdr->total_tiles = tiles;
+    hdr->total_cells = cells;
     if (out) hdr->total_units = assign_scene_groups(out->data(), n_views);
     return LUMEN_SUCCESS;
 }
@@ -395,7 +393,8 @@ static LumenStatus batch_impl(const LumenGpuBatchView* views, int n_views, const
     lc.track = 0;
     for (int v = 0; v < n_views; ++v)
         if (views[v].image.n_contrib || views[v].image.last_idx) lc.track = 1;
-    launch_pipeline(L, base, *opt, *f, slots, hdr.total_tiles, n_views, false, lc, ev, s, true, hdr.total_units);
+    launch_pipeline(L, base, *opt, *f, slots, hdr.total_tiles, hdr.total_cells, n_views, false, lc, ev, s, true,
+                    hdr.total_units);
     return map_cuda(cudaGetLastError());
 }
 
@@ -437,17 +436,22 @@ LumenStatus lumen_gpu_render_forward_ex(const LumenGpuGaussians* g, const LumenV
 LumenStatus lumen_gpu_read_counts(const LumenGpuFrame* f, LumenGpuCounts* c, void* stream) {
     if (!f || !c || !f->scratch) return LUMEN_ERROR_INVALID_ARGUMENT;
     cudaStream_t s = (cudaStream_t)stream;
-    Control h;
-    cudaError_t e = cudaMemcpyAsync(&h, f->scratch, sizeof(Control), cudaMemcpyDeviceToHost, s);
+    /* the counters at the start of the control block */
+    struct { alignas(Control) unsigned char bytes[offsetof(Control, proj_ticket)]; } head;
+    cudaError_t e = cudaMemcpyAsync(&head, f->scratch, sizeof(head), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return map_cuda(e);
+    const Control& h = *reinterpret_cast<const Control*>(&head);
     c->n_visible = h.n_visible;
     c->n_instances = (int64_t)h.n_instances;
     c->error_flags = h.error_flags;
-    c->sorted_buffer = h.tile_sort.sorted_buffer;
-    c->varying_digits = (h.tile_sort.varying & 0xFFu) | ((h.depth_sort.varying & 0xFFu) << 8);
+    c->sorted_buffer = h.list_buffer;
+    unsigned int tile_digits = 0;
+    for (int d = 0; d < 4; ++d)
+        if (((h.tile_or & h.tile_or_not) >> (8 * d)) & 0xFFu) tile_digits |= 1u << d;
+    c->varying_digits = tile_digits | ((h.depth_varying & 0xFFu) << 8);
     c->touched_tiles = h.touched_tiles;
-    c->depth_sorted_buffer = h.depth_sort.sorted_buffer;
+    c->depth_sorted_buffer = h.depth_buffer;
     c->reserved = 0;
     return LUMEN_SUCCESS;
 }
@@ -573,16 +577,16 @@ LumenStatus lumen_gpu_sort_pairs(uint64_t* keys0, uint32_t* vals0, uint64_t* key
     const int sms = device_sm_count();
     unsigned long long* k0 = reinterpret_cast<unsigned long long*>(keys0);
     unsigned long long* k1 = reinterpret_cast<unsigned long long*>(keys1);
-    launch_key_stats64(k0, n, &ctrl->tile_sort, sms, s);
+    launch_key_stats64(k0, n, &ctrl->cell_sort, sms, s);
     /* the tile-sort look-back region holds 8 digits x tiles x 256 entries */
-    launch_sort64(k0, vals0, k1, vals1, n, &ctrl->tile_sort, (unsigned int*)(base + L.tile_lb_off), L.sort_tiles,
+    launch_sort64(k0, vals0, k1, vals1, n, &ctrl->cell_sort, (unsigned int*)(base + L.tile_lb_off), L.sort_tiles,
                   &ctrl->error_flags, sms, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return map_cuda(e);
     Control h;
     e = cudaMemcpyAsync(&h, ctrl, sizeof(Control), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return map_cuda(e);
-    *sorted_buffer = h.tile_sort.sorted_buffer;
+    *sorted_buffer = h.cell_sort.sorted_buffer;
     return status_from_flags(h.error_flags);
 }
 

@@ -1,0 +1,399 @@
+/*
+ * lists.cu - the tiles' splat lists from the sorted (cell, splat) pairs.
+ *
+ * Reference: the key sort of rasterize_scene (src/raster/pipeline.mojo:152-166
+ * with radix_sort_64bit, src/raster/radix_sort.mojo:39-87) and
+ * TileRangeIndex.build_from_sorted_keys, src/raster/binning.mojo:51-73: the
+ * instances ordered by (tile, depth key, visible index), and each tile's
+ * first and last position, (-1, -1) where it has none.
+ *
+ * The emission writes one pair per cell (4x4 tiles) that a splat touches, in
+ * depth order, and the cell sort keeps that order within a cell. Here each
+ * cell's list is split over its 16 tiles by the pairs' tile masks, in order:
+ *
+ *   list_count_kernel   per segment of 256 pairs of a cell: the instances of
+ *                       each of its tiles before it
+ *   list_scan_kernel    an exclusive scan of the tiles' counts: the ranges, the
+ *                       touched tiles, each view's first instance
+ *   list_write_kernel   per segment: a vote per tile and 32 pairs gives every
+ *                       instance its position
+ *
+ * Why two levels: sorting the instances themselves by tile ranks every one of
+ * them twice (two digit passes, about 120 instructions per instance and pass)
+ * and moves 8 B per instance five times. A splat covers about 7 tiles but 2
+ * cells, so the ranked pairs are 3 to 4 times fewer, and the split needs no
+ * ranking. The instances are written once. From the depth order to the ranges,
+ * emission included, this took (us, before -> after): 1 M splats at
+ * 1080p 160 -> 130, 2 M at 4K 455 -> 260, 64 views of 300 k at 720p
+ * 2400 -> 1330, 512 splats at 800x600 34 -> 32.
+ */
+#include "splat_common.cuh"
+
+namespace lumen {
+
+namespace {
+
+constexpr int kCountThreads = 256;
+constexpr int kCountWarps = kCountThreads / 32;
+constexpr int kScanThreads = 1024;
+constexpr int kWriteThreads = 128;
+constexpr int kWriteWarps = kWriteThreads / 32;
+constexpr int kWriteCtas = 6;                   /* per SM */
+constexpr int kSegment = 256;                   /* pairs of a cell that a warp counts and writes at a time */
+constexpr int kCellTiles = kCellSide * kCellSide;
+
+/* A cell in its view. */
+struct Cell {
+    int x, y;                /* its first tile */
+    int tiles_x, tiles_y;
+    long long tile_begin;
+    /* batch-wide id of its tile k (bit k of the masks), or -1 beyond the view */
+    __device__ __forceinline__ long long tile(int k) const {
+        const int tx = x + k % kCellSide, ty = y + k / kCellSide;
+        return tx < tiles_x && ty < tiles_y ? tile_begin + (long long)ty * tiles_x + tx : -1;
+    }
+};
+
+__device__ __forceinline__ Cell find_cell(const ViewTable* vt, int n_views, long long cell) {
+    const ViewDesc& vd = vt->view[n_views == 1 ? 0 : find_view_by_cell(vt, n_views, cell)];
+    const int local = (int)(cell - vd.cell_begin);
+    Cell c;
+    c.y = local / vd.cells_x * kCellSide;
+    c.x = local % vd.cells_x * kCellSide;
+    c.tiles_x = vd.tiles_x;
+    c.tiles_y = (vd.cam.height + kTile - 1) / kTile;
+    c.tile_begin = vd.tile_begin;
+    return c;
+}
+
+/* The first of n sorted keys whose cell is `cell` or above, by a whole warp
+ * (32 probes per step). */
+__device__ __forceinline__ int first_of_cell(const unsigned int* __restrict__ keys, int n, unsigned int id_mask,
+                                             unsigned int cell) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, len = n;   /* the answer is in [lo, lo + len] */
+    while (len > 0) {
+        const int step = (len + 31) / 32;
+        const int at = lo + lane * step;
+        const bool below = lane * step < len && (keys[at] & id_mask) < cell;
+        const int k = __popc(__ballot_sync(0xffffffffu, below));   /* the first k probes are below */
+        if (k == 0) return lo;
+        const int end = lo + len;
+        lo += (k - 1) * step + 1;
+        len = min(step - 1, end - lo);
+    }
+    return lo;
+}
+
+/* The tile mask of a sorted pair of the cell whose first tile is (x, y). */
+__device__ __forceinline__ unsigned int pair_mask(bool packed, unsigned int key, unsigned int v,
+                                                  const uint64_t* __restrict__ rects, int x, int y) {
+    return packed ? key >> 16 : cell_mask(rects[v], x, y);
+}
+
+/* Tiles per scan group: at most kTileGroups groups. */
+__device__ __forceinline__ long long tile_group_size(long long n_tiles) {
+    long long g = kScanThreads;
+    while (g * kTileGroups < n_tiles) g *= 2;
+    return g;
+}
+
+struct SortedPairs {
+    const unsigned int* keys;
+    const unsigned int* vals;
+    int n;
+    bool packed;
+};
+
+__device__ __forceinline__ SortedPairs sorted_pairs(const LumenGpuFrame& f, const Control* ctrl,
+                                                    const ViewTable* vt) {
+    const unsigned int b = ctrl->cell_sort.sorted_buffer;
+    const long long n = (long long)ctrl->cell_sort.n;
+    return {b ? f.keys[1] : f.keys[0], b ? f.vals[1] : f.vals[0],
+            (int)(n < f.instance_capacity ? n : f.instance_capacity), vt->hdr.total_cells <= kPackedCells};
+}
+
+/* A segment: up to 256 consecutive pairs of one cell, as the count kernel
+ * leaves it for the write kernel. They lie in the cell sort's look-back rows,
+ * which nothing reads once it is done (2 B per instance that the frame can
+ * hold, against 80 B per 256 pairs and per cell). Without enough room, a warp
+ * writes a whole cell. */
+struct Segment {
+    int first, n;               /* its pairs */
+    unsigned int tile0;         /* the cell's first tile, and the view's tiles per row */
+    int tiles_x;
+    unsigned int before[kCellTiles];   /* per tile, its instances in the cell's pairs before */
+};
+static_assert(sizeof(Segment) == 80, "16-byte aligned");
+
+struct SegmentRoom {
+    Segment* p;
+    long long n;
+};
+
+__device__ __forceinline__ bool has_room(const SegmentRoom& room, const ViewTable* vt, int n_pairs) {
+    return n_pairs / kSegment + vt->hdr.total_cells <= room.n;
+}
+
+/* The cell's range among the sorted pairs to bounds[0], bounds[1]: as the
+ * cell sort's last pass left it, or searched by two warps when there was none
+ * (every pair in one cell) or no room for the ranges. A barrier must follow. */
+__device__ __forceinline__ void find_bounds(int* bounds, const SortedPairs& in, const int* ranges, long long cell) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (ranges) {
+        if (tid < 2) bounds[tid] = ranges[2 * cell + tid];
+    } else if (warp < 2) {
+        const unsigned int id_mask = in.packed ? (unsigned int)(kPackedCells - 1) : 0xFFFFFFFFu;
+        const int at = first_of_cell(in.keys, in.n, id_mask, (unsigned int)cell + (unsigned int)warp);
+        if (lane == 0) bounds[warp] = at;
+    }
+}
+
+/* One CTA per cell, eight segments at a time (a warp each, all its keys'
+ * reads in flight, the next eight's before these are counted). Bound by the
+ * latency of those reads (4 B per pair, once). */
+__global__ void __launch_bounds__(kCountThreads)
+list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, SegmentRoom room) {
+    chain_begin();
+    constexpr int kReads = kSegment / 32;
+    __shared__ int bounds[2];
+    __shared__ unsigned int slot_s;
+    __shared__ unsigned int count[2][kCountWarps][kCellTiles];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const SortedPairs in = sorted_pairs(f, ctrl, vt);
+    const bool noted = has_room(room, vt, in.n);
+    const int* cells = ctrl->cells_by_sort ? cell_ranges(f, ctrl, vt) : nullptr;
+    const long long n_cells = vt->hdr.total_cells, group = tile_group_size(vt->hdr.total_tiles);
+    const int n_views = vt->hdr.n_views;
+    for (long long cell = blockIdx.x; cell < n_cells; cell += gridDim.x) {
+        find_bounds(bounds, in, cells, cell);
+        const Cell c = find_cell(vt, n_views, cell);
+        __syncthreads();
+        const int first = bounds[0], end = bounds[1];
+        const int n_seg = first < end ? (end - first + kSegment - 1) / kSegment : 0;
+        if (tid == 0 && n_seg) slot_s = noted ? atomicAdd(&ctrl->n_segments, (unsigned int)n_seg) : 0u;
+        unsigned int m[kReads], base = 0u;   /* base: lane k < 16, tile k's instances so far */
+        auto read = [&](int seg) {
+#pragma unroll
+            for (int u = 0; u < kReads; ++u) {
+                const int i = first + seg * kSegment + 32 * u + lane;
+                m[u] = i < end ? pair_mask(in.packed, in.keys[i], in.packed ? 0u : in.vals[i], f.rects, c.x, c.y) : 0u;
+            }
+        };
+        read(warp);
+        for (int s0 = 0, buf = 0; s0 < n_seg; s0 += kCountWarps, buf ^= 1) {
+            const int seg = s0 + warp;
+            /* per lane: 16 counts in the bytes of four words (at most 8 each) */
+            unsigned int sum[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int u = 0; u < kReads; ++u)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) sum[q] += (((m[u] >> (4 * q)) & 0xFu) * 0x00204081u) & 0x01010101u;
+            read(seg + kCountWarps);
+            unsigned int mine = 0u;   /* lane 4 q + column: the tile's count */
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                /* columns 0 and 2, 1 and 3 as 16-bit fields */
+                const unsigned int even = __reduce_add_sync(0xffffffffu, sum[q] & 0x00FF00FFu);
+                const unsigned int odd = __reduce_add_sync(0xffffffffu, (sum[q] >> 8) & 0x00FF00FFu);
+                if ((lane >> 2) == q) mine = ((lane & 1 ? odd : even) >> (lane & 2 ? 16 : 0)) & 0xFFFFu;
+            }
+            if (lane < kCellTiles) count[buf][warp][lane] = mine;
+            __syncthreads();
+            if (lane < kCellTiles) {
+                unsigned int before = base;
+#pragma unroll
+                for (int w = 0; w < kCountWarps; ++w) {
+                    const unsigned int n = count[buf][w][lane];
+                    if (w < warp) before += n;
+                    base += n;
+                }
+                if (noted && seg < n_seg) room.p[slot_s + seg].before[lane] = before;
+            } else if (lane == kCellTiles && noted && seg < n_seg) {
+                const int i0 = first + seg * kSegment;
+                *reinterpret_cast<int4*>(room.p + slot_s + seg) =
+                    make_int4(i0, end - i0 < kSegment ? end - i0 : kSegment,
+                              (int)(c.tile_begin + (long long)c.y * c.tiles_x + c.x), c.tiles_x);
+            }
+        }
+        if (tid < kCellTiles) {
+            const long long t = c.tile(tid);
+            if (t >= 0) {
+                f.ranges[2 * t + 1] = (int)base;
+                if (base) atomicAdd(&ctrl->group_total[t / group], base);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kScanThreads)
+list_scan_kernel(ViewTable* vt, int* __restrict__ ranges, Control* ctrl) {
+    chain_begin();
+    __shared__ unsigned int warp_tot[kScanThreads / 32];
+    __shared__ unsigned int base_s;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const long long n_tiles = vt->hdr.total_tiles, group = tile_group_size(n_tiles);
+    const int n_views = vt->hdr.n_views;
+    if (blockIdx.x == 0 && tid == 0) {
+        ctrl->list_buffer = ctrl->cell_sort.sorted_buffer ^ 1u;
+        ctrl->depth_varying = ctrl->depth_sort.varying;
+        ctrl->depth_buffer = ctrl->depth_sort.sorted_buffer;
+    }
+    unsigned int touched = 0, id_or = 0, id_or_not = 0;
+    for (long long g = blockIdx.x; g * group < n_tiles; g += gridDim.x) {
+        unsigned int total = 0;
+        const unsigned int before = tid < g ? ctrl->group_total[tid] : 0u;   /* kTileGroups == kScanThreads */
+        block_exclusive_scan<kScanThreads>(before, warp_tot, &total);
+        if (tid == 0) base_s = total;
+        __syncthreads();
+        for (long long t0 = g * group; t0 < (g + 1) * group && t0 < n_tiles; t0 += kScanThreads) {
+            const long long t = t0 + tid;
+            const bool valid = t < n_tiles;
+            const unsigned int n = valid ? (unsigned int)ranges[2 * t + 1] : 0u;
+            const unsigned int start = base_s + block_exclusive_scan<kScanThreads>(n, warp_tot, &total);
+            if (valid) {
+                ranges[2 * t] = n ? (int)start : -1;
+                ranges[2 * t + 1] = n ? (int)(start + n) : -1;
+            }
+            if (n) {
+                ++touched;
+                id_or |= (unsigned int)t;
+                id_or_not |= ~(unsigned int)t;
+            }
+            /* a view's first instance is the smallest start among its tiles */
+            const unsigned int s0 = n ? start : 0xFFFFFFFFu;
+            const int v = !valid ? -1 : n_views > 1 ? find_view_by_tile(vt, n_views, t) : 0;
+            const int v0 = __shfl_sync(0xffffffffu, v, 0);
+            if (__all_sync(0xffffffffu, v == v0 || v < 0)) {
+                const unsigned int m = __reduce_min_sync(0xffffffffu, s0);
+                if (lane == 0 && m != 0xFFFFFFFFu)
+                    atomicMin(reinterpret_cast<unsigned long long*>(&vt->view[v0].inst_begin), (unsigned long long)m);
+            } else if (n) {
+                atomicMin(reinterpret_cast<unsigned long long*>(&vt->view[v].inst_begin), (unsigned long long)start);
+            }
+            __syncthreads();
+            if (tid == 0) base_s += total;
+            __syncthreads();
+        }
+    }
+    touched = __reduce_add_sync(0xffffffffu, touched);
+    id_or = __reduce_or_sync(0xffffffffu, id_or);
+    id_or_not = __reduce_or_sync(0xffffffffu, id_or_not);
+    if (lane == 0 && touched) {
+        atomicAdd(&ctrl->touched_tiles, touched);
+        atomicOr(&ctrl->tile_or, id_or);
+        atomicOr(&ctrl->tile_or_not, id_or_not);
+    }
+}
+
+/* A warp per segment: per tile and 32 pairs, a vote tells the lanes whose
+ * pair touches the tile, and they write its next instances. No warp waits for
+ * another: a segment's instances of a tile start at the tile's first position
+ * plus those of the cell's segments before, and segments are handed out
+ * evenly whatever cells they belong to (a warp per cell and 256 pairs, cell by
+ * cell, left a tail at long lists: 9 mixed views 193 us against 35).
+ * Bound by the votes' population counts (XU 52 %), issue (57 %) and the short
+ * runs' partial writes: 24 warps per SM are best (64 views of 300 k: the three
+ * kernels 464 us, with 32 warps 480, with 48 and segments of 128 pairs 769); a transpose and a gather in shared memory took half as many
+ * instructions again (2 M at 4K: 98 against 71 us). */
+__global__ void __launch_bounds__(kWriteThreads, kWriteCtas)
+list_write_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, SegmentRoom room) {
+    chain_begin();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const SortedPairs in = sorted_pairs(f, ctrl, vt);
+    const bool noted = has_room(room, vt, in.n);
+    const unsigned int out = ctrl->list_buffer;
+    unsigned int* __restrict__ kout = out ? f.keys[1] : f.keys[0];
+    unsigned int* __restrict__ vout = out ? f.vals[1] : f.vals[0];
+    const long long n_work = noted ? (long long)ctrl->n_segments : vt->hdr.total_cells;
+    const long long n_tiles = vt->hdr.total_tiles;
+    const unsigned int below = lanemask_lt();
+    for (long long w = (long long)blockIdx.x * kWriteWarps + warp; w < n_work; w += (long long)gridDim.x * kWriteWarps) {
+        int i0, end, tiles_x, cx = 0, cy = 0;
+        unsigned int tile0, before = 0u;
+        if (noted) {
+            const int4 seg = *reinterpret_cast<const int4*>(room.p + w);
+            i0 = seg.x;
+            end = seg.x + seg.y;
+            tile0 = (unsigned int)seg.z;
+            tiles_x = seg.w;
+            if (lane < kCellTiles) before = room.p[w].before[lane];
+            if (!in.packed) {
+                const ViewDesc& vd = vt->view[find_view_by_tile(vt, vt->hdr.n_views, tile0)];
+                cx = (int)((tile0 - vd.tile_begin) % tiles_x);
+                cy = (int)((tile0 - vd.tile_begin) / tiles_x);
+            }
+        } else {
+            const unsigned int id_mask = in.packed ? (unsigned int)(kPackedCells - 1) : 0xFFFFFFFFu;
+            i0 = first_of_cell(in.keys, in.n, id_mask, (unsigned int)w);
+            end = first_of_cell(in.keys, in.n, id_mask, (unsigned int)w + 1u);
+            const Cell c = find_cell(vt, vt->hdr.n_views, w);
+            tile0 = (unsigned int)(c.tile_begin + (long long)c.y * c.tiles_x + c.x);
+            tiles_x = c.tiles_x;
+            cx = c.x;
+            cy = c.y;
+        }
+        if (i0 >= end) continue;
+        /* lane k < 16: tile k's next position and its end (the ids of tiles
+         * beyond the view are other tiles', or none; no mask names them) */
+        const long long my_tile = (long long)tile0 + lane / kCellSide * tiles_x + lane % kCellSide;
+        const bool mine = lane < kCellTiles && my_tile < n_tiles;
+        unsigned int at = mine ? (unsigned int)max(f.ranges[2 * my_tile], 0) + before : 0u;
+        const unsigned int at_end =
+            mine ? (unsigned int)min(max(f.ranges[2 * my_tile + 1], 0), (int)f.instance_capacity) : 0u;
+        for (; i0 < end; i0 += kSegment) {
+            unsigned int m[kSegment / 32], v[kSegment / 32];
+#pragma unroll
+            for (int g = 0; g < kSegment / 32; ++g) {
+                const int i = i0 + g * 32 + lane;
+                v[g] = i < end ? in.vals[i] : 0u;
+                m[g] = i < end ? pair_mask(in.packed, in.keys[i], v[g], f.rects, cx, cy) : 0u;
+            }
+            unsigned int written = 0u;   /* lane k: the segment's instances of tile k */
+            bool fits = true;
+#pragma unroll
+            for (int k = 0; k < kCellTiles; ++k) {
+                unsigned int pos = __shfl_sync(0xffffffffu, at, k);
+                const unsigned int pos0 = pos, stop = __shfl_sync(0xffffffffu, at_end, k);
+                const unsigned int tile = tile0 + (unsigned int)(k / kCellSide * tiles_x + k % kCellSide);
+#pragma unroll
+                for (int g = 0; g < kSegment / 32; ++g) {
+                    const bool hit = (m[g] >> k) & 1u;
+                    const unsigned int b = __ballot_sync(0xffffffffu, hit);
+                    const unsigned int p = pos + __popc(b & below);
+                    if (hit && p < stop) {
+                        kout[p] = tile;
+                        vout[p] = v[g];
+                    }
+                    pos += __popc(b);
+                }
+                fits = fits && pos <= stop | pos == pos0;
+                if (lane == k) written = pos - pos0;
+            }
+            at += written;
+            /* self-check: more instances than were counted */
+            if (!fits && lane == 0) atomicOr(&ctrl->error_flags, LUMEN_GPU_ERR_BOUNDS);
+        }
+    }
+}
+
+int grid_of(long long n, long long cap) { return (int)(n < 1 ? 1 : n < cap ? n : cap); }
+
+}  // namespace
+
+/* n_cells, n_tiles: the batch's, or upper bounds for a persistent launch
+ * (the kernels read the batch's from the table; grids are strided). */
+void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, void* room, long long room_bytes,
+                  long long n_cells, long long n_tiles, int num_sms, cudaStream_t st) {
+    const SegmentRoom seg{static_cast<Segment*>(room), room_bytes / (long long)sizeof(Segment)};
+    launch_chained(list_count_kernel, dim3(grid_of(n_cells, 64ll * num_sms)), dim3(kCountThreads), 0, st,
+                   (const ViewTable*)vt, f, ctrl, seg);
+    launch_chained(list_scan_kernel, dim3(grid_of((n_tiles + kScanThreads - 1) / kScanThreads, 2ll * num_sms)),
+                   dim3(kScanThreads), 0, st, vt, f.ranges, ctrl);
+    const long long most = f.instance_capacity / kSegment + n_cells;   /* segments, or cells */
+    launch_chained(list_write_kernel, dim3(grid_of((most + kWriteWarps - 1) / kWriteWarps, kWriteCtas * num_sms)),
+                   dim3(kWriteThreads), 0, st, (const ViewTable*)vt, f, ctrl, seg);
+}
+
+}  // namespace lumen

@@ -48,7 +48,8 @@ static_assert(kSort64Tile == kSortTile, "the 64-bit sort's tile must be the tile
 constexpr size_t kControlBytes = align_up(sizeof(Control), 256) + align_up(view_table_bytes(1), 256);
 /* control block and a one-view table, then 8 digit passes x tiles x 256
  * look-back descriptors */
-constexpr size_t kScratchBytes = kControlBytes + (size_t)8 * (size_t)kTiles * 256 * sizeof(unsigned int);
+constexpr size_t kScratchBytes =
+    kControlBytes + align_up((size_t)8 * (size_t)(lookback_rows(kTiles) + 1) * 256 * sizeof(unsigned int), 256);
 constexpr size_t kAltKeysBytes = (size_t)kMaxPairs * sizeof(unsigned long long);
 constexpr size_t kAltValsBytes = (size_t)kMaxPairs * sizeof(unsigned int);
 
@@ -87,7 +88,7 @@ cudaError_t device_setup(void** out) {
  * alternate buffers (decided on the device). */
 __global__ void copy_back_kernel(const Control* ctrl, unsigned long long* keys, unsigned int* vals,
                                  const unsigned long long* alt_keys, const unsigned int* alt_vals, long long n) {
-    if (ctrl->tile_sort.sorted_buffer == 0) return;
+    if (ctrl->cell_sort.sorted_buffer == 0) return;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         keys[i] = alt_keys[i];
@@ -120,8 +121,8 @@ extern "C" LumenStatus lumen_gpu_sort_pairs_noalloc(uint64_t* keys, uint32_t* va
     /* the previous call's control block is still there: start from zero */
     if ((e = cudaMemsetAsync(ctrl, 0, sizeof(Control), s)) != cudaSuccess) return map_cuda(e);
     const int sms = device_sm_count();
-    launch_key_stats64(k, n, &ctrl->tile_sort, sms, s);
-    launch_sort64(k, vals, alt_keys, alt_vals, n, &ctrl->tile_sort, lb, kTiles, &ctrl->error_flags, sms, s);
+    launch_key_stats64(k, n, &ctrl->cell_sort, sms, s);
+    launch_sort64(k, vals, alt_keys, alt_vals, n, &ctrl->cell_sort, lb, kTiles, &ctrl->error_flags, sms, s);
     copy_back_kernel<<<sms * 4, 256, 0, s>>>(ctrl, k, vals, alt_keys, alt_vals, n);
     if ((e = cudaGetLastError()) != cudaSuccess) return map_cuda(e);
     unsigned int flags = 0;

@@ -1,6 +1,6 @@
 /*
- * project.cu - K1 (projection with the compacting scan) and K2 (instance
- * emission in depth order).
+ * project.cu - K1 (projection with the compacting scan) and K2 (emission
+ * of the splats' cells in depth order).
  *
  * Reference: the geometry-and-culling loop of rasterize_scene,
  * src/raster/pipeline.mojo:84-157. There, visible splats get consecutive
@@ -15,16 +15,17 @@
  * its Gaussian index, its tile rectangle and its depth key.
  *
  * K2 (after the visible splats were stably sorted by depth key): a block
- * takes 256 consecutive splats of the depth order, scans their tile counts
- * (decoupled look-back again), and writes one (tile id, visible index) pair
- * per covered tile, cooperatively, so consecutive threads write consecutive
- * instances. A stable sort of these pairs by tile id yields the reference's
- * permutation: in both, a tile's instances are ordered by (depth key,
- * visible index).
+ * takes 256 consecutive splats of the depth order, scans their cell counts
+ * (decoupled look-back again; a cell is 4x4 tiles), and writes one (cell and
+ * tile mask, visible index) pair per touched cell, cooperatively, so
+ * consecutive threads write consecutive pairs. A stable sort of these pairs by
+ * cell and a stable split of each cell's list over its tiles (lists.cu) yield
+ * the reference's permutation: in both, a tile's instances are ordered by
+ * (depth key, visible index).
  *
  * Memory: K1 reads 236 B per Gaussian once and writes 68 B per visible
  * splat + 4 B per Gaussian; K2 reads 12 B per visible splat and writes 8 B
- * per instance.
+ * per pair (about two pairs per splat where there are seven instances).
  */
 #include "splat_common.cuh"
 
@@ -172,31 +173,35 @@ project_kernel(const ViewTable* __restrict__ vt, int n_views_hint, LumenRenderOp
     }
 }
 
-/* Instances of an emission warp resolved to their splats per window. */
+/* Pairs of an emission warp resolved to their splats per window. */
 constexpr int kEmitWindow = 256;
 constexpr int kEmitPerLane = kEmitWindow / 32;
 static_assert(kEmitPerLane == 8, "two 16-byte slot groups per lane");
 
+constexpr int kEmitWarps = kEmitThreads / 32;
+constexpr int kEmitMaxRounds = 4;
+
 struct EmitSmem {
-    /* per warp and window slot: 1 + the lane whose splat holds the instance */
+    /* per warp and window slot: 1 + the lane whose splat holds the pair */
     __align__(16) unsigned int owner[kEmitThreads / 32][kEmitWindow];
     unsigned int blk;
-    unsigned int warp_tot[kEmitThreads / 32];
-    unsigned long long inst_base;
-    /* per splat: its first instance (block-relative), tiles per rectangle
-     * row, the batch-wide id of its first tile, tiles per view row */
+    unsigned int warp_pairs[kEmitMaxRounds][kEmitWarps], warp_tiles[kEmitMaxRounds][kEmitWarps];
+    unsigned long long base;             /* the blocks before: instances and pairs (pack_counts) */
+    /* per splat: its first pair (block-relative), cells per rectangle row,
+     * the batch-wide id of its first cell, cells per view row */
     uint4 run[kEmitThreads];
-    /* per splat: 1 / (tiles per rectangle row), as bits, for the row of an
-     * instance; its visible index */
+    /* per splat: 1 / (cells per rectangle row), as bits, for the row of a
+     * pair; its visible index */
     uint2 aux[kEmitThreads];
-    unsigned int hist[4][256];            /* the block's tile ids: counts of each digit value */
-    unsigned long long key_or, key_or_not;
+    unsigned long long rect[kEmitThreads];
+    unsigned int hist[4][256];            /* the CTA's cell ids: counts of each digit value */
+    unsigned int cut, cut_tiles, kept;    /* at the instance capacity (emit_cut) */
 };
 static_assert(kEmitThreads == 256, "one emission thread per digit value clears and adds the block's counts");
 
 /* Owners of the warp's window [a, a + kEmitWindow): slot k of s.owner[warp]
- * gets 1 + the lane whose splat holds instance a + k (block-relative). Returns
- * the window's instance count. */
+ * gets 1 + the lane whose splat holds pair a + k (block-relative). Returns
+ * the window's pair count. */
 __device__ __forceinline__ unsigned int emit_window_owners(EmitSmem& s, int warp, int lane, unsigned int a,
                                                            unsigned int excl, unsigned int cnt, unsigned int w_end) {
     unsigned int* own = s.owner[warp];
@@ -226,10 +231,10 @@ __device__ __forceinline__ unsigned int emit_window_owners(EmitSmem& s, int warp
     return w_end - a < (unsigned int)kEmitWindow ? w_end - a : kEmitWindow;
 }
 
-/* Batch-wide tile id of block-relative instance j of splat lo: rows outer,
- * columns inner (pipeline.mojo:152-153). */
-__device__ __forceinline__ unsigned int emit_tile(const EmitSmem& s, int lo, unsigned int j) {
-    const uint4 rn = s.run[lo];
+/* Row of block-relative pair j of splat lo in its rectangle of cells (rows
+ * outer, columns inner) and *column. */
+__device__ __forceinline__ unsigned int emit_row(const EmitSmem& s, int lo, const uint4& rn, unsigned int j,
+                                                 unsigned int* column) {
     const unsigned int w = rn.y;
     const unsigned int q = j - rn.x;
     /* q / w through the reciprocal (exact after one correction step while
@@ -242,50 +247,107 @@ __device__ __forceinline__ unsigned int emit_tile(const EmitSmem& s, int lo, uns
     } else {
         row = q / w;
     }
-    return rn.z + row * rn.w + (q - row * w);
+    *column = q - row * w;
+    return row;
 }
 
-/* Writes the instance at pos when it is within the capacity; counts its low
- * tile-id digit. Returns whether it was written. */
-__device__ __forceinline__ bool emit_store(const LumenGpuFrame& f, EmitSmem& s, unsigned long long pos,
-                                           long long cap, unsigned int tile, int lo) {
-    if (pos >= (unsigned long long)cap) return false;
-    f.keys[0][pos] = tile;
-    f.vals[0][pos] = s.aux[lo].y;
-    atomicAdd(&s.hist[0][tile & 0xFFu], 1u);
-    return true;
-}
-
-/* The higher tile-id digits of the warp's written instances (a prefix of
- * its lanes). They change rarely from one instance to the next (a splat's
- * row of tiles): each run of equal values over consecutive lanes is counted
- * once, by its first lane. */
-__device__ __forceinline__ void emit_count(EmitSmem& s, int lane, int nd, unsigned int tile, bool kept) {
-    const unsigned int n_kept = __popc(__ballot_sync(0xffffffffu, kept));
-    for (int d = 1; d < nd; ++d) {
-        const unsigned int dv = kept ? (tile >> (8 * d)) & 0xFFu : 0x100u;
-        const unsigned int prev = __shfl_up_sync(0xffffffffu, dv, 1);
-        const bool first = kept && (lane == 0 || prev != dv);
-        const unsigned int firsts = __ballot_sync(0xffffffffu, first);
-        if (first) {
-            const unsigned int later = firsts & ~((2u << lane) - 1u);
-            const unsigned int run_end = later ? (unsigned int)(__ffs(later) - 1) : n_kept;
-            atomicAdd(&s.hist[d][dv], run_end - (unsigned int)lane);
+/* The block in which the instances reach the capacity (`room` of its own are
+ * kept): the first splat that does not fit wholly (s.cut), how many of its
+ * tiles do (s.cut_tiles, row-major in its rectangle, a prefix of its cells)
+ * and the block's pairs up to there (s.kept). One thread; a frame that
+ * overflows is rendered again. */
+__device__ __noinline__ void emit_cut(EmitSmem& s, unsigned int room, int n) {
+    s.cut = (unsigned int)n;
+    s.cut_tiles = 0u;
+    s.kept = 0u;
+    unsigned long long used = 0ull;
+    for (int k = 0; k < n; ++k) {
+        const unsigned long long r = s.rect[k];
+        const unsigned int w = (unsigned int)(rect_max_tx(r) - rect_min_tx(r) + 1);
+        const unsigned int h = (unsigned int)(rect_max_ty(r) - rect_min_ty(r) + 1);
+        if (used + (unsigned long long)w * h <= room) {
+            used += (unsigned long long)w * h;
+            continue;
         }
+        const unsigned int left = room - (unsigned int)used;
+        s.cut = (unsigned int)k;
+        s.cut_tiles = left;
+        const unsigned int row = left / w, col = left - row * w;   /* `row` whole rows and `col` tiles of the next */
+        const unsigned int cx0 = rect_min_tx(r) / kCellSide, cy0 = rect_min_ty(r) / kCellSide, cw = s.run[k].y;
+        unsigned int cells = 0u;
+        if (row > 0) cells = cw * ((rect_min_ty(r) + row - 1) / kCellSide - cy0 + 1);
+        if (col > 0) {
+            const unsigned int before = cw * ((rect_min_ty(r) + row) / kCellSide - cy0);
+            cells = max(cells, before + (rect_min_tx(r) + col - 1) / kCellSide - cx0 + 1);
+        }
+        s.kept = s.run[k].x + cells;
+        return;
     }
 }
 
-/* Like project_kernel: 256 consecutive splats of the depth order per ticket.
- * Tile ids are batch-wide (view tile_begin + ty * tiles_x + tx).
+/* The tiles of the cell whose first tile is (x, y) among the first `left`
+ * of the rectangle's, row-major. */
+__device__ __noinline__ unsigned int emit_cut_mask(unsigned long long r, int x, int y, unsigned int mask,
+                                                   unsigned int left) {
+    const int w = rect_max_tx(r) - rect_min_tx(r) + 1;
+    for (int k = 0; k < 16; ++k) {
+        const long long q = (long long)(y + k / 4 - rect_min_ty(r)) * w + (x + k % 4 - rect_min_tx(r));
+        if (q >= (long long)left) mask &= ~(1u << k);
+    }
+    return mask;
+}
+
+/* A splat's rectangle in cells, and its tile and cell counts. */
+struct CellRect {
+    unsigned int tiles;   /* below 2^24, so that 256 of them fit 32 bits */
+    unsigned int cx, cy, cw, pairs;
+};
+
+__device__ __forceinline__ CellRect cell_rect(unsigned long long r) {
+    const unsigned int mnx = rect_min_tx(r), mny = rect_min_ty(r), mxx = rect_max_tx(r), mxy = rect_max_ty(r);
+    CellRect c;
+    c.tiles = (mxx - mnx + 1u) * (mxy - mny + 1u);
+    c.cx = mnx / kCellSide;
+    c.cy = mny / kCellSide;
+    c.cw = mxx / kCellSide - c.cx + 1u;
+    c.pairs = c.cw * (mxy / kCellSide - c.cy + 1u);
+    return c;
+}
+
+/* A warp whose splats touch at most this many cells each writes them one
+ * splat per lane; beyond, its lanes share the pairs evenly (a splat over the
+ * whole image would hold its warp up). */
+constexpr unsigned int kEmitLaneCells = 16;
+
+/* kRounds rounds of 256 consecutive splats of the depth order per ticket: one
+ * pair per cell that a splat's rectangle touches (batch-wide cell id and tile
+ * mask, visible index), in depth order, cells row-major. Tickets are taken in
+ * order, and a ticket's splats sum up their predecessors' instances and pairs
+ * by decoupled look-back.
  *
- * The emission also does the tile sort's preparation, so that the sort
- * needs no pass of its own over the instances: it counts the digit values
- * of the tile ids it writes (per block in shared memory, then added to the
- * sort's histogram), clears the sort's look-back descriptors of the
- * 256 * sort_items-key tiles that start among its instances, and fills the
- * tile ranges with (-1, -1). */
-template <bool kPersistent>
-__global__ void __launch_bounds__(kEmitThreads, 8)
+ * The emission also does the cell sort's preparation, so that the sort
+ * needs no pass of its own over the pairs: it counts the digit values of the
+ * cell ids it writes (per CTA in shared memory, added to the sort's histogram
+ * once all its tickets are done) and clears the sort's look-back descriptors of
+ * the 256 * sort_items-key tiles that start among its pairs. It also fills the
+ * cells' ranges with (-1, -1) for the sort's last pass.
+ *
+ * Instances (the tiles of the rectangles) are only counted here; those
+ * beyond the capacity are left out of the pairs, so that the lists hold the
+ * first `capacity` instances of the depth order, row-major per splat.
+ *
+ * Bound by the random 8-byte gathers of the rectangles, and before that by
+ * the look-back: the resident CTAs start together, so inclusive sums travel
+ * 32 tickets per step of about 0.45 us, and with 256 splats per ticket 1 M
+ * splats waited 40 of 57 us. Four rounds per ticket make the chain a quarter
+ * as long and keep four gathers per thread in flight: 57 -> 41 us at 1 M
+ * splats and 1080p, 123 -> 74 at 2 M and 4K, 850 -> 570 for 64 views of
+ * 300 k. Below three tickets of 1024 per SM one round spreads the splats
+ * over more CTAs (250 k splats: 23 us, against 33 with four). Wider look-back
+ * steps (8 descriptors per lane) and a scan in kernels of its own were slower
+ * (1 M: 78 and 61 us). */
+template <int kRounds>
+__global__ void __launch_bounds__(kEmitThreads, 6)
 emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, unsigned long long* lb,
             unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys) {
     chain_begin();
@@ -293,125 +355,202 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long V = ctrl->n_visible;
     const unsigned int* order = ctrl->depth_sort.sorted_buffer ? f.depth_order[1] : f.depth_order[0];
-    const long long cap = f.instance_capacity;
-    /* the tile-id bytes that can vary: ids are below the batch's tile count */
-    const long long n_tiles = vt->hdr.total_tiles;
+    const unsigned int cap = (unsigned int)f.instance_capacity;   /* below 2^30 */
+    /* the cell-id bytes that can vary: ids are below the batch's cell count */
+    const long long n_cells = vt->hdr.total_cells;
+    const bool packed = n_cells <= kPackedCells;
     int nd = 0;
-    for (long long t = n_tiles - 1; t > 0 && nd < 4; t >>= 8) ++nd;
-    {
+    for (long long t = n_cells - 1; t > 0 && nd < 4; t >>= 8) ++nd;
+    for (int d = 0; d < 4; ++d) s.hist[d][tid] = 0u;
+    if (int* ranges = cell_ranges(f, ctrl, vt)) {
         const long long nthreads = (long long)gridDim.x * blockDim.x;
-        for (long long j = (long long)blockIdx.x * blockDim.x + tid; j < 2 * n_tiles; j += nthreads) f.ranges[j] = -1;
+        for (long long j = (long long)blockIdx.x * blockDim.x + tid; j < 2 * n_cells; j += nthreads) ranges[j] = -1;
     }
+    unsigned int kor = 0u, knot = 0u;
+    unsigned long long tile_sum = 0ull;
     for (;;) {
-        if (tid == 0) {
-            s.blk = atomicAdd(&ctrl->emit_ticket, 1u);
-            s.key_or = 0ull;
-            s.key_or_not = 0ull;
-        }
-        for (int d = 0; d < nd; ++d) s.hist[d][tid] = 0u;
+        if (tid == 0) s.blk = atomicAdd(&ctrl->emit_ticket, 1u);
         __syncthreads();
         const int blk = (int)s.blk;
-        if ((long long)blk * kEmitThreads >= V) break;   /* past the visible splats: no look-back waits on it */
-        const long long p = (long long)blk * kEmitThreads + tid;
-        unsigned int cnt = 0, v = 0, w = 1, tile0 = 0, tiles_x = 0;
-        if (p < V) {
-            v = order[p];
-            const unsigned long long r = f.rects[v];
-            const int mnx = rect_min_tx(r), mny = rect_min_ty(r);
-            w = (unsigned int)(rect_max_tx(r) - mnx + 1);
-            const unsigned int h = (unsigned int)(rect_max_ty(r) - mny + 1);
-            cnt = w * h;
-            const ViewDesc& vd = vt->view[rect_view(r)];
-            tiles_x = (unsigned int)vd.tiles_x;
-            tile0 = (unsigned int)vd.tile_begin + (unsigned int)mny * tiles_x + (unsigned int)mnx;
-        }
-        unsigned int block_inst = 0;
-        const unsigned int excl = block_exclusive_scan<kEmitThreads>(cnt, s.warp_tot, &block_inst);
-        if (tid == 0) st_volatile_u64(lb + blk, (blk == 0 ? kDescIncl64 : kDescAgg64) | block_inst);
-        s.run[tid] = make_uint4(excl, w, tile0, tiles_x);
-        s.aux[tid] = make_uint2(__float_as_uint(1.0f / (float)w), v);
-        if (warp == 0) {
-            const unsigned long long e = blk > 0 ? lookback64(lb, blk, &ctrl->error_flags) : 0ull;
-            if (lane == 0) {
-                s.inst_base = e;
-                if (blk > 0) st_volatile_u64(lb + blk, kDescIncl64 | (e + block_inst));
-            }
-        }
-        __syncthreads();
-        const unsigned long long inst_base = s.inst_base;
-        unsigned int kor = 0u, knot = 0u;
-        /* The warp's instances (those of its 32 splats, consecutive in the
-         * block's instance order), kEmitWindow at a time. Each splat marks
-         * the slot where its run of instances enters the window (the splat
-         * already running at the window's start marks slot 0); a prefix
-         * maximum over the marks then gives every slot its splat without a
-         * search, and consecutive lanes write consecutive instances. Warps
-         * work through their windows independently: only warp barriers. */
-        const unsigned int my_end = excl + cnt;
-        const unsigned int w_begin = __shfl_sync(0xffffffffu, excl, 0);
-        const unsigned int w_end = __shfl_sync(0xffffffffu, my_end, 31);
-        for (unsigned int a = w_begin; a < w_end; a += kEmitWindow) {
-            const unsigned int nwin = emit_window_owners(s, warp, lane, a, excl, cnt, w_end);
-            for (unsigned int b0 = 0; b0 < nwin; b0 += 32) {
-                const unsigned int jj = b0 + lane;
-                unsigned int tile = 0u;
-                bool kept = false;
-                if (jj < nwin) {
-                    const int lo = warp * 32 + (int)s.owner[warp][jj] - 1;
-                    tile = emit_tile(s, lo, a + jj);
-                    kor |= tile;
-                    knot |= ~tile;
-                    kept = emit_store(f, s, inst_base + a + jj, cap, tile, lo);
-                }
-                emit_count(s, lane, nd, tile, kept);
-            }
-            __syncwarp();
+        const long long p0 = (long long)blk * (kRounds * kEmitThreads);
+        if (p0 >= V) break;   /* past the visible splats: no look-back waits on it */
+        /* every round's splat of the thread (the gathers in flight together) */
+        unsigned int vis[kRounds], first_pair[kRounds];
+        unsigned long long rects[kRounds];
+#pragma unroll
+        for (int q = 0; q < kRounds; ++q) {
+            const long long p = p0 + q * kEmitThreads + tid;
+            vis[q] = p < V ? order[p] : 0xFFFFFFFFu;
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            kor |= __shfl_xor_sync(0xffffffffu, kor, o);
-            knot |= __shfl_xor_sync(0xffffffffu, knot, o);
-        }
-        if (lane == 0 && block_inst) {
-            atomicOr(&s.key_or, (unsigned long long)kor);
-            atomicOr(&s.key_or_not, (unsigned long long)knot);
+        for (int q = 0; q < kRounds; ++q) rects[q] = vis[q] != 0xFFFFFFFFu ? f.rects[vis[q]] : 0ull;
+        /* in-round scans over the warp's pairs, its sums to shared memory */
+#pragma unroll
+        for (int q = 0; q < kRounds; ++q) {
+            const CellRect c = cell_rect(rects[q]);
+            const unsigned int tiles = vis[q] != 0xFFFFFFFFu ? c.tiles : 0u, pairs = vis[q] != 0xFFFFFFFFu ? c.pairs : 0u;
+            unsigned int x = pairs;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            first_pair[q] = x - pairs;
+            const unsigned int warp_tiles = __reduce_add_sync(0xffffffffu, tiles);
+            if (lane == 31) {
+                s.warp_pairs[q][warp] = x;
+                s.warp_tiles[q][warp] = warp_tiles;
+            }
         }
         __syncthreads();
-        for (int d = 0; d < nd; ++d) {
-            const unsigned int c = s.hist[d][tid];
-            if (c) atomicAdd(&ctrl->tile_sort.hist[d][tid], c);
-        }
-        /* look-back descriptors of the sort tiles whose first key is one of
-         * this block's instances (every tile of the sort has one) */
-        {
-            /* only the first `capacity` instances are sorted (capacity < 2^30) */
-            const unsigned long long ucap = (unsigned long long)cap;
-            const unsigned long long e0 = inst_base, e1 = inst_base + block_inst;
-            const unsigned int i0 = (unsigned int)(e0 < ucap ? e0 : ucap), i1 = (unsigned int)(e1 < ucap ? e1 : ucap);
-            const unsigned int tk = (unsigned int)sort_tile_keys;
-            const unsigned int t0 = (i0 + tk - 1u) / tk;
-            unsigned int t1 = (i1 + tk - 1u) / tk;
-            if ((long long)t1 > sort_lb_tiles) t1 = (unsigned int)sort_lb_tiles;
-            for (int d = 0; d < nd; ++d) {
-                unsigned int* region = sort_lb + (size_t)d * (size_t)sort_lb_tiles * 256;
-                for (unsigned int j = t0 * 256u + (unsigned int)tid; j < t1 * 256u; j += kEmitThreads) region[j] = 0u;
+        if (warp == 0) {
+            /* the block's sums, round by round, saturated as in the descriptors */
+            unsigned long long block = 0ull;
+            for (int q = 0; q < kRounds; ++q) {
+                const unsigned int p = __reduce_add_sync(0xffffffffu, lane < kEmitWarps ? s.warp_pairs[q][lane] : 0u);
+                const unsigned int t = __reduce_add_sync(0xffffffffu, lane < kEmitWarps ? s.warp_tiles[q][lane] : 0u);
+                block = add_counts(block, pack_counts(min(t, kSaturated), min(p, kSaturated)));
+                tile_sum += t;
+            }
+            if (lane == 0) st_volatile_u64(lb + blk, (blk == 0 ? kDescIncl64 : kDescAgg64) | block);
+            const unsigned long long e = blk > 0 ? lookback_counts(lb, blk, &ctrl->error_flags) : 0ull;
+            if (lane == 0) {
+                s.base = e;
+                if (blk > 0) st_volatile_u64(lb + blk, kDescIncl64 | add_counts(e, block));
             }
         }
-        if (tid == 0) {
-            if (block_inst) {
-                atomicOr(&ctrl->tile_sort.key_or, s.key_or);
-                atomicOr(&ctrl->tile_sort.key_or_not, s.key_or_not);
+        __syncthreads();
+        unsigned long long base = s.base;
+        for (int q = 0; q < kRounds && p0 + q * kEmitThreads < V; ++q) {
+            const unsigned int v = vis[q];
+            const unsigned long long r = rects[q];
+            CellRect c = cell_rect(r);
+            unsigned int cell0 = 0u, cells_x = 0u;
+            if (v != 0xFFFFFFFFu) {
+                const ViewDesc& vd = vt->view[rect_view(r)];
+                cells_x = (unsigned int)vd.cells_x;
+                cell0 = (unsigned int)vd.cell_begin + c.cy * cells_x + c.cx;
+            } else {
+                c.pairs = 0u;
             }
-            if ((long long)blk == (V - 1) / kEmitThreads) {
-                const unsigned long long K = inst_base + block_inst;
-                ctrl->n_instances = K;
-                ctrl->tile_sort.n = K;
-                if (K > (unsigned long long)cap) atomicOr(&ctrl->error_flags, LUMEN_GPU_ERR_CAPACITY);
+            unsigned int excl = first_pair[q], block_pairs = 0u, block_tiles = 0u;
+#pragma unroll
+            for (int w = 0; w < kEmitWarps; ++w) {
+                if (w == warp) excl += block_pairs;
+                block_pairs += s.warp_pairs[q][w];
+                block_tiles += s.warp_tiles[q][w];
             }
+            s.rect[tid] = r;
+            s.run[tid] = make_uint4(excl, c.cw, cell0, cells_x);
+            s.aux[tid] = make_uint2(__float_as_uint(1.0f / (float)c.cw), v);
+            __syncwarp();
+            const unsigned int tile_base = (unsigned int)(base >> 31) & 0x7FFFFFFFu;
+            const unsigned int pair_base = (unsigned int)base & 0x7FFFFFFFu;
+            /* the capacity is reached in this block or before it */
+            const bool over = tile_base + min(block_tiles, kSaturated) > cap;
+            unsigned int kept_pairs = block_pairs, cut = kEmitThreads;
+            if (over) {
+                __syncthreads();
+                if (tid == 0) {
+                    const long long left = V - p0 - q * kEmitThreads;
+                    emit_cut(s, tile_base < cap ? cap - tile_base : 0u, (int)(left < kEmitThreads ? left : kEmitThreads));
+                }
+                __syncthreads();
+                kept_pairs = s.kept;
+                cut = s.cut;
+            }
+            /* one pair of splat lo (rectangle rect, first tile of the cell's column and row), block-relative index j */
+            auto store = [&](unsigned int lo, unsigned long long rect, unsigned int cx, unsigned int cy, unsigned int cell,
+                             unsigned int vis, unsigned int j) {
+                unsigned int key = cell;
+                if (packed) {
+                    const int x = (int)cx * kCellSide, y = (int)cy * kCellSide;
+                    unsigned int mask = cell_mask(rect, x, y);
+                    if (over && lo == cut) mask = emit_cut_mask(rect, x, y, mask, s.cut_tiles);
+                    key |= mask << 16;
+                }
+                const unsigned int pos = pair_base + j;   /* below the capacity, like the instances */
+                if (pos >= cap) return;
+                kor |= cell;
+                knot |= ~cell;
+                f.keys[0][pos] = key;
+                f.vals[0][pos] = vis;
+                for (int d = 0; d < nd; ++d) atomicAdd(&s.hist[d][(cell >> (8 * d)) & 0xFFu], 1u);
+            };
+            const unsigned int most = __reduce_max_sync(0xffffffffu, c.pairs);
+            if (most <= kEmitLaneCells) {
+                unsigned int col = 0u, row = 0u;
+                for (unsigned int k = 0; k < most; ++k) {
+                    if (k < c.pairs && excl + k < kept_pairs)
+                        store((unsigned int)tid, r, c.cx + col, c.cy + row, cell0 + row * cells_x + col, v, excl + k);
+                    if (++col == c.cw) {
+                        col = 0u;
+                        ++row;
+                    }
+                }
+            } else {
+                /* The warp's pairs (those of its 32 splats, consecutive in the
+                 * block's order), kEmitWindow at a time. Each splat marks the
+                 * slot where its run of pairs enters the window (the splat
+                 * already running at the window's start marks slot 0); a prefix
+                 * maximum over the marks then gives every slot its splat without
+                 * a search, and consecutive lanes write consecutive pairs. */
+                const unsigned int my_end = excl + c.pairs;
+                const unsigned int w_begin = __shfl_sync(0xffffffffu, excl, 0);
+                const unsigned int w_end = min(__shfl_sync(0xffffffffu, my_end, 31), kept_pairs);
+                for (unsigned int a = w_begin; a < w_end; a += kEmitWindow) {
+                    const unsigned int nwin = emit_window_owners(s, warp, lane, a, excl, c.pairs, w_end);
+                    for (unsigned int jj = lane; jj < nwin; jj += 32) {
+                        const int lo = warp * 32 + (int)s.owner[warp][jj] - 1;
+                        const uint4 rn = s.run[lo];
+                        unsigned int column;
+                        const unsigned int row = emit_row(s, lo, rn, a + jj, &column);
+                        const unsigned long long rect = s.rect[lo];
+                        store((unsigned int)lo, rect, rect_min_tx(rect) / kCellSide + column,
+                              rect_min_ty(rect) / kCellSide + row, rn.z + row * rn.w + column, s.aux[lo].y, a + jj);
+                    }
+                    __syncwarp();
+                }
+            }
+            /* look-back descriptors of the sort tiles whose first key is one of
+             * this block's pairs (every tile of the sort has one) */
+            {
+                const unsigned int i0 = min(pair_base, cap), i1 = min(pair_base + kept_pairs, cap);
+                const unsigned int tk = (unsigned int)sort_tile_keys;
+                const unsigned int t0 = (i0 + tk - 1u) / tk;
+                unsigned int t1 = (i1 + tk - 1u) / tk;
+                if ((long long)t1 > sort_lb_tiles) t1 = (unsigned int)sort_lb_tiles;
+                for (int d = 0; d < nd; ++d) {
+                    unsigned int* region = sort_lb + (size_t)d * (size_t)lookback_rows(sort_lb_tiles) * 256;
+                    for (unsigned int t = t0; t < t1; ++t) {
+                        region[(size_t)t * 256 + tid] = 0u;
+                        if (t % kLookbackGroup == 0)   /* its group's row */
+                            region[((size_t)sort_lb_tiles + t / kLookbackGroup) * 256 + tid] = 0u;
+                    }
+                }
+            }
+            if (tid == 0) {
+                const bool last = p0 + (q + 1) * kEmitThreads >= V;
+                if (over ? tile_base <= cap : last) ctrl->cell_sort.n = (unsigned long long)(pair_base + kept_pairs);
+                if (over && last) atomicOr(&ctrl->error_flags, LUMEN_GPU_ERR_CAPACITY);
+            }
+            base = add_counts(base, pack_counts(min(block_tiles, kSaturated), min(block_pairs, kSaturated)));
+            if (over) __syncthreads();
+            __syncwarp();
         }
-        if (!kPersistent) break;
         __syncthreads();
     }
+    for (int d = 0; d < nd; ++d) {
+        const unsigned int n = s.hist[d][tid];
+        if (n) atomicAdd(&ctrl->cell_sort.hist[d][tid], n);
+    }
+    kor = __reduce_or_sync(0xffffffffu, kor);
+    knot = __reduce_or_sync(0xffffffffu, knot);
+    if (lane == 0 && (kor | knot)) {
+        atomicOr(&ctrl->cell_sort.key_or, (unsigned long long)kor);
+        atomicOr(&ctrl->cell_sort.key_or_not, (unsigned long long)knot);
+    }
+    if (tid == 0 && tile_sum) atomicAdd(&ctrl->n_instances, tile_sum);
 }
 
 /* ---------------------------------------------------------------------
@@ -668,7 +807,7 @@ void prime_persistent_launches() {
     cudaFuncSetAttribute(project_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjStageBytes);
     cudaFuncSetAttribute(project_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjStageBytes);
     g_project_per_sm = resident_ctas((const void*)project_kernel<true>, kProjThreads, kProjStageBytes);
-    g_emit_per_sm = resident_ctas((const void*)emit_kernel<true>, kEmitThreads, 0);
+    g_emit_per_sm = resident_ctas((const void*)emit_kernel<1>, kEmitThreads, 0);
     cudaFuncSetAttribute(batch_project_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kProjStageBytes);
     cudaFuncSetAttribute(batch_project_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -718,21 +857,22 @@ void launch_project(const ViewTable* vt, int n_views, const LumenRenderOptions& 
     }
 }
 
-/* sort_lb: the tile sort's look-back region (sort_lb_tiles descriptor
+/* sort_lb: the cell sort's look-back region (sort_lb_tiles descriptor
  * tiles per digit) for digit passes of sort_tile_keys keys per tile. */
 void launch_emit(const ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned long long* lb,
                  unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys, long long n_blocks,
                  bool persistent, int num_sms, cudaStream_t st) {
     if (n_blocks <= 0) return;
-    if (persistent) {
-        const int per_sm = g_emit_per_sm > 0 ? g_emit_per_sm : 1;
-        launch_chained(emit_kernel<true>, dim3(per_sm * num_sms), dim3(kEmitThreads), 0, st, vt, f, ctrl, lb, sort_lb,
-                       sort_lb_tiles, sort_tile_keys);
-    } else {
-        launch_chained(emit_kernel<false>,
-                       dim3((unsigned int)((n_blocks * kProjThreads + kEmitThreads - 1) / kEmitThreads)),
+    const long long resident = (long long)(g_emit_per_sm > 0 ? g_emit_per_sm : 1) * num_sms;
+    auto run = [&](auto kernel, int rounds) {
+        const long long blocks = (n_blocks * kProjThreads + rounds * kEmitThreads - 1) / (rounds * kEmitThreads);
+        launch_chained(kernel, dim3((unsigned int)(persistent || blocks > resident ? resident : blocks)),
                        dim3(kEmitThreads), 0, st, vt, f, ctrl, lb, sort_lb, sort_lb_tiles, sort_tile_keys);
-    }
+    };
+    if (n_blocks * kProjThreads >= 3ll * num_sms * kEmitMaxRounds * kEmitThreads)
+        run(emit_kernel<kEmitMaxRounds>, kEmitMaxRounds);
+    else
+        run(emit_kernel<1>, 1);
 }
 
 }  // namespace lumen

@@ -40,8 +40,8 @@ LumenStatus map_cuda(cudaError_t e);
 void launch_init(const ScratchLayout& L, unsigned char* base, const BatchHeader* hdr, const ViewDesc* v0,
                  cudaStream_t s);
 void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRenderOptions& opt,
-                     const LumenGpuFrame& f, long long n_slots, long long n_tiles, int n_views, bool persistent,
-                     const LaunchConfig& lc, cudaEvent_t* ev, cudaStream_t s, bool with_composite,
+                     const LumenGpuFrame& f, long long n_slots, long long n_tiles, long long n_cells, int n_views,
+                     bool persistent, const LaunchConfig& lc, cudaEvent_t* ev, cudaStream_t s, bool with_composite,
                      long long n_units);
 
 namespace {
@@ -262,14 +262,14 @@ cudaError_t alloc_slot(LumenServer* srv, Slot* s) {
 
 /* The batch's work on the slot's stream, up to the counter read-back. */
 void enqueue_batch_work(LumenServer* srv, Slot* s, const LaunchConfig& lc, bool persistent, long long n_slots,
-                        long long n_tiles, int n_views, size_t table_bytes, long long n_units) {
+                        long long n_tiles, long long n_cells, int n_views, size_t table_bytes, long long n_units) {
     unsigned char* base = (unsigned char*)s->frame.scratch;
     cudaMemcpyAsync(base + s->layout.table_off, s->h_table, table_bytes, cudaMemcpyHostToDevice, s->stream);
     {
         /* batches in flight share the GPU: plain launches (see ChainedLaunches) */
         ChainedLaunches plain(false);
         launch_init(s->layout, base, nullptr, nullptr, s->stream);
-        launch_pipeline(s->layout, base, srv->cfg.options, s->frame, n_slots, n_tiles, n_views, persistent, lc,
+        launch_pipeline(s->layout, base, srv->cfg.options, s->frame, n_slots, n_tiles, n_cells, n_views, persistent, lc,
                         nullptr, s->stream, true, n_units);
     }
     cudaMemcpyAsync(s->h_back, base + s->layout.control_off, sizeof(Control), cudaMemcpyDeviceToHost, s->stream);
@@ -281,7 +281,8 @@ cudaError_t capture(LumenServer* srv, Slot* s, int variant) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
-    enqueue_batch_work(srv, s, kVariantTable[variant], true, srv->max_slots, srv->max_tiles, 0,
+    /* at most a cell per tile */
+    enqueue_batch_work(srv, s, kVariantTable[variant], true, srv->max_slots, srv->max_tiles, srv->max_tiles, 0,
                        view_table_bytes(srv->cfg.max_views_per_batch), 0);
     e = cudaStreamEndCapture(s->stream, &g);
     if (e != cudaSuccess) return e;
@@ -293,9 +294,10 @@ cudaError_t capture(LumenServer* srv, Slot* s, int variant) {
 /* Fill the slot's page-locked view table for its batch; returns the
  * batch's projection slots, tiles and projection units (views of one scene
  * share their units). */
-void build_table(LumenServer* srv, Slot* s, long long* n_slots, long long* n_tiles, long long* n_units) {
+void build_table(LumenServer* srv, Slot* s, long long* n_slots, long long* n_tiles, long long* n_cells,
+                 long long* n_units) {
     ViewTable* vt = (ViewTable*)s->h_table;
-    long long blocks = 0, tiles = 0, pix = 0;
+    long long blocks = 0, tiles = 0, cells = 0, pix = 0;
     const int nv = (int)s->batch.size();
     for (int v = 0; v < nv; ++v) {
         const Request& r = *s->batch[(size_t)v];
@@ -307,7 +309,10 @@ void build_table(LumenServer* srv, Slot* s, long long* n_slots, long long* n_til
         d.img.rgb8 = s->d_rgb8 + pix * 3;
         d.block_begin = blocks;
         d.tile_begin = tiles;
+        d.cells_x = cells_along(d.tiles_x);
+        d.cell_begin = cells;
         d.inst_begin = -1;
+        cells += (long long)d.cells_x * cells_along((r.cam.height + kTile - 1) / kTile);
         blocks += (d.g.count + kProjThreads - 1) / kProjThreads;
         tiles += r.tiles;
         pix += r.pixels;
@@ -316,17 +321,19 @@ void build_table(LumenServer* srv, Slot* s, long long* n_slots, long long* n_til
     vt->hdr.n_views = nv;
     vt->hdr.total_blocks = blocks;
     vt->hdr.total_tiles = tiles;
+    vt->hdr.total_cells = cells;
     vt->hdr.total_units = assign_scene_groups(vt->view, nv);
     *n_slots = blocks * kProjThreads;
     *n_tiles = tiles;
+    *n_cells = cells;
     *n_units = vt->hdr.total_units;
 }
 
 /* Scheduler-thread side of a launch (no lock held). */
 cudaError_t launch_batch(LumenServer* srv, Slot* s) {
     cudaSetDevice(srv->device);
-    long long n_slots = 0, n_tiles = 0, n_units = 0;
-    build_table(srv, s, &n_slots, &n_tiles, &n_units);
+    long long n_slots = 0, n_tiles = 0, n_cells = 0, n_units = 0;
+    build_table(srv, s, &n_slots, &n_tiles, &n_cells, &n_units);
     const LaunchConfig lc = kVariantTable[s->variant];
     cudaError_t e = cudaEventRecord(s->ev_start, s->stream);
     if (e != cudaSuccess) return e;
@@ -334,7 +341,7 @@ cudaError_t launch_batch(LumenServer* srv, Slot* s) {
         if (!s->exec[s->variant] && (e = capture(srv, s, s->variant)) != cudaSuccess) return e;
         if ((e = cudaGraphLaunch(s->exec[s->variant], s->stream)) != cudaSuccess) return e;
     } else {
-        enqueue_batch_work(srv, s, lc, false, n_slots, n_tiles, (int)s->batch.size(),
+        enqueue_batch_work(srv, s, lc, false, n_slots, n_tiles, n_cells, (int)s->batch.size(),
                            view_table_bytes((int)s->batch.size()), n_units);
     }
     long long pix = 0;

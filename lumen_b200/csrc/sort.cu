@@ -1,15 +1,13 @@
 /*
- * sort.cu - stable LSD radix sort of (key, value) pairs on the device, and
- * the per-tile ranges.
+ * sort.cu - stable LSD radix sort of (key, value) pairs on the device.
  *
  * Reference: radix_sort_64bit, src/raster/radix_sort.mojo:39-87 (eight
- * stable 8-bit LSD passes with 256 buckets), and
- * TileRangeIndex.build_from_sorted_keys, src/raster/binning.mojo:51-73.
+ * stable 8-bit LSD passes with 256 buckets).
  *
  * B200 design (onesweep, Adinets & Merrill 2022), for 32- or 64-bit keys:
  *  - one histogram pass reads the keys once and counts every digit that
- *    varies (the frame's tile sort needs none: the emission that writes the
- *    tile ids counts them). A digit is constant when no two keys differ in
+ *    varies (the frame's cell sort needs none: the emission that writes the
+ *    cell ids counts them). A digit is constant when no two keys differ in
  *    that byte (the OR of all keys and the OR of all complemented keys,
  *    gathered by the kernel that produced them, tell which); a pass over a
  *    constant digit leaves a stable sort unchanged, so it is skipped on the
@@ -23,12 +21,6 @@
  *    written out in digit runs.
  *  - every wait on another CTA's descriptor is bounded.
  * Per pass and pair: (sizeof key + 4) B read and written.
- *
- * Tile ranges: the frame's tile sort leaves its ids in final order in the
- * pass over the highest varying byte, which writes each tile's range from
- * the edges of the runs of equal ids in its pass tiles (atomic minimum of
- * the run starts, maximum of the run ends); a small kernel then counts the
- * touched tiles and finds each view's first instance from the ranges.
  */
 #include "splat_common.cuh"
 
@@ -48,7 +40,7 @@ __device__ __forceinline__ long long sort_count(const SortControl* c, long long 
 }
 
 /* Histogram of every varying digit; clears the look-back regions of the
- * passes that will run; optionally fills the tile ranges with -1.
+ * passes that will run.
  *
  * Each thread counts runs of kRun consecutive keys: equal digits in a row
  * are summed in a register and added to the warp's shared histogram once
@@ -58,7 +50,7 @@ __device__ __forceinline__ long long sort_count(const SortControl* c, long long 
 template <typename KeyT>
 __global__ void __launch_bounds__(256)
 histogram_kernel(const KeyT* __restrict__ keys, long long capacity, SortControl* sc, unsigned int* lb,
-                 long long lb_tiles_cap, int tile_keys, int* ranges, const long long* n_range_tiles) {
+                 long long lb_tiles_cap, int tile_keys) {
     chain_begin();
     constexpr int kBytes = (int)sizeof(KeyT);
     constexpr int kRun = kBytes == 8 ? 8 : 16;           /* 64 bytes of keys per thread and run */
@@ -122,13 +114,11 @@ histogram_kernel(const KeyT* __restrict__ keys, long long capacity, SortControl*
         const long long tiles = (K + tile_keys - 1) / tile_keys;
         for (int d = 0; d < kBytes; ++d) {
             if (!(varying & (1u << d))) continue;
-            unsigned int* region = lb + (size_t)d * (size_t)lb_tiles_cap * 256;
+            unsigned int* region = lb + (size_t)d * (size_t)lookback_rows(lb_tiles_cap) * 256;
             for (long long j = gtid; j < tiles * 256; j += nthreads) region[j] = 0u;
+            const long long groups = (tiles + kLookbackGroup - 1) / kLookbackGroup;
+            for (long long j = gtid; j < groups * 256; j += nthreads) region[lb_tiles_cap * 256 + j] = 0u;
         }
-    }
-    if (ranges) {
-        const long long n_range_ints = 2 * *n_range_tiles;
-        for (long long j = gtid; j < n_range_ints; j += nthreads) ranges[j] = -1;
     }
     if (blockIdx.x == 0 && tid == 0) {
         sc->varying = varying;
@@ -149,41 +139,72 @@ struct PassSmem {
     unsigned int tile;
 };
 
-/* Sum over earlier tiles of digit t's count, walking back until a tile with
- * an inclusive prefix is found. The descriptors are read kLookbackWindow at
- * a time (independent loads, one round trip per window): when every CTA
- * starts at once, tile k's walk is about k/2 tiles long. A descriptor not
- * yet published stops the window; the walk resumes from it. Wider windows
- * measured slower (more loads per step than the walks save). */
+/* Sum over earlier tiles of digit t's count. Within the tile's group of 16
+ * the tiles' rows are walked back; beyond, a group is one step: its last
+ * tile's row if that is inclusive by now, or else its sum, to which every tile
+ * has added its count (and 1 in the upper bits: complete at 16). A walk over
+ * every earlier tile, when all resident CTAs start at once, reads about half
+ * a row per pair of tiles, 100 MB for 444 tiles, which bound the passes. The
+ * rows are read kLookbackWindow at a time (independent loads); one that is
+ * not there yet stops the window, and the walk resumes from it. */
 constexpr int kLookbackWindow = 4;
+constexpr unsigned int kGroupOne = 1u << 20;   /* 16 tiles of at most 6144 keys stay below */
 
-__device__ __forceinline__ unsigned int lookback_digit(const unsigned int* lb, int tile, int t, unsigned int* err) {
+__device__ __forceinline__ unsigned int lookback_digit(const unsigned int* lb, const unsigned int* groups, int tile,
+                                                       int t, unsigned int* err) {
     unsigned int excl = 0;
-    int j = tile - 1;
     int spins = 0;
-    while (j >= 0) {
+    const int g0 = tile / kLookbackGroup;
+    for (int j = tile - 1; j >= g0 * kLookbackGroup;) {
         unsigned int d[kLookbackWindow];
 #pragma unroll
         for (int w = 0; w < kLookbackWindow; ++w)
-            d[w] = j - w >= 0 ? ld_volatile_u32(lb + (size_t)(j - w) * 256 + t) : 0u;
-        bool done = false, stalled = false;
+            d[w] = j - w >= g0 * kLookbackGroup ? ld_volatile_u32(lb + (size_t)(j - w) * 256 + t) : 0u;
+        bool stalled = false;
 #pragma unroll
         for (int w = 0; w < kLookbackWindow; ++w) {
-            if (done || stalled) continue;
+            if (stalled || j < g0 * kLookbackGroup) continue;
             const unsigned int v = d[w];
             if (!(v >> 30)) {
                 stalled = true;
             } else {
                 excl += v & kDescMask32;
+                if ((v >> 30) == 2) return excl;
                 --j;
-                if ((v >> 30) == 2) done = true;
             }
         }
-        if (done) break;
         if (stalled) {
             if (++spins >= kSpinLimit) {
                 atomicOr(err, LUMEN_GPU_ERR_SPIN_TIMEOUT);
-                break;
+                return excl;
+            }
+            __nanosleep(32);
+        }
+    }
+    for (int g = g0 - 1; g >= 0;) {
+        unsigned int last[kLookbackWindow], sum[kLookbackWindow];
+#pragma unroll
+        for (int w = 0; w < kLookbackWindow; ++w) {
+            const int gw = g - w;
+            last[w] = gw >= 0 ? ld_volatile_u32(lb + ((size_t)gw * kLookbackGroup + kLookbackGroup - 1) * 256 + t) : 0u;
+            sum[w] = gw >= 0 ? ld_volatile_u32(groups + (size_t)gw * 256 + t) : 0u;
+        }
+        bool stalled = false;
+#pragma unroll
+        for (int w = 0; w < kLookbackWindow; ++w) {
+            if (stalled || g < 0) continue;
+            if ((last[w] >> 30) == 2) return excl + (last[w] & kDescMask32);
+            if (sum[w] / kGroupOne == (unsigned int)kLookbackGroup) {
+                excl += sum[w] % kGroupOne;
+                --g;
+            } else {
+                stalled = true;
+            }
+        }
+        if (stalled) {
+            if (++spins >= kSpinLimit) {
+                atomicOr(err, LUMEN_GPU_ERR_SPIN_TIMEOUT);
+                return excl;
             }
             __nanosleep(32);
         }
@@ -191,41 +212,36 @@ __device__ __forceinline__ unsigned int lookback_digit(const unsigned int* lb, i
     return excl;
 }
 
-/* Where the tile sort's last digit pass writes the tile ranges
- * (binning.mojo:51-73), or ranges == nullptr for every other sort. The
- * ranges hold (-1, -1) before the sort. */
-struct TileRangeSink {
-    int* ranges;
-    const long long* n_tiles;   /* the batch's tile count (ids at or above it are a bounds error) */
-    unsigned int* done;         /* set to 1 by the pass that wrote the ranges */
+/* The frame's cell sort: its last digit pass also writes the cells' ranges
+ * (first, end) from the runs of equal cells that it sees. ctrl == nullptr for
+ * every other sort. */
+struct CellSink {
+    Control* ctrl;
+    const ViewTable* vt;
+    LumenGpuFrame frame;
 };
 
 /* Key j of a pass tile (nvalid keys, in sorted order in shared memory) went
  * to global position pos. A digit's keys go to consecutive positions, so a
- * run of equal ids inside the pass tile covers consecutive positions: the
- * tile's range starts at the smallest run start over all pass tiles and ends
- * after the largest run end (a range's -1 start is the largest unsigned
- * value, so the minimum replaces it). */
+ * run of equal cells inside the pass tile covers consecutive positions: the
+ * cell's range starts at the smallest run start over all pass tiles and ends
+ * after the largest run end (the ranges hold (-1, -1) before: -1 is the
+ * largest unsigned value, so the minimum replaces it). */
 template <typename KeyT>
-__device__ __forceinline__ void tile_range_edges(const TileRangeSink& sink, const KeyT* skeys, int j, int nvalid,
-                                                 KeyT kk, long long pos, long long n_tiles, unsigned int* err) {
-    const bool first = j == 0 || skeys[j - 1] != kk;
-    const bool last = j + 1 == nvalid || skeys[j + 1] != kk;
-    if (!first && !last) return;
-    const unsigned int t = (unsigned int)kk;
-    if ((long long)t >= n_tiles) {   /* self-check: a tile id outside the grid */
-        atomicOr(err, LUMEN_GPU_ERR_BOUNDS);
-        return;
-    }
-    if (first) atomicMin(reinterpret_cast<unsigned int*>(sink.ranges + 2 * (size_t)t), (unsigned int)pos);
-    if (last) atomicMax(sink.ranges + 2 * (size_t)t + 1, (int)(pos + 1));
+__device__ __forceinline__ void cell_edges(int* ranges, unsigned int id_mask, const KeyT* skeys, int j, int nvalid,
+                                           KeyT kk, long long pos) {
+    const unsigned int c = (unsigned int)kk & id_mask;
+    if (j == 0 || ((unsigned int)skeys[j - 1] & id_mask) != c)
+        atomicMin(reinterpret_cast<unsigned int*>(ranges + 2 * (size_t)c), (unsigned int)pos);
+    if (j + 1 == nvalid || ((unsigned int)skeys[j + 1] & id_mask) != c)
+        atomicMax(ranges + 2 * (size_t)c + 1, (int)(pos + 1));
 }
 
 /* kItems keys per thread: tiles of 256 * kItems keys. */
 template <typename KeyT, int kItems>
 __global__ void __launch_bounds__(kSortThreads, sizeof(KeyT) == 4 ? (kItems <= 8 ? 4 : kItems <= 16 ? 3 : 2) : 2)
 onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, long long capacity, SortControl* sc,
-                     unsigned int* lb_all, long long lb_tiles_cap, unsigned int* err, int digit, TileRangeSink sink) {
+                     unsigned int* lb_all, long long lb_tiles_cap, unsigned int* err, int digit, CellSink sink) {
     chain_begin();
     constexpr int kTileKeys = kSortThreads * kItems;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -248,13 +264,15 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
     const long long K = sort_count(sc, capacity);
     const long long ntiles = (K + kTileKeys - 1) / kTileKeys;
     const int shift = 8 * digit;
-    unsigned int* lb = lb_all + (size_t)digit * (size_t)lb_tiles_cap * 256;
-    /* the pass over the highest varying digit leaves the ids in their final
-     * order and writes the tile ranges from the run edges it sees in each
-     * pass tile (32-bit tile ids only) */
-    const bool emit_ranges = sizeof(KeyT) == 4 && sink.ranges != nullptr && (varying >> digit) == 1u;
-    const long long n_tiles = emit_ranges ? *sink.n_tiles : 0;
-    if (emit_ranges && blockIdx.x == 0 && tid == 0) *sink.done = 1u;
+    unsigned int* lb = lb_all + (size_t)digit * (size_t)lookback_rows(lb_tiles_cap) * 256;
+    unsigned int* groups = lb + (size_t)lb_tiles_cap * 256;
+    int* edges = nullptr;
+    unsigned int id_mask = 0xFFFFFFFFu;
+    if (sizeof(KeyT) == 4 && sink.ctrl && (varying >> digit) == 1u) {   /* the pass over the highest varying byte */
+        edges = cell_ranges(sink.frame, sink.ctrl, sink.vt);
+        if (sink.vt->hdr.total_cells <= kPackedCells) id_mask = (unsigned int)(kPackedCells - 1);
+        if (edges && blockIdx.x == 0 && tid == 0) sink.ctrl->cells_by_sort = 1u;
+    }
 
     /* global exclusive offsets of this digit's buckets */
     {
@@ -315,6 +333,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
         }
         const unsigned int count = run;
         st_volatile_u32(lb + (size_t)tile * 256 + t, (tile == 0 ? kDescIncl32 : kDescAgg32) | count);
+        atomicAdd(groups + (size_t)(tile / kLookbackGroup) * 256 + t, kGroupOne + count);
         {
             unsigned int x = count;
 #pragma unroll
@@ -366,7 +385,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
          * registers are free for a wide window of descriptors) */
         unsigned int excl = 0;
         if (tile > 0) {
-            excl = lookback_digit(lb, (int)tile, t, err);
+            excl = lookback_digit(lb, groups, (int)tile, t, err);
             st_volatile_u32(lb + (size_t)tile * 256 + t, kDescIncl32 | (excl + count));
         }
         s.gbase[t] = (long long)s.goffset[t] + (long long)excl - (long long)s.digit_start[t];
@@ -381,7 +400,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
                 const long long out = s.gbase[d] + j;
                 kout[out] = kk;
                 vout[out] = s.vals[j];
-                if (emit_ranges) tile_range_edges(sink, s.keys, j, kTileKeys, kk, out, n_tiles, err);
+                if (edges) cell_edges(edges, id_mask, s.keys, j, kTileKeys, kk, out);
             }
         } else {
             for (int j = tid; j < nvalid; j += kSortThreads) {
@@ -390,115 +409,11 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
                 const long long out = s.gbase[d] + j;
                 kout[out] = kk;
                 vout[out] = s.vals[j];
-                if (emit_ranges) tile_range_edges(sink, s.keys, j, nvalid, kk, out, n_tiles, err);
+                if (edges) cell_edges(edges, id_mask, s.keys, j, nvalid, kk, out);
             }
         }
         __syncthreads();
     }
-}
-
-/* When the tile sort's last digit pass wrote the ranges: the touched-tile
- * count and each view's first instance (the smallest range start among its
- * tiles; tile ids are view-major), from the 2 * n_tiles range entries. */
-__device__ void ranges_epilogue(ViewTable* vt, const int* ranges, Control* ctrl) {
-    const long long n_tiles = vt->hdr.total_tiles;
-    const int n_views = vt->hdr.n_views;
-    const int lane = threadIdx.x & 31;
-    const long long nthreads = (long long)gridDim.x * blockDim.x;
-    unsigned int touched = 0;
-    for (long long wb = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); wb < n_tiles; wb += nthreads) {
-        const long long t = wb + lane;
-        const bool valid = t < n_tiles;
-        /* an empty tile's start, -1, is the largest unsigned value */
-        const unsigned int start = valid ? (unsigned int)ranges[2 * (size_t)t] : 0xFFFFFFFFu;
-        touched += start != 0xFFFFFFFFu;
-        const int v = !valid ? -1 : n_views > 1 ? find_view_by_tile(vt, n_views, t) : 0;
-        const int v0 = __shfl_sync(0xffffffffu, v, 0);
-        if (__all_sync(0xffffffffu, v == v0 || v < 0)) {
-            const unsigned int m = __reduce_min_sync(0xffffffffu, start);
-            if (lane == 0 && m != 0xFFFFFFFFu)
-                atomicMin(reinterpret_cast<unsigned long long*>(&vt->view[v0].inst_begin), (unsigned long long)m);
-        } else if (start != 0xFFFFFFFFu) {
-            atomicMin(reinterpret_cast<unsigned long long*>(&vt->view[v].inst_begin), (unsigned long long)start);
-        }
-    }
-    touched = __reduce_add_sync(0xffffffffu, touched);
-    if (lane == 0 && touched) atomicAdd(&ctrl->touched_tiles, touched);
-}
-
-/* binning.mojo:51-73 in parallel, on tile-sorted 32-bit tile ids: a tile's
- * range starts where its id first appears and ends after it last appears.
- * Empty tiles keep the (-1, -1) written before the sort. When a tile-id byte
- * varies, the tile sort's last digit pass has written the ranges and this
- * kernel only finishes them (ranges_epilogue); otherwise it reads the ids:
- *
- * Each lane takes 8 consecutive ids per round (two 16-byte loads; the
- * frame's key buffers are 16-byte aligned) and its neighbours' ids come
- * from the adjacent lanes. The ids are sorted, so when the id before the
- * group equals the id after it, all eight equal it and the group holds no
- * boundary: one comparison for almost every group. */
-constexpr int kRangeIds = 8;
-
-__global__ void __launch_bounds__(256)
-tile_ranges_kernel(const unsigned int* k0, const unsigned int* k1, long long capacity, ViewTable* vt,
-                   int* ranges, Control* ctrl) {
-    chain_begin();
-    if (ctrl->ranges_by_sort) {
-        ranges_epilogue(vt, ranges, ctrl);
-        return;
-    }
-    const SortControl* sc = &ctrl->tile_sort;
-    const long long n_tiles = vt->hdr.total_tiles;
-    const int n_views = vt->hdr.n_views;
-    const long long K = sort_count(sc, capacity);
-    const unsigned int* __restrict__ keys = sc->sorted_buffer ? k1 : k0;
-    const int lane = threadIdx.x & 31;
-    const long long nthreads = (long long)gridDim.x * blockDim.x;
-    unsigned int touched = 0;
-    /* the warp's first id, so that the loop and its shuffles are warp-uniform */
-    for (long long wb = ((long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) * kRangeIds; wb < K;
-         wb += nthreads * kRangeIds) {
-        const long long i0 = wb + kRangeIds * lane;
-        unsigned int k[kRangeIds];
-        if (i0 + kRangeIds - 1 < K) {
-            const uint4 q0 = *reinterpret_cast<const uint4*>(keys + i0);
-            const uint4 q1 = *reinterpret_cast<const uint4*>(keys + i0 + 4);
-            k[0] = q0.x; k[1] = q0.y; k[2] = q0.z; k[3] = q0.w;
-            k[4] = q1.x; k[5] = q1.y; k[6] = q1.z; k[7] = q1.w;
-        } else {
-#pragma unroll
-            for (int r = 0; r < kRangeIds; ++r) k[r] = i0 + r < K ? keys[i0 + r] : 0xFFFFFFFFu;
-        }
-        const unsigned int up = __shfl_up_sync(0xffffffffu, k[kRangeIds - 1], 1);
-        const unsigned int down = __shfl_down_sync(0xffffffffu, k[0], 1);
-        if (i0 >= K) continue;
-        const unsigned int prev = lane > 0 ? up : (i0 > 0 ? keys[i0 - 1] : 0xFFFFFFFFu);
-        const unsigned int next = lane < 31 ? down : (i0 + kRangeIds < K ? keys[i0 + kRangeIds] : 0xFFFFFFFFu);
-        if (i0 > 0 && i0 + kRangeIds < K && prev == next && (long long)next < n_tiles) continue;
-#pragma unroll
-        for (int r = 0; r < kRangeIds; ++r) {
-            const long long i = i0 + r;
-            if (i >= K) break;
-            const unsigned int t = k[r];
-            if ((long long)t >= n_tiles) {   /* self-check: a tile id outside the grid */
-                atomicOr(&ctrl->error_flags, LUMEN_GPU_ERR_BOUNDS);
-                continue;
-            }
-            const unsigned int before = r == 0 ? prev : k[r - 1];
-            const unsigned int after = r == kRangeIds - 1 ? next : k[r + 1];   /* 0xFFFFFFFF past the end */
-            if (i == 0 || before != t) {
-                ranges[2 * (size_t)t] = (int)i;
-                ++touched;
-                /* the first instance of a view (tile ids are view-major) */
-                const int v = find_view_by_tile(vt, n_views, t);
-                if (i == 0 || (long long)before < vt->view[v].tile_begin) vt->view[v].inst_begin = i;
-            }
-            if (i == K - 1 || after != t) ranges[2 * (size_t)t + 1] = (int)(i + 1);
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) touched += __shfl_xor_sync(0xffffffffu, touched, o);
-    if (lane == 0 && touched) atomicAdd(&ctrl->touched_tiles, touched);
 }
 
 /* OR and OR-of-complement of n keys and the pair count, for sorts whose
@@ -530,10 +445,9 @@ key_stats_kernel(const KeyT* __restrict__ keys, long long n, SortControl* sc) {
 __global__ void sorted_keys64_kernel(const unsigned int* k0, const unsigned int* k1, const unsigned int* v0,
                                      const unsigned int* v1, const LumenSplatRecord* records, long long capacity,
                                      int key_mode, const Control* ctrl, unsigned long long* out) {
-    const SortControl* sc = &ctrl->tile_sort;
-    const long long K = sort_count(sc, capacity);
-    const unsigned int* keys = sc->sorted_buffer ? k1 : k0;
-    const unsigned int* vals = sc->sorted_buffer ? v1 : v0;
+    const long long K = (long long)ctrl->n_instances < capacity ? (long long)ctrl->n_instances : capacity;
+    const unsigned int* keys = ctrl->list_buffer ? k1 : k0;
+    const unsigned int* vals = ctrl->list_buffer ? v1 : v0;
     const long long nthreads = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < K; i += nthreads) {
         const unsigned int v = vals[i];
@@ -546,74 +460,59 @@ __global__ void sorted_keys64_kernel(const unsigned int* k0, const unsigned int*
  * once). */
 template <typename KeyT, int kItems>
 void launch_sort_impl(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, long long capacity, SortControl* sc,
-                      unsigned int* lb, long long lb_tiles_cap, int* ranges, const long long* n_range_tiles,
-                      unsigned int* err, int key_bytes, int num_sms, cudaStream_t st, bool counted = false,
-                      TileRangeSink sink = TileRangeSink{}) {
-    if (!counted)
+                      unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int key_bytes, int num_sms,
+                      cudaStream_t st, const CellSink* sink = nullptr) {
+    if (!sink)
         launch_chained(histogram_kernel<KeyT>, dim3(num_sms * 4), dim3(256), 0, st, (const KeyT*)k0, capacity, sc, lb,
-                       lb_tiles_cap, kSortThreads * kItems, ranges, n_range_tiles);
+                       lb_tiles_cap, kSortThreads * kItems);
     const size_t smem = sizeof(PassSmem<KeyT, kItems>);
     /* matches __launch_bounds__: all CTAs resident */
     const int ctas_per_sm = sizeof(KeyT) == 4 ? (kItems <= 8 ? 4 : kItems <= 16 ? 3 : 2) : 2;
     const int nd = key_bytes < (int)sizeof(KeyT) ? key_bytes : (int)sizeof(KeyT);
     for (int d = 0; d < nd; ++d)
         launch_chained(onesweep_pass_kernel<KeyT, kItems>, dim3(num_sms * ctas_per_sm), dim3(kSortThreads), smem, st,
-                       k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, d, sink);
+                       k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, d, sink ? *sink : CellSink{});
 }
 
 /* items: keys per thread of a digit pass, 8, 16 or 24 (tiles of 2048, 4096
  * or 6144 keys); lb_tiles_cap must hold ceil(capacity / (256 * items))
  * tiles. */
-void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1, long long capacity,
-                   SortControl* sc, unsigned int* lb, long long lb_tiles_cap, int* ranges,
-                   const long long* n_range_tiles, unsigned int* err, int items, int key_bytes, int num_sms,
-                   cudaStream_t st) {
+static void launch_sort_items(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1,
+                              long long capacity, SortControl* sc, unsigned int* lb, long long lb_tiles_cap,
+                              unsigned int* err, int items, int key_bytes, const CellSink* sink, int num_sms,
+                              cudaStream_t st) {
     if (items == 8)
-        launch_sort_impl<unsigned int, 8>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, ranges, n_range_tiles, err,
-                                          key_bytes, num_sms, st);
+        launch_sort_impl<unsigned int, 8>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, key_bytes, num_sms, st,
+                                          sink);
     else if (items == 24)
-        launch_sort_impl<unsigned int, 24>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, ranges, n_range_tiles,
-                                           err, key_bytes, num_sms, st);
+        launch_sort_impl<unsigned int, 24>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, key_bytes, num_sms,
+                                           st, sink);
     else
-        launch_sort_impl<unsigned int, 16>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, ranges, n_range_tiles,
-                                           err, key_bytes, num_sms, st);
+        launch_sort_impl<unsigned int, 16>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, key_bytes, num_sms,
+                                           st, sink);
 }
 
-/* The frame's tile sort when the emission has counted the digit values,
- * cleared the look-back tiles and filled the ranges with -1: the digit
- * passes only, the last of which writes the tile ranges. */
-void launch_tile_sort_counted(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1,
-                              long long capacity, Control* ctrl, ViewTable* vt, int* ranges, unsigned int* lb,
-                              long long lb_tiles_cap, int items, int key_bytes, int num_sms, cudaStream_t st) {
-    SortControl* sc = &ctrl->tile_sort;
-    unsigned int* err = &ctrl->error_flags;
-    const TileRangeSink sink{ranges, &vt->hdr.total_tiles, &ctrl->ranges_by_sort};
-    if (items == 8)
-        launch_sort_impl<unsigned int, 8>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, nullptr, nullptr, err,
-                                          key_bytes, num_sms, st, true, sink);
-    else if (items == 24)
-        launch_sort_impl<unsigned int, 24>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, nullptr, nullptr, err,
-                                           key_bytes, num_sms, st, true, sink);
-    else
-        launch_sort_impl<unsigned int, 16>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, nullptr, nullptr, err,
-                                           key_bytes, num_sms, st, true, sink);
+void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1, long long capacity,
+                   SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int items,
+                   int key_bytes, int num_sms, cudaStream_t st) {
+    launch_sort_items(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, items, key_bytes, nullptr, num_sms, st);
+}
+
+/* The frame's cell sort: the emission has counted the pairs' digits, cleared
+ * the look-back tiles and filled the cells' ranges with -1, so only the digit
+ * passes run, the last of which writes the ranges. */
+void launch_cell_sort(const LumenGpuFrame& f, Control* ctrl, const ViewTable* vt, unsigned int* lb,
+                      long long lb_tiles_cap, int items, int key_bytes, int num_sms, cudaStream_t st) {
+    const CellSink sink{ctrl, vt, f};
+    launch_sort_items(f.keys[0], f.vals[0], f.keys[1], f.vals[1], f.instance_capacity, &ctrl->cell_sort, lb,
+                      lb_tiles_cap, &ctrl->error_flags, items, key_bytes, &sink, num_sms, st);
 }
 
 void launch_sort64(unsigned long long* k0, unsigned int* v0, unsigned long long* k1, unsigned int* v1,
                    long long capacity, SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err,
                    int num_sms, cudaStream_t st) {
-    launch_sort_impl<unsigned long long, kSort64Items>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, nullptr,
-                                                       nullptr, err, 8, num_sms, st);
-}
-
-void launch_ranges(const LumenGpuFrame& f, Control* ctrl, ViewTable* vt, int num_sms, cudaStream_t st) {
-    /* the tile sort's last digit pass writes the ranges whenever a tile-id
-     * byte varies, and this launch then reads only the ranges (2 * n_tiles
-     * ints); otherwise (every id equal, or none) the ids are one run, which
-     * a grid-stride loop over num_sms * 2 CTAs reads in a few rounds */
-    const long long grid = (long long)num_sms * 2;
-    launch_chained(tile_ranges_kernel, dim3((unsigned int)grid), dim3(256), 0, st, (const unsigned int*)f.keys[0],
-                   (const unsigned int*)f.keys[1], (long long)f.instance_capacity, vt, f.ranges, ctrl);
+    launch_sort_impl<unsigned long long, kSort64Items>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, 8,
+                                                       num_sms, st);
 }
 
 void launch_key_stats64(const unsigned long long* keys, long long n, SortControl* sc, int num_sms, cudaStream_t st) {

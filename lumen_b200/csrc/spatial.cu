@@ -44,9 +44,8 @@ int device_sm_count();
 void configure_once();
 void launch_key_stats32(const unsigned int* keys, long long n, SortControl* sc, int num_sms, cudaStream_t st);
 void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1, long long capacity,
-                   SortControl* sc, unsigned int* lb, long long lb_tiles_cap, int* ranges,
-                   const long long* n_range_tiles, unsigned int* err, int items, int key_bytes, int num_sms,
-                   cudaStream_t st);
+                   SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int items,
+                   int key_bytes, int num_sms, cudaStream_t st);
 
 namespace {
 
@@ -106,7 +105,7 @@ BvhLayout make_layout(long long n) {
     B.keys1_off = align_up(B.vals0_off + (size_t)n * 4, 256);
     B.vals1_off = align_up(B.keys1_off + (size_t)n * 4, 256);
     B.lb_off = align_up(B.vals1_off + (size_t)n * 4, 256);
-    B.total = align_up(B.lb_off + (size_t)8 * (size_t)(B.sort_tiles > 0 ? B.sort_tiles : 1) * 256 * 4, 256);
+    B.total = align_up(B.lb_off + (size_t)8 * (size_t)lookback_rows(B.sort_tiles > 0 ? B.sort_tiles : 1) * 256 * 4, 256);
     return B;
 }
 
@@ -776,8 +775,7 @@ LumenStatus lumen_gpu_bvh_build(const LumenGpuGaussians* g, LumenGpuBvh* bvh, vo
     bbox_kernel<<<(unsigned int)grid, 256, 0, s>>>(g->means, n, ctrl);
     morton_kernel<<<(unsigned int)grid, 256, 0, s>>>(g->means, n, ctrl, k0, v0);
     launch_key_stats32(k0, n, &ctrl->sort, sms, s);
-    launch_sort32(k0, v0, k1, v1, n, &ctrl->sort, lb, B.sort_tiles, nullptr, nullptr, &ctrl->error_flags,
-                  kBvhSortItems, 4, sms, s);
+    launch_sort32(k0, v0, k1, v1, n, &ctrl->sort, lb, B.sort_tiles, &ctrl->error_flags, kBvhSortItems, 4, sms, s);
     for (int L0 = 0; L0 + 1 < lv.n_levels; L0 += kRefitSpan) {
         const long long blocks = (lv.count[L0] + kRefitNodes - 1) / kRefitNodes;
         bvh_levels_kernel<<<(unsigned int)blocks, kRefitThreads, 0, s>>>(g->means, g->scales, n, ctrl, v0, v1,

@@ -40,23 +40,41 @@ struct SortControl {
     unsigned int hist[8][256];           /* histograms of the varying digits */
 };
 
+/* Tiles are scanned in at most this many groups (list_scan_kernel). */
+constexpr int kTileGroups = 1024;
+
 /* Control block at the start of a frame's scratch. Zeroed by the host
- * before every frame (one cudaMemsetAsync), then owned by the kernels. */
+ * before every frame (one cudaMemsetAsync), then owned by the kernels. The
+ * fields before proj_ticket are what the host reads back. */
 struct Control {
     unsigned long long n_instances;      /* K, even if above capacity */
     unsigned int n_visible;              /* V */
-    unsigned int proj_ticket;            /* block order of the project look-back */
-    unsigned int emit_ticket;            /* block order of the emit look-back */
     unsigned int error_flags;            /* LUMEN_GPU_ERR_* */
     unsigned int touched_tiles;
+    unsigned int list_buffer;            /* 0 or 1: which of keys/vals holds the tiles' lists */
+    unsigned int tile_or, tile_or_not;   /* OR and OR-of-complement of the touched tiles' ids */
+    unsigned int depth_varying;          /* the depth sort's varying bytes and final buffer */
+    unsigned int depth_buffer;
+    unsigned int proj_ticket;            /* block order of the project look-back */
+    unsigned int cells_by_sort;          /* 1: the cell sort's last digit pass wrote the cells' ranges */
+    unsigned int emit_ticket;            /* block order of the emit look-back */
     unsigned int composite_ticket;       /* tile order of the compositor */
     unsigned int count_ticket;           /* unit order of the batch visibility count */
     unsigned int offsets_ticket;         /* tile order of the batch offset scan */
-    unsigned int ranges_by_sort;         /* 1: the tile sort's last digit pass wrote the tile ranges */
-    unsigned int pad[5];
+    unsigned int n_segments, pad[1];
+    unsigned int group_total[kTileGroups];   /* instances per group of tiles */
     SortControl depth_sort;              /* visible splats by depth key */
-    SortControl tile_sort;               /* instances by tile id */
+    SortControl cell_sort;               /* (cell, splat) pairs by cell */
 };
+
+/* A cell is a block of 4x4 tiles (fewer at the right and bottom edges). The
+ * emission writes one pair per cell that a splat's tile rectangle touches;
+ * the pairs' keys are the batch-wide cell id and, while ids fit 16 bits, the
+ * 16-bit mask of the cell's tiles (bit 4 row + column) that the rectangle
+ * covers in the upper half. With more cells the key is the id alone and the
+ * mask is formed again from the rectangle. */
+constexpr int kCellSide = 4;
+constexpr long long kPackedCells = 1ll << 16;
 
 constexpr int kProjThreads = 128;   /* Gaussians per projection block (a view's slots are a multiple) */
 constexpr int kEmitThreads = 256;   /* splats per emission block */
@@ -67,11 +85,18 @@ constexpr int kSortTileMin = kSortThreads * 8;         /* the smallest tile a di
 constexpr int kSort64Items = 16;                       /* keys per thread of the 64-bit pair sort */
 constexpr int kSort64Tile = kSortThreads * kSort64Items;
 
+/* A digit pass' look-back rows (256 u32 each): one per key tile and, after
+ * those, one per group of 16 tiles. */
+constexpr int kLookbackGroup = 16;
+__host__ __device__ constexpr inline int64_t lookback_rows(int64_t tiles) {
+    return tiles + (tiles + kLookbackGroup - 1) / kLookbackGroup;
+}
+
 /* Launch parameters an autotuner may choose; none of them changes a result. */
 struct LaunchConfig {
     int composite_chunk;   /* instances staged per compositing round: 128, 256 or 512 */
     int depth_sort_items;  /* keys per thread in a depth-sort digit pass: 8 or 16 */
-    int tile_sort_items;   /* keys per thread in a tile-sort digit pass: 8, 16 or 24 */
+    int tile_sort_items;   /* keys per thread in a cell-sort digit pass: 8, 16 or 24 */
     int track;             /* 1: some view's image asks for contributor counts or last-visited
                               offsets (the compositor then keeps them); set by the host */
 };
@@ -102,8 +127,9 @@ struct DevCamera {
  * batch of one. Projection treats the batch as consecutive 128-Gaussian
  * blocks (block_begin: the view's first block; its Gaussian i has slot
  * block_begin * 128 + i), and tiles get batch-wide ids (tile_begin: the
- * global id of the view's tile 0), so one sort orders every view at once:
- * the tile-id key carries the view in its high part. */
+ * global id of the view's tile 0) and cells batch-wide ids (cell_begin), so
+ * one sort orders every view at once: the cell id carries the view in its
+ * high part. */
 struct ViewDesc {
     LumenGpuGaussians g;
     LumenViewCamera cam;
@@ -111,13 +137,16 @@ struct ViewDesc {
     LumenGpuImage img;
     long long block_begin;
     long long tile_begin;
+    long long cell_begin;     /* batch-wide id of the view's cell 0 */
     long long inst_begin;     /* first tile-sorted instance of the view, or -1
-                                 (written on the device by the range pass) */
+                                 (written on the device by the list scan) */
     long long unit_begin;     /* batch projection: the first unit of the view's scene group
                                  when the view leads the group (units of the views before it
                                  otherwise, so the view owns none) */
     int group_next;           /* the next view of the same scene, or -1 */
     int group_lead;           /* 1: the first view of its scene in the batch */
+    int cells_x;
+    int reserved0;
     DevCamera dcam;           /* derived from cam on the device before projection */
 };
 
@@ -126,6 +155,7 @@ struct BatchHeader {
     int reserved0;
     long long total_blocks;   /* projection blocks of all views */
     long long total_tiles;    /* tiles of all views */
+    long long total_cells;    /* cells of all views */
     long long total_units;    /* batch projection: blocks of the batch's distinct scenes */
 };
 
@@ -141,9 +171,9 @@ __host__ __device__ constexpr inline size_t view_table_bytes(int max_views) {
 
 /* Scratch layout: [Control][project look-back: u64 per block][emit
  * look-back: u64 per block][view table][depth-sort look-back: 4 passes x
- * 2048-key tiles x 256 x u32][tile-sort look-back: 8 passes x 4096-key tiles
+ * 2048-key tiles x 256 x u32][cell-sort look-back: 8 passes x 4096-key tiles
  * x 256 x u32, which is also 4 passes x 2048-key tiles (8 passes for the
- * standalone 64-bit pair sort)]. n counts projection slots (the Gaussians
+ * standalone 64-bit pair sort)]; look-back regions hold lookback_rows(). n counts projection slots (the Gaussians
  * of all views, each view rounded up to a multiple of kProjThreads). The
  * emit look-back uses at most as many entries as the project look-back. */
 struct ScratchLayout {
@@ -159,8 +189,9 @@ struct ScratchLayout {
         L.emit_lb_off = align_up(L.proj_lb_off + (size_t)L.proj_blocks * sizeof(unsigned long long), 256);
         L.table_off = align_up(L.emit_lb_off + (size_t)L.proj_blocks * sizeof(unsigned long long), 256);
         L.depth_lb_off = align_up(L.table_off + view_table_bytes(max_views), 256);
-        L.tile_lb_off = align_up(L.depth_lb_off + (size_t)4 * (size_t)L.depth_tiles * 256 * sizeof(unsigned int), 256);
-        L.total = align_up(L.tile_lb_off + (size_t)8 * (size_t)L.sort_tiles * 256 * sizeof(unsigned int), 256);
+        L.tile_lb_off = align_up(L.depth_lb_off + (size_t)4 * (size_t)lookback_rows(L.depth_tiles) * 256 * sizeof(unsigned int), 256);
+        L.total = align_up(L.tile_lb_off + (size_t)8 * (size_t)(lookback_rows(L.sort_tiles) + 1) * 256 * sizeof(unsigned int),
+                           256);
         return L;
     }
     /* bytes zeroed before a frame: control and both scans */
@@ -193,6 +224,18 @@ inline long long assign_scene_groups(ViewDesc* v, int n) {
     return units;
 }
 
+/* Where a frame's cell ranges (first, end; 2 n_cells ints) are kept between
+ * the cell sort and the tiles' lists: the depth keys' buffer that the depth
+ * sort left unsorted, which nothing reads after the emission, when it is long
+ * enough (it has an entry per Gaussian of every view); otherwise nullptr. */
+__device__ __forceinline__ int* cell_ranges(const LumenGpuFrame& f, const Control* ctrl, const ViewTable* vt) {
+    if (2 * vt->hdr.total_cells > (vt->hdr.total_blocks - 1) * kProjThreads) return nullptr;
+    return reinterpret_cast<int*>(ctrl->depth_sort.sorted_buffer ? f.depth_keys[0] : f.depth_keys[1]);
+}
+
+/* A view's cells. */
+__host__ __device__ inline int cells_along(int tiles) { return (tiles + kCellSide - 1) / kCellSide; }
+
 /* Tile rectangle of a visible splat and its view: 12 bits per bound (tile
  * coordinates below 4096, images up to 65520 pixels a side), view in the
  * top 16 bits. */
@@ -209,6 +252,16 @@ __host__ __device__ inline int rect_min_ty(unsigned long long r) { return (int)(
 __host__ __device__ inline int rect_max_tx(unsigned long long r) { return (int)((r >> 24) & 0xFFF); }
 __host__ __device__ inline int rect_max_ty(unsigned long long r) { return (int)((r >> 36) & 0xFFF); }
 __host__ __device__ inline int rect_view(unsigned long long r) { return (int)(r >> 48); }
+
+/* The mask of the tiles of the cell whose first tile is (x, y) that the
+ * rectangle covers (it touches the cell). */
+__device__ __forceinline__ unsigned int cell_mask(unsigned long long rect, int x, int y) {
+    const int x0 = max(rect_min_tx(rect) - x, 0), x1 = min(rect_max_tx(rect) - x, kCellSide - 1);
+    const int y0 = max(rect_min_ty(rect) - y, 0), y1 = min(rect_max_ty(rect) - y, kCellSide - 1);
+    const unsigned int columns = (0xFu >> (3 - x1)) & (0xFu << x0);
+    const unsigned int rows = (0xFFFFu >> (4 * (3 - y1))) & (0xFFFFu << (4 * y0));
+    return (columns * 0x1111u) & rows;
+}
 
 /* The view whose [begin, next begin) holds x: the last view with begin <= x
  * (views with no blocks or tiles are skipped over). */
@@ -227,6 +280,14 @@ __device__ __forceinline__ int find_view_by_unit(const ViewTable* vt, int n_view
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (vt->view[mid].unit_begin <= u) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+__device__ __forceinline__ int find_view_by_cell(const ViewTable* vt, int n_views, long long cell) {
+    int lo = 0, hi = n_views - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (vt->view[mid].cell_begin <= cell) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
@@ -618,6 +679,53 @@ __device__ __forceinline__ unsigned long long lookback64(const unsigned long lon
         base -= 32;
     }
     return excl;
+}
+
+/* The emission's sums, two in one word: the tile instances
+ * (bits 31..61) and the cell pairs (bits 0..30), each saturating at 2^30 (the
+ * instance capacity is below that, and there are at most as many pairs as
+ * instances). */
+constexpr unsigned int kSaturated = 1u << 30;
+__host__ __device__ constexpr unsigned long long pack_counts(unsigned int tiles, unsigned int pairs) {
+    return ((unsigned long long)tiles << 31) | pairs;
+}
+
+__device__ __forceinline__ unsigned long long add_counts(unsigned long long a, unsigned long long b) {
+    const unsigned int t = (unsigned int)(a >> 31 & 0x7FFFFFFFu) + (unsigned int)(b >> 31 & 0x7FFFFFFFu);
+    const unsigned int p = (unsigned int)(a & 0x7FFFFFFFu) + (unsigned int)(b & 0x7FFFFFFFu);
+    return pack_counts(min(t, kSaturated), min(p, kSaturated));
+}
+
+/* The sum of all descriptors before blk; called by one full warp, 32
+ * descriptors per step. */
+__device__ __forceinline__ unsigned long long lookback_counts(const unsigned long long* desc, int blk,
+                                                              unsigned int* err) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long sum = 0ull;
+    for (int base = blk - 1; base >= 0; base -= 32) {
+        const int idx = base - lane;
+        unsigned long long v = kDescIncl64;   /* before block 0: inclusive 0 */
+        if (idx >= 0) {
+            for (int spins = 0;;) {
+                v = ld_volatile_u64(desc + idx);
+                if (v >> 62) break;
+                if (++spins >= kSpinLimit) {
+                    atomicOr(err, LUMEN_GPU_ERR_SPIN_TIMEOUT);
+                    v = kDescIncl64;
+                    break;
+                }
+                __nanosleep(32);
+            }
+        }
+        __syncwarp();
+        const unsigned int incl = __ballot_sync(0xffffffffu, (v >> 62) == 2);
+        unsigned long long mine = incl && lane > __ffs(incl) - 1 ? 0ull : v & kDescMask64;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mine = add_counts(mine, __shfl_xor_sync(0xffffffffu, mine, o));
+        sum = add_counts(sum, mine);
+        if (incl) break;
+    }
+    return sum;
 }
 
 /* Block-wide exclusive scan of one value per thread (kThreads threads). */
