@@ -416,6 +416,186 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
     }
 }
 
+/* A whole sort of up to 131072 keys in one launch, by one cluster of CTAs.
+ * Each CTA holds an equal run of the keys and runs a pass as above, but the
+ * digit counts of the CTAs before it come from their shared memory (a cluster
+ * barrier instead of descriptors to wait for), and the next pass starts at a
+ * cluster barrier instead of a launch. The pairs move between the CTAs through
+ * the L2.
+ *
+ * A sort of so few keys is bound by latency: with the histogram and a launch
+ * per digit, most of it went to launches (2.5 us each on the device, 4 us to
+ * issue) and the passes' fixed 7 to 10 us. The sort of the depth keys, before
+ * and after: 512 splats 27 -> 11 us, 50 k 34 -> 22, 100 k 40 -> 30, and four
+ * launches fewer. Eight CTAs is the largest portable cluster and 16 keys per
+ * thread what the shared memory holds, hence the limit; up to 1024 keys one
+ * CTA does. */
+constexpr int kClusterThreads = 1024;
+constexpr int kClusterItems = 16;
+constexpr int kClusterCtas = 8;
+constexpr int kClusterKeys = kClusterThreads * kClusterItems;   /* per CTA */
+constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kCountParts = kClusterThreads / 256;
+
+struct ClusterSmem {
+    unsigned int keys[kClusterKeys], vals[kClusterKeys];
+    unsigned int whist[kClusterWarps][256];
+    unsigned int match[kClusterWarps][256];
+    unsigned int part[kCountParts][256];
+    unsigned int count[256];          /* the CTA's digit counts, read by the whole cluster */
+    unsigned int digit_start[256];
+    unsigned int gbase[256];
+    unsigned int warp_sums[8];
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+/* The word at p of the cluster's CTA rank. */
+__device__ __forceinline__ unsigned int cluster_read(const unsigned int* p, unsigned int rank) {
+    unsigned int addr = (unsigned int)__cvta_generic_to_shared(p), v;
+    asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(addr) : "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+/* Exclusive scan of x over threads 0 to 255 (the other threads only keep the
+ * barriers). */
+__device__ __forceinline__ unsigned int digit_scan(unsigned int x, unsigned int* warp_sums) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned int incl = x;
+    if (warp < 8) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) warp_sums[warp] = incl;
+    }
+    __syncthreads();
+    if (warp < 8)
+        for (int w = 0; w < warp; ++w) incl += warp_sums[w];
+    return incl - x;
+}
+
+__global__ void __launch_bounds__(kClusterThreads, 1)
+cluster_sort_kernel(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1, long long capacity,
+                    SortControl* sc) {
+    chain_begin();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    ClusterSmem& s = *reinterpret_cast<ClusterSmem*>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned int rank, ctas;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+    const int K = (int)sort_count(sc, capacity);   /* at most ctas * kClusterKeys */
+    const unsigned int varying = K > 1 ? varying_digits(sc, 4) : 0u;
+    if (rank == 0 && tid == 0) {
+        sc->varying = varying;
+        sc->sorted_buffer = (unsigned int)(__popc(varying) & 1);
+    }
+    const int items = (K + (int)ctas * kClusterThreads - 1) / ((int)ctas * kClusterThreads);
+    const int base = (int)rank * items * kClusterThreads;
+    const int nvalid = min(max(K - base, 0), items * kClusterThreads);
+    const int wbase = base + warp * items * 32;   /* warp w owns items * 32 consecutive keys */
+    const unsigned int *kin = k0, *vin = v0;
+    unsigned int *kout = k1, *vout = v1;
+    for (int shift = 0; shift < 32; shift += 8) {
+        if (!(varying & (1u << (shift / 8)))) continue;
+        unsigned int k[kClusterItems], v[kClusterItems];
+#pragma unroll
+        for (int it = 0; it < kClusterItems; ++it) {
+            const int i = wbase + it * 32 + lane;
+            const bool valid = it < items && i < K;
+            k[it] = valid ? __ldcg(kin + i) : 0u;
+            v[it] = valid ? __ldcg(vin + i) : 0u;
+        }
+        for (int b = lane; b < 256; b += 32) {
+            s.whist[warp][b] = 0u;
+            s.match[warp][b] = 0u;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int it = 0; it < kClusterItems; ++it)
+            if (it < items && wbase + it * 32 + lane < K) atomicAdd(&s.whist[warp][(k[it] >> shift) & 0xFFu], 1u);
+        __syncthreads();
+        /* digit t's warp-exclusive offsets, eight warps per thread */
+        const int t = tid & 255, part = tid >> 8;
+        unsigned int run = 0u, n[kClusterWarps / kCountParts];
+#pragma unroll
+        for (int w = 0; w < kClusterWarps / kCountParts; ++w) {
+            n[w] = s.whist[part * (kClusterWarps / kCountParts) + w][t];
+            run += n[w];
+        }
+        s.part[part][t] = run;
+        __syncthreads();
+        unsigned int before = 0u, count = 0u;
+#pragma unroll
+        for (int p = 0; p < kCountParts; ++p) {
+            const unsigned int x = s.part[p][t];
+            if (p < part) before += x;
+            count += x;
+        }
+#pragma unroll
+        for (int w = 0; w < kClusterWarps / kCountParts; ++w) {
+            s.whist[part * (kClusterWarps / kCountParts) + w][t] = before;
+            before += n[w];
+        }
+        if (part == 0) s.count[t] = count;
+        cluster_arrive();   /* the counts are there once every CTA has arrived */
+        const unsigned int start = digit_scan(count, s.warp_sums);
+        if (part == 0) s.digit_start[t] = start;
+        __syncthreads();
+        /* the warp-level multisplit of the digit pass, with one set of masks */
+#pragma unroll
+        for (int it = 0; it < kClusterItems; ++it) {
+            if (it >= items) break;
+            const bool valid = wbase + it * 32 + lane < K;
+            const unsigned int d = (k[it] >> shift) & 0xFFu;
+            if (valid) atomicOr(&s.match[warp][d], 1u << lane);
+            __syncwarp();
+            const unsigned int peers = valid ? s.match[warp][d] : 0u;
+            const unsigned int prior = valid ? s.whist[warp][d] : 0u;
+            __syncwarp();
+            if (valid) {
+                if (lane == __ffs(peers) - 1) {
+                    s.whist[warp][d] = prior + __popc(peers);
+                    s.match[warp][d] = 0u;
+                }
+                const unsigned int pos = s.digit_start[d] + prior + __popc(peers & lanemask_lt());
+                s.keys[pos] = k[it];
+                s.vals[pos] = v[it];
+            }
+            __syncwarp();
+        }
+        cluster_wait();
+        /* digit t's place among all keys, less its place in the CTA's */
+        unsigned int total = 0u, earlier = 0u;
+        if (part == 0)
+            for (unsigned int c = 0; c < ctas; ++c) {
+                const unsigned int x = cluster_read(&s.count[t], c);
+                if (c < rank) earlier += x;
+                total += x;
+            }
+        const unsigned int first = digit_scan(total, s.warp_sums);
+        if (part == 0) s.gbase[t] = first + earlier - start;
+        __syncthreads();
+        for (int j = tid; j < nvalid; j += kClusterThreads) {
+            const unsigned int kk = s.keys[j];
+            const unsigned int out = s.gbase[(kk >> shift) & 0xFFu] + (unsigned int)j;
+            kout[out] = kk;
+            vout[out] = s.vals[j];
+        }
+        /* every pair of the pass is written, and no count is read any more */
+        cluster_arrive();
+        cluster_wait();
+        kin = kin == k0 ? k1 : k0;
+        vin = vin == v0 ? v1 : v0;
+        kout = kout == k0 ? k1 : k0;
+        vout = vout == v0 ? v1 : v0;
+    }
+}
+
 /* OR and OR-of-complement of n keys and the pair count, for sorts whose
  * keys come from the caller (lumen_gpu_sort_pairs). */
 template <typename KeyT>
@@ -495,6 +675,12 @@ static void launch_sort_items(unsigned int* k0, unsigned int* v0, unsigned int* 
 void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1, long long capacity,
                    SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int items,
                    int key_bytes, int num_sms, cudaStream_t st) {
+    if (capacity <= (long long)kClusterCtas * kClusterKeys && key_bytes >= 4) {
+        const bool one = capacity <= kClusterThreads;
+        launch_chained_cluster(cluster_sort_kernel, one ? 1 : kClusterCtas, dim3(one ? 1 : kClusterCtas),
+                               dim3(kClusterThreads), sizeof(ClusterSmem), st, k0, v0, k1, v1, capacity, sc);
+        return;
+    }
     launch_sort_items(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, items, key_bytes, nullptr, num_sms, st);
 }
 
@@ -530,6 +716,7 @@ void launch_sorted_keys64(const LumenGpuFrame& f, const Control* ctrl, int key_m
 }
 
 void configure_sort_kernels() {
+    cudaFuncSetAttribute(cluster_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterSmem));
     cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(PassSmem<unsigned int, 8>));
     cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
