@@ -423,7 +423,7 @@ composite_backward_kernel(const LumenSplatRecord* __restrict__ records, LumenGpu
                           const float* __restrict__ grad_alpha, float* __restrict__ grad2d, float minus_one) {
     chain_begin();
     __shared__ BackwardSmem<kDepth> s;
-    const int tile = blockIdx.x;
+    const int tile = (int)tile_in_line(ctrl, blockIdx.x);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = tile % tiles_x, ty = tile / tiles_x;
     /* the compositor's pixels: a lane's two are one above the other */

@@ -55,12 +55,6 @@ __device__ __forceinline__ unsigned char to_byte(float c) {
 constexpr int kVoteGroup = 4;
 constexpr int kCompositeThreads = 128;
 
-/* Resident CTAs per SM the compositor is compiled for (72 registers per
- * thread). 6, 7, 8 and 9 take 0.154, 0.152, 0.152 and 0.163 ms for 1 M
- * Gaussians at 1080p and 0.105, 0.112, 0.116 and 0.124 ms for 250 k at 720p,
- * where the longest tiles are the tail. */
-constexpr int kCompositeBlocksPerSm = 7;
-
 template <int kChunk>
 struct CompositeSmem {
     float4 geo[kChunk + 1];             /* cx, -cy, depth, opacity; slot kChunk: the padding splat */
@@ -442,12 +436,12 @@ template <int kChunk, bool kTrack>
 __global__ void __launch_bounds__(kCompositeThreads, kCompositeBlocksPerSm)
 composite_kernel(const ViewTable* __restrict__ vt, int n_views, const LumenSplatRecord* __restrict__ records,
                  LumenGpuFrame f, long long capacity, Control* __restrict__ ctrl, LumenRenderOptions opt,
-                 long long tile_offset, float t_stop, float minus_one) {
+                 long long tile_offset, bool in_line, float t_stop, float minus_one) {
     chain_begin();
     __shared__ CompositeSmem<kChunk> s;
     init_padding_splat(s);
     composite_tile<kChunk, kTrack>(s, vt, records, f, capacity, ctrl, opt, t_stop, splat2(minus_one), n_views,
-                                   tile_offset + blockIdx.x);
+                                   in_line ? tile_in_line(ctrl, blockIdx.x) : tile_offset + blockIdx.x);
 }
 
 /* Persistent form for a grid fixed in advance (a captured graph replayed
@@ -467,7 +461,8 @@ composite_persistent_kernel(const ViewTable* __restrict__ vt, const LumenSplatRe
         __syncthreads();
         const long long t = s.ticket;
         if (t >= total) break;
-        composite_tile<kChunk, kTrack>(s, vt, records, f, capacity, ctrl, opt, t_stop, splat2(minus_one), n_views, t);
+        composite_tile<kChunk, kTrack>(s, vt, records, f, capacity, ctrl, opt, t_stop, splat2(minus_one), n_views,
+                                       tile_in_line(ctrl, t));
         __syncthreads();
     }
 }
@@ -496,7 +491,7 @@ static float stop_transmittance(const LumenRenderOptions& opt) {
 
 template <int kChunk, bool kTrack>
 static void launch_composite_chunk(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
-                                   const LumenRenderOptions& opt, long long tile_offset, long long n_tiles,
+                                   const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
                                    bool persistent, int num_sms, cudaStream_t st) {
     if (persistent) {
         launch_chained(composite_persistent_kernel<kChunk, kTrack>, dim3(kCompositeBlocksPerSm * num_sms),
@@ -506,18 +501,18 @@ static void launch_composite_chunk(const ViewTable* vt, int n_views, const Lumen
     } else {
         launch_chained(composite_kernel<kChunk, kTrack>, dim3((unsigned int)n_tiles), dim3(kCompositeThreads), 0, st, vt,
                        n_views, (const LumenSplatRecord*)f.records, f, (long long)f.instance_capacity, ctrl, opt,
-                       tile_offset, stop_transmittance(opt), -1.0f);
+                       tile_offset, whole, stop_transmittance(opt), -1.0f);
     }
 }
 
 template <int kChunk>
 static void launch_composite_track(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
-                                   const LumenRenderOptions& opt, long long tile_offset, long long n_tiles,
+                                   const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
                                    bool persistent, bool track, int num_sms, cudaStream_t st) {
     if (track)
-        launch_composite_chunk<kChunk, true>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, persistent, num_sms, st);
+        launch_composite_chunk<kChunk, true>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, num_sms, st);
     else
-        launch_composite_chunk<kChunk, false>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, persistent, num_sms, st);
+        launch_composite_chunk<kChunk, false>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, num_sms, st);
 }
 
 /* chunk: instances staged per round, one of kCompositeChunks. Plain
@@ -525,20 +520,26 @@ static void launch_composite_track(const ViewTable* vt, int n_views, const Lumen
  * persistent launches take every tile of the table by ticket. track: some
  * view's image asks for contributor counts or last-visited offsets. */
 void launch_composite(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
-                      const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool persistent,
+                      const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole, bool persistent,
                       int chunk, bool track, int num_sms, cudaStream_t st) {
     if (n_tiles <= 0) return;
+    /* Not chained: blocks that are resident before the list kernel ends are
+     * placed where that leaves room, so the first (longest) tiles crowd on a
+     * few SMs. Launched after it, they spread over all: 100 k splats at
+     * 999x563 74 -> 58 us without an order, 79 -> 40 with one; 50 k at 640x480
+     * the whole frame 110 -> 98.5 us. */
+    ChainedLaunches chained(false);
     switch (chunk) {
         case 128:
-            launch_composite_track<128>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, persistent, track, num_sms,
+            launch_composite_track<128>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, track, num_sms,
                                         st);
             break;
         case 512:
-            launch_composite_track<512>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, persistent, track, num_sms,
+            launch_composite_track<512>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, track, num_sms,
                                         st);
             break;
         default:
-            launch_composite_track<256>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, persistent, track, num_sms,
+            launch_composite_track<256>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, track, num_sms,
                                         st);
             break;
     }

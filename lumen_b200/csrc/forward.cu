@@ -20,7 +20,6 @@
  * Passes whose digit is constant exit at once (decided on the device).
  */
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -44,9 +43,8 @@ void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigne
                    int key_bytes, int num_sms, cudaStream_t st);
 void launch_cell_sort(const LumenGpuFrame& f, Control* ctrl, const ViewTable* vt, unsigned int* lb,
                       long long lb_tiles_cap, int items, int key_bytes, int num_sms, cudaStream_t st);
-void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, void* room, long long room_bytes,
-                  long long n_cells, long long n_tiles,
-                  int num_sms, cudaStream_t st);
+void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned char* scratch, long long room_offset,
+                  long long room_bytes, long long n_cells, long long n_tiles, int num_sms, cudaStream_t st);
 void launch_sort64(unsigned long long* k0, unsigned int* v0, unsigned long long* k1, unsigned int* v1,
                    long long capacity, SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err,
                    int num_sms, cudaStream_t st);
@@ -54,7 +52,7 @@ void launch_key_stats64(const unsigned long long* keys, long long n, SortControl
 void launch_sorted_keys64(const LumenGpuFrame& f, const Control* ctrl, int key_mode, unsigned long long* out,
                           int num_sms, cudaStream_t st);
 void launch_composite(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
-                      const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool persistent,
+                      const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole, bool persistent,
                       int chunk, bool track, int num_sms, cudaStream_t st);
 void configure_sort_kernels();
 
@@ -212,10 +210,11 @@ void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRen
         cudaEventRecord(ev[1], s);
     }
     if (ev) cudaEventRecord(ev[2], s);
-    launch_lists(vt, f, ctrl, cell_lb, (long long)(L.total - L.tile_lb_off), n_cells, n_tiles, sms, s);
+    launch_lists(vt, f, ctrl, base, (long long)L.tile_lb_off, (long long)(L.total - L.tile_lb_off),
+                 n_cells, n_tiles, sms, s);
     if (ev) cudaEventRecord(ev[3], s);
     if (!with_composite) return;
-    launch_composite(vt, n_views, f, ctrl, opt, 0, n_tiles, persistent, lc.composite_chunk, lc.track != 0, sms, s);
+    launch_composite(vt, n_views, f, ctrl, opt, 0, n_tiles, true, persistent, lc.composite_chunk, lc.track != 0, sms, s);
     if (ev) cudaEventRecord(ev[4], s);
 }
 
@@ -315,7 +314,7 @@ LumenStatus forward_banded(const LumenGpuGaussians* g, const LumenViewCamera* ca
     if (n_bands > tiles_y) n_bands = tiles_y;
     for (int b = 0; b < n_bands; ++b) {
         const int r0 = (int)((long long)tiles_y * b / n_bands), r1 = (int)((long long)tiles_y * (b + 1) / n_bands);
-        launch_composite(vt, 1, *f, ctrl, *opt, (long long)r0 * tiles_x, (long long)(r1 - r0) * tiles_x, false,
+        launch_composite(vt, 1, *f, ctrl, *opt, (long long)r0 * tiles_x, (long long)(r1 - r0) * tiles_x, false, false,
                          kDefaultLaunch.composite_chunk, img->n_contrib || img->last_idx, sms, s);
         const int y0 = r0 * kTile, y1 = r1 * kTile < cam->height ? r1 * kTile : cam->height;
         if (after_band) after_band(ctx, y0, y1, s);

@@ -126,10 +126,34 @@ struct Segment {
 };
 static_assert(sizeof(Segment) == 80, "16-byte aligned");
 
+/* Scratch after the cell sort: the tiles' order (u32 per tile), if there is to
+ * be one, then the segments. offset: of p in the frame's scratch. */
+struct Room {
+    unsigned char* p;
+    long long bytes, offset;
+    long long order_min, order_max;   /* frames of so many tiles get an order */
+};
+
+__device__ __forceinline__ bool has_order(const Room& room, const ViewTable* vt) {
+    const long long n = vt->hdr.total_tiles;
+    return n >= room.order_min && n <= room.order_max && n * 4 <= room.bytes;
+}
+
 struct SegmentRoom {
     Segment* p;
     long long n;
 };
+
+__device__ __forceinline__ SegmentRoom segment_room(const Room& room, const ViewTable* vt) {
+    const long long order = has_order(room, vt) ? (vt->hdr.total_tiles * 4 + 15) / 16 * 16 : 0;
+    return {reinterpret_cast<Segment*>(room.p + order), max(room.bytes - order, 0ll) / (long long)sizeof(Segment)};
+}
+
+/* Class of a tile's list length n: higher for longer lists. */
+__device__ __forceinline__ int length_class(unsigned int n) {
+    const int log2 = 31 - __clz((int)(n | 1u));
+    return n < 2u ? (int)n : 2 * log2 + (int)((n >> (log2 - 1)) & 1u);
+}
 
 __device__ __forceinline__ bool has_room(const SegmentRoom& room, const ViewTable* vt, int n_pairs) {
     return n_pairs / kSegment + vt->hdr.total_cells <= room.n;
@@ -153,8 +177,10 @@ __device__ __forceinline__ void find_bounds(int* bounds, const SortedPairs& in, 
  * reads in flight, the next eight's before these are counted). Bound by the
  * latency of those reads (4 B per pair, once). */
 __global__ void __launch_bounds__(kCountThreads)
-list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, SegmentRoom room) {
+list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, Room scratch) {
     chain_begin();
+    const SegmentRoom room = segment_room(scratch, vt);
+    const bool order = has_order(scratch, vt);
     constexpr int kReads = kSegment / 32;
     __shared__ int bounds[2];
     __shared__ unsigned int slot_s;
@@ -221,6 +247,11 @@ list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ct
             if (t >= 0) {
                 f.ranges[2 * t + 1] = (int)base;
                 if (base) atomicAdd(&ctrl->group_total[t / group], base);
+                if (order) {
+                    const int cls = length_class(base);
+                    const unsigned int same = __match_any_sync(__activemask(), cls);
+                    if (lane == __ffs(same) - 1) atomicAdd(&ctrl->class_total[cls], (unsigned int)__popc(same));
+                }
             }
         }
         __syncthreads();
@@ -228,8 +259,9 @@ list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ct
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-list_scan_kernel(ViewTable* vt, int* __restrict__ ranges, Control* ctrl) {
+list_scan_kernel(ViewTable* vt, int* __restrict__ ranges, Control* ctrl, Room room) {
     chain_begin();
+    __shared__ unsigned int class_start[kTileClasses], class_n[kTileClasses], class_base[kTileClasses];
     __shared__ unsigned int warp_tot[kScanThreads / 32];
     __shared__ unsigned int base_s;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -239,6 +271,16 @@ list_scan_kernel(ViewTable* vt, int* __restrict__ ranges, Control* ctrl) {
         ctrl->list_buffer = ctrl->cell_sort.sorted_buffer ^ 1u;
         ctrl->depth_varying = ctrl->depth_sort.varying;
         ctrl->depth_buffer = ctrl->depth_sort.sorted_buffer;
+        if (has_order(room, vt)) ctrl->order_offset = (unsigned int)(room.offset / 256);
+    }
+    /* longest lists first: a class starts after the tiles of all higher ones */
+    unsigned int* order = has_order(room, vt) ? reinterpret_cast<unsigned int*>(room.p) : nullptr;
+    if (order) {
+        const int cls = kTileClasses - 1 - tid;
+        unsigned int all;
+        const unsigned int before = block_exclusive_scan<kScanThreads>(cls >= 0 ? ctrl->class_total[cls] : 0u, warp_tot, &all);
+        if (cls >= 0) class_start[cls] = before;
+        __syncthreads();
     }
     unsigned int touched = 0, id_or = 0, id_or_not = 0;
     for (long long g = blockIdx.x; g * group < n_tiles; g += gridDim.x) {
@@ -255,6 +297,17 @@ list_scan_kernel(ViewTable* vt, int* __restrict__ ranges, Control* ctrl) {
             if (valid) {
                 ranges[2 * t] = n ? (int)start : -1;
                 ranges[2 * t + 1] = n ? (int)(start + n) : -1;
+            }
+            if (order) {
+                if (tid < kTileClasses) class_n[tid] = 0u;
+                __syncthreads();
+                const int cls = length_class(n);
+                const unsigned int rank = valid ? atomicAdd(&class_n[cls], 1u) : 0u;
+                __syncthreads();
+                if (tid < kTileClasses && class_n[tid])
+                    class_base[tid] = class_start[tid] + atomicAdd(&ctrl->class_taken[tid], class_n[tid]);
+                __syncthreads();
+                if (valid) order[class_base[cls] + rank] = (unsigned int)t;
             }
             if (n) {
                 ++touched;
@@ -295,11 +348,13 @@ list_scan_kernel(ViewTable* vt, int* __restrict__ ranges, Control* ctrl) {
  * cell, left a tail at long lists: 9 mixed views 193 us against 35).
  * Bound by the votes' population counts (XU 52 %), issue (57 %) and the short
  * runs' partial writes: 24 warps per SM are best (64 views of 300 k: the three
- * kernels 464 us, with 32 warps 480, with 48 and segments of 128 pairs 769); a transpose and a gather in shared memory took half as many
- * instructions again (2 M at 4K: 98 against 71 us). */
+ * kernels 464 us, with 32 warps 480, with 48 and segments of 128 pairs 769); a
+ * transpose and a gather in shared memory took half as many instructions again
+ * (2 M at 4K: 98 against 71 us). */
 __global__ void __launch_bounds__(kWriteThreads, kWriteCtas)
-list_write_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, SegmentRoom room) {
+list_write_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, Room scratch) {
     chain_begin();
+    const SegmentRoom room = segment_room(scratch, vt);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const SortedPairs in = sorted_pairs(f, ctrl, vt);
     const bool noted = has_room(room, vt, in.n);
@@ -384,16 +439,25 @@ int grid_of(long long n, long long cap) { return (int)(n < 1 ? 1 : n < cap ? n :
 
 /* n_cells, n_tiles: the batch's, or upper bounds for a persistent launch
  * (the kernels read the batch's from the table; grids are strided). */
-void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, void* room, long long room_bytes,
-                  long long n_cells, long long n_tiles, int num_sms, cudaStream_t st) {
-    const SegmentRoom seg{static_cast<Segment*>(room), room_bytes / (long long)sizeof(Segment)};
+void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned char* scratch, long long room_offset,
+                  long long room_bytes, long long n_cells, long long n_tiles, int num_sms, cudaStream_t st) {
+    /* Longest lists first: a tile with a long list that starts late runs on
+     * alone. Of use from one and a half to ten tiles per resident CTA of the
+     * compositor. Compositor, in tile order and longest first: 100 k splats at
+     * 999x563 (2268 tiles) 58 -> 40 us and its adjoint 87 -> 70, 250 k at
+     * 1279x719 (3600) 113 -> 88, 1 M at 1080p (8160) 155 -> 151. With fewer (50 k
+     * at 640x480, 1200 tiles) it gains nothing and the order costs 2 us; with
+     * more, neighbouring tiles no longer share their splats in the L2 (2 M at
+     * 4K, 32400 tiles: 288 -> 301). */
+    const long long line = (long long)kCompositeBlocksPerSm * num_sms;
+    const Room room{scratch + room_offset, room_bytes, room_offset, line + line / 2, 10 * line};
     launch_chained(list_count_kernel, dim3(grid_of(n_cells, 64ll * num_sms)), dim3(kCountThreads), 0, st,
-                   (const ViewTable*)vt, f, ctrl, seg);
+                   (const ViewTable*)vt, f, ctrl, room);
     launch_chained(list_scan_kernel, dim3(grid_of((n_tiles + kScanThreads - 1) / kScanThreads, 2ll * num_sms)),
-                   dim3(kScanThreads), 0, st, vt, f.ranges, ctrl);
+                   dim3(kScanThreads), 0, st, vt, f.ranges, ctrl, room);
     const long long most = f.instance_capacity / kSegment + n_cells;   /* segments, or cells */
     launch_chained(list_write_kernel, dim3(grid_of((most + kWriteWarps - 1) / kWriteWarps, kWriteCtas * num_sms)),
-                   dim3(kWriteThreads), 0, st, (const ViewTable*)vt, f, ctrl, seg);
+                   dim3(kWriteThreads), 0, st, (const ViewTable*)vt, f, ctrl, room);
 }
 
 }  // namespace lumen

@@ -126,3 +126,15 @@ def test_emission_rounds(n):
     scene = R.Scene(*_dev([a.astype(np.float32) for a in (sc.means, s, sc.quats, op.reshape(-1), sc.sh)]))
     cams = scenes.orbit_cameras(2, 320, 180, fov=50.0, radius=10.0)
     _check_batch([(scene, c) for c in cams])
+
+
+@pytest.mark.parametrize("size", [(37 * 16, 42 * 16), (5 * 16, 311 * 16), (56 * 16, 185 * 16 - 5), (13 * 16, 797 * 16)])
+def test_tiles_in_line(size):
+    """1554 to 10360 tiles (1.5 and 10 per resident CTA of 148 SMs) are shaded longest list first."""
+    _check(_scene(3000, size[0], scale=(0.001, 0.3)), _cam(*size))
+
+
+def test_tiles_in_line_backward():
+    """The adjoint's sums over 1720 tiles, against 64-bit autograd with its bound at other sizes."""
+    from test_gpu_backward_sums import _check as check_gradients
+    check_gradients(30, (40 * 16, 43 * 16), (0.02, 0.5), 2e-4, depth=True, alpha=True, white=False)
