@@ -34,11 +34,15 @@ class _RenderFunction(torch.autograd.Function):
         opt = options.with_(params_are_logits=True)
         n = means.shape[0]
         tensors = [t.detach().contiguous().float() for t in (means, log_scales, quats, opacity_logits)]
+        logits = tensors[3].reshape(n)
         sh_flat = sh.detach().contiguous().float().reshape(n, 48)
-        res = R.render(tensors[0], tensors[1], tensors[2], tensors[3].reshape(n), sh_flat, camera, opt)
-        ctx.camera, ctx.options, ctx.frame = camera, opt, res.frame
+        # the backward pass takes the same camera and options (copies, as C structures)
+        ctx.c_camera, ctx.c_options = L.view_camera(camera), L.render_options(opt)
+        res = R._render(tensors[0], tensors[1], tensors[2], logits, sh_flat, ctx.c_camera, ctx.c_options,
+                        camera.n_tiles, opt, None, None)
+        ctx.frame = res.frame
         ctx.sh_shape = sh.shape
-        ctx.save_for_backward(tensors[0], tensors[1], tensors[2], tensors[3].reshape(n), sh_flat, res.rgb, res.depth,
+        ctx.save_for_backward(tensors[0], tensors[1], tensors[2], logits, sh_flat, res.rgb, res.depth,
                               res.alpha, res.last_idx)
         ctx.mark_non_differentiable(res.last_idx)
         ctx.set_materialize_grads(False)   # an output without a gradient passes None, not zeros to read
@@ -55,14 +59,12 @@ class _RenderFunction(torch.autograd.Function):
         if n == 0:
             return grads[0], grads[1], grads[2], grads[3], grads[4].reshape(ctx.sh_shape), None, None
         splat2d = torch.empty((n, 12), dtype=torch.float32, device=dev)
-        out = L.LumenGpuGradients()
-        out.means, out.scales, out.quats, out.opacities, out.sh = (g.data_ptr() for g in grads)
-        out.splat2d = splat2d.data_ptr()
+        out = L.LumenGpuGradients(*(g.data_ptr() for g in grads), splat2d.data_ptr())
         g = R.gaussians_struct(means, log_scales, quats, logits, sh)
-        cam, opt = L.view_camera(ctx.camera), L.render_options(ctx.options)
+        cam, opt = ctx.c_camera, ctx.c_options
         fs = ctx.frame.c_struct()
         g_rgb = g_rgb.contiguous().float() if g_rgb is not None else torch.zeros(
-            (ctx.camera.height, ctx.camera.width, 3), device=dev)
+            (cam.height, cam.width, 3), device=dev)
         g_depth = g_depth.contiguous().float() if g_depth is not None else None
         g_alpha = g_alpha.contiguous().float() if g_alpha is not None else None
         fwd = L.LumenGpuImage()
@@ -72,7 +74,7 @@ class _RenderFunction(torch.autograd.Function):
                                               g_rgb.data_ptr(),
                                               None if g_depth is None else g_depth.data_ptr(),
                                               None if g_alpha is None else g_alpha.data_ptr(), C.byref(out),
-                                              torch.cuda.current_stream(dev).cuda_stream), "render_backward")
+                                              R._stream_handle(dev)), "render_backward")
         return grads[0], grads[1], grads[2], grads[3].reshape(logits.shape), grads[4].reshape(ctx.sh_shape), None, None
 
 
@@ -93,7 +95,7 @@ class _L1Function(torch.autograd.Function):
         loss = torch.empty((), dtype=torch.float32, device=p.device)
         scratch = torch.empty(int(lib.lumen_gpu_l1_loss_scratch_bytes()), dtype=torch.uint8, device=p.device)
         L.check(lib.lumen_gpu_l1_loss(p.data_ptr(), t.data_ptr(), p.numel(), grad.data_ptr(), loss.data_ptr(),
-                                      scratch.data_ptr(), torch.cuda.current_stream(p.device).cuda_stream), "l1_loss")
+                                      scratch.data_ptr(), R._stream_handle(p.device)), "l1_loss")
         ctx.save_for_backward(grad)
         return loss
 

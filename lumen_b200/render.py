@@ -10,6 +10,7 @@ keys and values, tile ranges) for inspection.
 from __future__ import annotations
 
 import ctypes as C
+import math
 from dataclasses import dataclass
 from typing import Optional
 
@@ -26,7 +27,18 @@ def _p(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream_handle(device: torch.device) -> int:
+    if device.type == "cuda" and device.index is not None:
+        return torch._C._cuda_getCurrentRawStream(device.index)   # no Stream object is made
     return torch.cuda.current_stream(device).cuda_stream
+
+
+# Frames up to this size are one allocation, cut into tensors when they are
+# asked for: a render without a frame to reuse spends 5 us on its buffers
+# instead of 30 (14 tensors made, and freed, one by one). Larger frames keep
+# one tensor per buffer, so that holding on to one does not hold them all.
+_ONE_BUFFER_BYTES = 64 << 20
+_FRAME_TENSORS = ("records", "visible_ids", "radii", "rects", "depth_keys", "depth_order", "keys", "vals", "ranges",
+                  "scratch")
 
 
 @dataclass
@@ -51,6 +63,19 @@ class Frame:
         n1 = max(n, 1)
         scratch_bytes = int(lib.lumen_gpu_scratch_bytes(n1, capacity, tiles))
         kw = dict(device=device)
+        # one buffer: offsets of the tensors (256-byte steps), in the order of LumenGpuFrame
+        up = lambda b: (b + 255) & ~255
+        per, cap = up(4 * n1), up(4 * capacity)
+        o, offsets = 0, []
+        for b in (up(4 * RECORD_FLOATS * n1), per, per, up(8 * n1), per, per, per, per, cap, cap, cap, cap,
+                  up(8 * tiles), scratch_bytes):
+            offsets.append(o)
+            o += b
+        if o <= _ONE_BUFFER_BYTES and capacity > 0 and tiles > 0:
+            f = Frame.__new__(Frame)
+            f.capacity = capacity
+            f._one = (torch.empty(o, dtype=torch.uint8, **kw), offsets, n1, tiles, scratch_bytes)
+            return f
         i32 = lambda m: torch.empty(m, dtype=torch.int32, **kw)
         return Frame(torch.empty((n1, RECORD_FLOATS), dtype=torch.float32, **kw), i32(n1), i32(n1),
                      torch.empty(n1, dtype=torch.int64, **kw), [i32(n1), i32(n1)], [i32(n1), i32(n1)],
@@ -58,10 +83,35 @@ class Frame:
                      torch.empty((tiles, 2), dtype=torch.int32, **kw),
                      torch.empty(scratch_bytes, dtype=torch.uint8, **kw), capacity)
 
+    def __getattr__(self, name):
+        """A tensor of a one-buffer frame, on its first use."""
+        if name not in _FRAME_TENSORS or "_one" not in self.__dict__:
+            raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
+        buf, o, n, tiles, scratch_bytes = self._one
+        cut = lambda i, dtype, *shape: buf[o[i]:o[i] + math.prod(shape) * dtype.itemsize].view(dtype).view(shape)
+        i32, cap = torch.int32, self.capacity
+        made = {"records": lambda: cut(0, torch.float32, n, RECORD_FLOATS), "visible_ids": lambda: cut(1, i32, n),
+                "radii": lambda: cut(2, i32, n), "rects": lambda: cut(3, torch.int64, n),
+                "depth_keys": lambda: [cut(4, i32, n), cut(5, i32, n)],
+                "depth_order": lambda: [cut(6, i32, n), cut(7, i32, n)],
+                "keys": lambda: [cut(8, i32, cap), cut(9, i32, cap)],
+                "vals": lambda: [cut(10, i32, cap), cut(11, i32, cap)], "ranges": lambda: cut(12, i32, tiles, 2),
+                "scratch": lambda: cut(13, torch.uint8, scratch_bytes)}[name]()
+        setattr(self, name, made)
+        return made
+
     def fits(self, n: int, tiles: int) -> bool:
+        if "_one" in self.__dict__ and self.__dict__.keys().isdisjoint(_FRAME_TENSORS):
+            return self._one[2] >= max(n, 1) and self._one[3] >= tiles
         return self.records.shape[0] >= max(n, 1) and self.ranges.shape[0] >= tiles
 
     def c_struct(self) -> L.LumenGpuFrame:
+        if "_one" in self.__dict__ and self.__dict__.keys().isdisjoint(_FRAME_TENSORS):
+            buf, o, _, _, scratch_bytes = self._one
+            b, two = buf.data_ptr(), C.c_void_p * 2
+            return L.LumenGpuFrame(b, b + o[1], b + o[2], b + o[3], two(b + o[4], b + o[5]), two(b + o[6], b + o[7]),
+                                   two(b + o[8], b + o[9]), two(b + o[10], b + o[11]), self.capacity, b + o[12],
+                                   b + o[13], scratch_bytes)
         f = L.LumenGpuFrame()
         f.records, f.visible_ids, f.radii = _p(self.records), _p(self.visible_ids), _p(self.radii)
         f.rects = _p(self.rects)
@@ -126,12 +176,10 @@ def gaussians_struct(means, scales, quats, opacities, sh) -> L.LumenGpuGaussians
                            ("opacities", opacities, (n,)), ("sh", sh, (n, 48))):
         if t.dtype != torch.float32 or not t.is_cuda or not t.is_contiguous():
             raise ValueError(f"{name} must be a contiguous float32 CUDA tensor")
-        if tuple(t.reshape(shape).shape) != shape:
+        if t.shape != shape and tuple(t.reshape(shape).shape) != shape:
             raise ValueError(f"{name} has shape {tuple(t.shape)}, expected {shape}")
-    g = L.LumenGpuGaussians()
-    g.means, g.scales, g.quats, g.opacities, g.sh = _p(means), _p(scales), _p(quats), _p(opacities), _p(sh)
-    g.count = n
-    return g
+    return L.LumenGpuGaussians(means.data_ptr(), scales.data_ptr(), quats.data_ptr(), opacities.data_ptr(),
+                               sh.data_ptr(), n)
 
 
 _capacity_hint = {}
@@ -144,20 +192,26 @@ def render(means: torch.Tensor, scales: torch.Tensor, quats: torch.Tensor, opaci
     and in [0, 1] unless ``options.params_are_logits``. Waits for the frame to
     finish (it reads the instance count back to check the buffer capacity)."""
     options = options or RenderOptions()
+    return _render(means, scales, quats, opacities, sh, L.view_camera(camera), L.render_options(options), camera.n_tiles,
+                   options, frame, capacity)
+
+
+def _render(means, scales, quats, opacities, sh, cam: L.LumenViewCamera, opt: L.LumenRenderOptions, tiles: int,
+            options: RenderOptions, frame: Optional[Frame], capacity: Optional[int]) -> RenderResult:
+    """render() with the camera and the options as C structures."""
     lib = L.load()
     dev = means.device
     n = int(means.shape[0])
-    H, W = int(camera.height), int(camera.width)
-    tiles = camera.n_tiles
-    g = gaussians_struct(means, scales, quats, opacities, sh.reshape(n, 48) if n else sh.reshape(0, 48))
-    cam, opt = L.view_camera(camera), L.render_options(options)
+    H, W = cam.height, cam.width
+    if sh.shape != (n, 48):
+        sh = sh.reshape(n, 48) if n else sh.reshape(0, 48)
+    g = gaussians_struct(means, scales, quats, opacities, sh)
     rgb = torch.empty((H, W, 3), dtype=torch.float32, device=dev)
     depth = torch.empty((H, W), dtype=torch.float32, device=dev)
     alpha = torch.empty((H, W), dtype=torch.float32, device=dev)
     ncon = torch.empty((H, W), dtype=torch.int32, device=dev)
     last = torch.empty((H, W), dtype=torch.int32, device=dev)
-    img = L.LumenGpuImage()
-    img.rgb, img.depth, img.alpha, img.n_contrib, img.last_idx = _p(rgb), _p(depth), _p(alpha), _p(ncon), _p(last)
+    img = L.LumenGpuImage(rgb.data_ptr(), depth.data_ptr(), alpha.data_ptr(), ncon.data_ptr(), last.data_ptr())
     key = (n, W, H)
     if capacity is None:
         capacity = _capacity_hint.get(key, max(1 << 16, 8 * n))
