@@ -32,9 +32,8 @@ namespace lumen {
 void launch_batch_project(const ViewTable* vt, const LumenRenderOptions& opt, const LumenGpuFrame& f,
                           Control* ctrl, unsigned long long* lb, long long n_units, long long n_blocks,
                           bool persistent, int num_sms, cudaStream_t st);
-void launch_project(const ViewTable* vt, int n_views, const LumenRenderOptions& opt, const LumenGpuFrame& f,
-                    Control* ctrl, unsigned long long* lb, long long n_blocks, bool persistent, int num_sms,
-                    cudaStream_t st);
+void launch_project(const ViewTable* vt, const LumenRenderOptions& opt, const LumenGpuFrame& f, Control* ctrl,
+                    unsigned long long* lb, long long n_blocks, cudaStream_t st);
 void launch_emit(const ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned long long* lb,
                  unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys, long long n_blocks,
                  bool persistent, int num_sms, cudaStream_t st);
@@ -170,14 +169,21 @@ __global__ void frame_init_kernel(unsigned long long* zero, long long n_words, V
     }
 }
 
+/* A single view of at most so many 128-Gaussian blocks is projected by one
+ * kernel. Projection, one kernel and three: 512 Gaussians 13.3 and 19.9 us
+ * (and two launches fewer to issue), 50 k 20.8 and 22.2, 100 k 13.5 and 18.4
+ * (without the launch before); 250 k 43 and 39.6, where the look-back is the
+ * longer way. */
+constexpr long long kOnePassBlocks = 1024;
+
 /* The frame's kernels after the view table is in place. n_slots, n_tiles and
  * n_cells are the batch's (plain launches) or upper bounds (persistent
  * launches, whose kernels read the batch's sizes from the table); n_views
  * is the batch's view count, or 0 when only the table knows it; n_units
  * the projection units (plain launches). Projection is a visibility count,
  * an offset scan and the projection proper, Gaussian-major (each distinct
- * scene read once); with n_units 0 a single view instead runs the one-pass
- * kernel with its compacting scan fused in (project_kernel). */
+ * scene read once); a single view of few Gaussians runs one kernel with its
+ * compacting scan fused in (project_kernel). */
 void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRenderOptions& opt,
                      const LumenGpuFrame& f, long long n_slots, long long n_tiles, long long n_cells, int n_views,
                      bool persistent, const LaunchConfig& lc, cudaEvent_t* ev, cudaStream_t s, bool with_composite,
@@ -190,8 +196,9 @@ void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRen
     unsigned int* cell_lb = (unsigned int*)(base + L.tile_lb_off);
     const int sms = device_sm_count();
     if (n_slots > 0) {
-        if (n_views == 1 && n_units == 0)
-            launch_project(vt, n_views, opt, f, ctrl, proj_lb, L.proj_blocks, persistent, sms, s);
+        const long long n_blocks = (n_slots + kProjThreads - 1) / kProjThreads;
+        if (n_views == 1 && !persistent && n_blocks <= kOnePassBlocks)
+            launch_project(vt, opt, f, ctrl, proj_lb, n_blocks, s);
         else
             launch_batch_project(vt, opt, f, ctrl, proj_lb, n_units, L.proj_blocks, persistent, sms, s);
         if (ev) cudaEventRecord(ev[1], s);

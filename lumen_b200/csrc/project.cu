@@ -7,9 +7,9 @@
  * indices in Gaussian order (pipeline.mojo:141-149) and each appends one
  * key per covered tile (:152-157); the keys are then stably sorted (:166).
  *
- * K1: a block of 128 threads projects 128 consecutive Gaussians (their SH
- * coefficients staged in shared memory by asynchronous copies) and scans
- * their visibility flags; the global offset comes from a decoupled look-back
+ * K1, for one view of few Gaussians (below for the rest): a block of 128
+ * threads projects 128 consecutive Gaussians (their SH coefficients staged in
+ * shared memory by asynchronous copies) and scans their visibility flags; the global offset comes from a decoupled look-back
  * over blocks taken in ticket order, so visible indices are exactly the
  * reference's sequential ones. Each visible splat writes its 48-byte record,
  * its Gaussian index, its tile rectangle and its depth key.
@@ -32,144 +32,131 @@
 namespace lumen {
 
 struct ProjSmem {
-    ViewDesc vd;                 /* the block's view, copied from the table */
+    LumenGpuGaussians g;         /* the view's */
+    DevCamera cam;
     unsigned int blk;
-    int view;
     unsigned int warp_tot[kProjThreads / 32];
     unsigned long long vis_base;
     unsigned long long key_or, key_or_not;
 };
 
-constexpr int kViewWords = (int)(sizeof(ViewDesc) / 4);
-static_assert(sizeof(ViewDesc) % 4 == 0 && kViewWords <= kProjThreads - 32, "view copy layout");
+constexpr int kCamWords = (int)(sizeof(DevCamera) / 4);
+constexpr int kGaussiansWords = (int)(sizeof(LumenGpuGaussians) / 4);
+static_assert(sizeof(DevCamera) % 4 == 0 && kCamWords <= kProjThreads, "camera copy layout");
+static_assert(sizeof(LumenGpuGaussians) % 4 == 0 && kGaussiansWords <= 32, "scene copy layout");
 
-/* Each CTA takes a 128-Gaussian block by ticket (kPersistent: blocks until
- * the batch's blocks are exhausted, for a grid fixed in advance). Block b
- * belongs to the last view whose block_begin <= b, and covers that view's
- * Gaussians (b - block_begin) * 128 onward; visible indices run over the
- * whole batch in block order. n_views_hint: the batch's view count, or 0
- * to read it from the table; with one view, the view is copied to shared
- * memory while the ticket is being taken. */
-template <bool kPersistent>
+__device__ __forceinline__ void copy_camera(DevCamera& dst, const DevCamera& src) {
+    const int tid = threadIdx.x;
+    if (tid < kCamWords) reinterpret_cast<unsigned int*>(&dst)[tid] = reinterpret_cast<const unsigned int*>(&src)[tid];
+}
+
+/* The projection of one view of few Gaussians (kOnePassBlocks): each CTA takes
+ * a 128-Gaussian block by ticket, and visible indices run over the blocks in
+ * order. One launch, but the look-back is a chain: the resident CTAs start
+ * together, and sums travel 32 blocks per step of about 0.45 us. */
 __global__ void __launch_bounds__(kProjThreads)
-project_kernel(const ViewTable* __restrict__ vt, int n_views_hint, LumenRenderOptions opt, LumenGpuFrame f,
-               Control* ctrl, unsigned long long* lb) {
+project_kernel(const ViewTable* __restrict__ vt, LumenRenderOptions opt, LumenGpuFrame f, Control* ctrl,
+               unsigned long long* lb) {
     chain_begin();
     __shared__ ProjSmem s;
     extern __shared__ float4 sh_stage[];   /* kProjThreads x 12: the block's SH coefficients */
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n_views = n_views_hint > 0 ? n_views_hint : vt->hdr.n_views;
     const long long total_blocks = vt->hdr.total_blocks;
-    if (n_views == 1) {
-        if (tid >= 32 && tid < 32 + kViewWords)
-            reinterpret_cast<unsigned int*>(&s.vd)[tid - 32] = reinterpret_cast<const unsigned int*>(&vt->view[0])[tid - 32];
-        if (tid == 0) s.view = 0;
+    copy_camera(s.cam, vt->view[0].dcam);
+    if (tid >= kProjThreads - kGaussiansWords) {
+        const int w = tid - (kProjThreads - kGaussiansWords);
+        reinterpret_cast<unsigned int*>(&s.g)[w] = reinterpret_cast<const unsigned int*>(&vt->view[0].g)[w];
     }
-    for (;;) {
-        if (tid == 0) {
-            s.blk = atomicAdd(&ctrl->proj_ticket, 1u);
-            s.key_or = 0ull;
-            s.key_or_not = 0ull;
+    if (tid == 0) {
+        s.blk = atomicAdd(&ctrl->proj_ticket, 1u);
+        s.key_or = 0ull;
+        s.key_or_not = 0ull;
+    }
+    __syncthreads();
+    const int blk = (int)s.blk;
+    if ((long long)blk >= total_blocks) return;
+    const long long i0 = (long long)blk * kProjThreads, i = i0 + tid;
+    const long long count = s.g.count;
+    /* the block's SH rows (192 B per Gaussian, contiguous) go to shared
+     * memory with coalesced 16-byte asynchronous copies, overlapped with
+     * the loads of the other parameters */
+    {
+        const int nblk = (int)(count - i0 < kProjThreads ? count - i0 : kProjThreads);
+        const float4* src = reinterpret_cast<const float4*>(s.g.sh + i0 * 48);
+        for (int c = tid; c < nblk * 12; c += kProjThreads) {
+            const int t = c / 12, q = c - 12 * t;
+            cp_async16(sh_stage + 12 * t + (q ^ sh_swizzle(t)), src + c);
         }
-        __syncthreads();
-        const int blk = (int)s.blk;
-        if ((long long)blk >= total_blocks) break;
-        if (n_views > 1) {
-            if (warp == 0) {
-                const int v = find_view_by_block(vt, n_views, blk);
-                const unsigned int* src = reinterpret_cast<const unsigned int*>(&vt->view[v]);
-                for (int w = lane; w < kViewWords; w += 32) reinterpret_cast<unsigned int*>(&s.vd)[w] = src[w];
-                if (lane == 0) s.view = v;
-            }
-            __syncthreads();
-        }
-        const long long slot = (long long)blk * kProjThreads + tid;
-        const long long i0 = (long long)(blk - s.vd.block_begin) * kProjThreads;
-        const long long i = i0 + tid;
-        const long long count = s.vd.g.count;
-        /* the block's SH rows (192 B per Gaussian, contiguous) go to shared
-         * memory with coalesced 16-byte asynchronous copies, overlapped with
-         * the loads of the other parameters */
-        {
-            const int nblk = (int)(count - i0 < kProjThreads ? count - i0 : kProjThreads);
-            const float4* src = reinterpret_cast<const float4*>(s.vd.g.sh + i0 * 48);
-            for (int c = tid; c < nblk * 12; c += kProjThreads) {
-                const int t = c / 12, q = c - 12 * t;
-                cp_async16(sh_stage + 12 * t + (q ^ sh_swizzle(t)), src + c);
-            }
-            cp_async_commit();
-        }
-        float mx = 0.0f, my = 0.0f, mz = 0.0f, sx = 0.0f, sy = 0.0f, sz = 0.0f, op = 0.0f;
-        float4 q = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
-        if (i < count) {
-            const LumenGpuGaussians& g = s.vd.g;
-            const float* m = g.means + i * 3;
-            const float* sc = g.scales + i * 3;
-            q = __ldg(reinterpret_cast<const float4*>(g.quats) + i);
-            mx = __ldg(m); my = __ldg(m + 1); mz = __ldg(m + 2);
-            sx = __ldg(sc); sy = __ldg(sc + 1); sz = __ldg(sc + 2);
-            op = __ldg(g.opacities + i);
-        }
-        cp_async_wait_all();
-        __syncthreads();
+        cp_async_commit();
+    }
+    float mx = 0.0f, my = 0.0f, mz = 0.0f, sx = 0.0f, sy = 0.0f, sz = 0.0f, op = 0.0f;
+    float4 q = make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+    if (i < count) {
+        const LumenGpuGaussians& g = s.g;
+        const float* m = g.means + i * 3;
+        const float* sc = g.scales + i * 3;
+        q = __ldg(reinterpret_cast<const float4*>(g.quats) + i);
+        mx = __ldg(m); my = __ldg(m + 1); mz = __ldg(m + 2);
+        sx = __ldg(sc); sy = __ldg(sc + 1); sz = __ldg(sc + 2);
+        op = __ldg(g.opacities + i);
+    }
+    cp_async_wait_all();
+    __syncthreads();
 
-        Projected p;
-        p.visible = false;
-        p.radius = 0;
-        if (i < count) {
-            p = project_gaussian(s.vd.dcam, mx, my, mz, sx, sy, sz, Quat{q.x, q.y, q.z, q.w}, op,
-                                 reinterpret_cast<const float*>(sh_stage + tid * 12), opt, sh_swizzle(tid));
-            if (f.radii) f.radii[slot] = p.visible ? p.radius : 0;
+    Projected p;
+    p.visible = false;
+    p.radius = 0;
+    if (i < count) {
+        p = project_gaussian(s.cam, mx, my, mz, sx, sy, sz, Quat{q.x, q.y, q.z, q.w}, op,
+                             reinterpret_cast<const float*>(sh_stage + tid * 12), opt, sh_swizzle(tid));
+        if (f.radii) f.radii[i] = p.visible ? p.radius : 0;
+    }
+    unsigned int block_vis = 0;
+    const unsigned int vis_local = block_exclusive_scan<kProjThreads>(p.visible ? 1u : 0u, s.warp_tot, &block_vis);
+    if (tid == 0) st_volatile_u64(lb + blk, (blk == 0 ? kDescIncl64 : kDescAgg64) | block_vis);
+    if (warp == 0) {
+        const unsigned long long e = blk > 0 ? lookback64(lb, blk, &ctrl->error_flags) : 0ull;
+        if (lane == 0) {
+            s.vis_base = e;
+            if (blk > 0) st_volatile_u64(lb + blk, kDescIncl64 | (e + block_vis));
         }
-        unsigned int block_vis = 0;
-        const unsigned int vis_local = block_exclusive_scan<kProjThreads>(p.visible ? 1u : 0u, s.warp_tot, &block_vis);
-        if (tid == 0) st_volatile_u64(lb + blk, (blk == 0 ? kDescIncl64 : kDescAgg64) | block_vis);
-        if (warp == 0) {
-            const unsigned long long e = blk > 0 ? lookback64(lb, blk, &ctrl->error_flags) : 0ull;
-            if (lane == 0) {
-                s.vis_base = e;
-                if (blk > 0) st_volatile_u64(lb + blk, kDescIncl64 | (e + block_vis));
-            }
-        }
-        __syncthreads();
-        const unsigned long long vis_base = s.vis_base;
-        unsigned long long kor = 0ull, knot = 0ull;
-        if (p.visible) {
-            const unsigned long long vid = vis_base + vis_local;
-            float4* dst = reinterpret_cast<float4*>(f.records + vid);
-            dst[0] = make_float4(p.cx, p.cy, p.z, p.op);
-            dst[1] = make_float4(p.ic00, p.ic01, p.ic11, 0.0f);
-            dst[2] = make_float4(p.r, p.g, p.b, 0.0f);
-            f.visible_ids[vid] = (unsigned int)i;
-            f.rects[vid] = pack_rect(p.min_tx, p.min_ty, p.max_tx, p.max_ty, s.view);
-            const unsigned int dk = depth_key(p.z, opt.key_mode);
-            f.depth_keys[0][vid] = dk;
-            f.depth_order[0][vid] = (unsigned int)vid;
-            kor = dk;
-            knot = ~(unsigned long long)dk & 0xFFFFFFFFull;
-        }
+    }
+    __syncthreads();
+    const unsigned long long vis_base = s.vis_base;
+    unsigned long long kor = 0ull, knot = 0ull;
+    if (p.visible) {
+        const unsigned long long vid = vis_base + vis_local;
+        float4* dst = reinterpret_cast<float4*>(f.records + vid);
+        dst[0] = make_float4(p.cx, p.cy, p.z, p.op);
+        dst[1] = make_float4(p.ic00, p.ic01, p.ic11, 0.0f);
+        dst[2] = make_float4(p.r, p.g, p.b, 0.0f);
+        f.visible_ids[vid] = (unsigned int)i;
+        f.rects[vid] = pack_rect(p.min_tx, p.min_ty, p.max_tx, p.max_ty, 0);
+        const unsigned int dk = depth_key(p.z, opt.key_mode);
+        f.depth_keys[0][vid] = dk;
+        f.depth_order[0][vid] = (unsigned int)vid;
+        kor = dk;
+        knot = ~(unsigned long long)dk & 0xFFFFFFFFull;
+    }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            kor |= __shfl_xor_sync(0xffffffffu, kor, o);
-            knot |= __shfl_xor_sync(0xffffffffu, knot, o);
+    for (int o = 16; o > 0; o >>= 1) {
+        kor |= __shfl_xor_sync(0xffffffffu, kor, o);
+        knot |= __shfl_xor_sync(0xffffffffu, knot, o);
+    }
+    if (lane == 0 && block_vis) {
+        atomicOr(&s.key_or, kor);
+        atomicOr(&s.key_or_not, knot);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        if (block_vis) {
+            atomicOr(&ctrl->depth_sort.key_or, s.key_or);
+            atomicOr(&ctrl->depth_sort.key_or_not, s.key_or_not);
         }
-        if (lane == 0 && block_vis) {
-            atomicOr(&s.key_or, kor);
-            atomicOr(&s.key_or_not, knot);
+        if ((long long)blk == total_blocks - 1) {
+            ctrl->n_visible = (unsigned int)(vis_base + block_vis);
+            ctrl->depth_sort.n = vis_base + block_vis;
         }
-        __syncthreads();
-        if (tid == 0) {
-            if (block_vis) {
-                atomicOr(&ctrl->depth_sort.key_or, s.key_or);
-                atomicOr(&ctrl->depth_sort.key_or_not, s.key_or_not);
-            }
-            if ((long long)blk == total_blocks - 1) {
-                ctrl->n_visible = (unsigned int)(vis_base + block_vis);
-                ctrl->depth_sort.n = vis_base + block_vis;
-            }
-        }
-        if (!kPersistent) break;
-        __syncthreads();
     }
 }
 
@@ -572,8 +559,6 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
  *                         rectangle and depth key at the view's offset.
  * --------------------------------------------------------------------- */
 
-constexpr int kCamWords = (int)(sizeof(DevCamera) / 4);
-static_assert(sizeof(DevCamera) % 4 == 0 && kCamWords <= kProjThreads, "camera copy layout");
 constexpr int kOffsetsThreads = 1024;
 constexpr int kOffsetsItems = 8;    /* 8192 counts per tile: one tile for a 1M-Gaussian view */
 constexpr int kOffsetsTile = kOffsetsThreads * kOffsetsItems;
@@ -591,11 +576,6 @@ struct BatchProjSmem {
  * descriptors, in the project look-back region of the scratch. */
 __device__ __forceinline__ unsigned long long* offsets_desc(unsigned long long* lb, long long total_blocks) {
     return lb + (total_blocks + 1) / 2;
-}
-
-__device__ __forceinline__ void copy_camera(DevCamera& dst, const DevCamera& src) {
-    const int tid = threadIdx.x;
-    if (tid < kCamWords) reinterpret_cast<unsigned int*>(&dst)[tid] = reinterpret_cast<const unsigned int*>(&src)[tid];
 }
 
 /* The unit's Gaussian parameters (zeros past the scene's end). */
@@ -798,15 +778,13 @@ static int resident_ctas(const void* kernel, int threads, size_t smem) {
     return per_sm;
 }
 
-static int g_project_per_sm = 0, g_emit_per_sm = 0, g_batch_count_per_sm = 0, g_batch_project_per_sm = 0;
+static int g_emit_per_sm = 0, g_batch_count_per_sm = 0, g_batch_project_per_sm = 0;
 constexpr size_t kProjStageBytes = (size_t)kProjThreads * 48 * sizeof(float);
 
 /* Kernel attributes and the occupancy of the persistent kernels, set and
  * queried once (before any capture). */
 void prime_persistent_launches() {
-    cudaFuncSetAttribute(project_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjStageBytes);
-    cudaFuncSetAttribute(project_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjStageBytes);
-    g_project_per_sm = resident_ctas((const void*)project_kernel<true>, kProjThreads, kProjStageBytes);
+    cudaFuncSetAttribute(project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjStageBytes);
     g_emit_per_sm = resident_ctas((const void*)emit_kernel<1>, kEmitThreads, 0);
     cudaFuncSetAttribute(batch_project_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kProjStageBytes);
@@ -841,20 +819,12 @@ void launch_batch_project(const ViewTable* vt, const LumenRenderOptions& opt, co
                    vt, opt, f, ctrl, (const unsigned long long*)lb);
 }
 
-/* Plain launches: one CTA per block (n_blocks known on the host).
- * Persistent launches: every resident CTA, taking tickets. */
-void launch_project(const ViewTable* vt, int n_views, const LumenRenderOptions& opt, const LumenGpuFrame& f,
-                    Control* ctrl, unsigned long long* lb, long long n_blocks, bool persistent, int num_sms,
-                    cudaStream_t st) {
+/* One view of n_blocks blocks. */
+void launch_project(const ViewTable* vt, const LumenRenderOptions& opt, const LumenGpuFrame& f, Control* ctrl,
+                    unsigned long long* lb, long long n_blocks, cudaStream_t st) {
     if (n_blocks <= 0) return;
-    if (persistent) {
-        const int per_sm = g_project_per_sm > 0 ? g_project_per_sm : 1;
-        launch_chained(project_kernel<true>, dim3(per_sm * num_sms), dim3(kProjThreads), kProjStageBytes, st, vt,
-                       n_views, opt, f, ctrl, lb);
-    } else {
-        launch_chained(project_kernel<false>, dim3((unsigned int)n_blocks), dim3(kProjThreads), kProjStageBytes, st,
-                       vt, n_views, opt, f, ctrl, lb);
-    }
+    launch_chained(project_kernel, dim3((unsigned int)n_blocks), dim3(kProjThreads), kProjStageBytes, st, vt, opt, f,
+                   ctrl, lb);
 }
 
 /* sort_lb: the cell sort's look-back region (sort_lb_tiles descriptor

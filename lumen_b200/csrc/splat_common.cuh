@@ -278,16 +278,6 @@ __device__ __forceinline__ unsigned int cell_mask(unsigned long long rect, int x
     return (columns * 0x1111u) & rows;
 }
 
-/* The view whose [begin, next begin) holds x: the last view with begin <= x
- * (views with no blocks or tiles are skipped over). */
-__device__ __forceinline__ int find_view_by_block(const ViewTable* vt, int n_views, long long blk) {
-    int lo = 0, hi = n_views - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (vt->view[mid].block_begin <= blk) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
 /* The scene group that owns batch projection unit u: the last view with
  * unit_begin <= u (non-leading views own no units). */
 __device__ __forceinline__ int find_view_by_unit(const ViewTable* vt, int n_views, long long u) {
