@@ -35,13 +35,13 @@ void launch_batch_project(const ViewTable* vt, const LumenRenderOptions& opt, co
 void launch_project(const ViewTable* vt, const LumenRenderOptions& opt, const LumenGpuFrame& f, Control* ctrl,
                     unsigned long long* lb, long long n_blocks, cudaStream_t st);
 void launch_emit(const ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned long long* lb,
-                 unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys, long long n_blocks,
+                 unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys, bool wide, long long n_blocks,
                  bool persistent, int num_sms, cudaStream_t st);
 void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1, long long capacity,
                    SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int items,
                    int key_bytes, int num_sms, cudaStream_t st);
 void launch_cell_sort(const LumenGpuFrame& f, Control* ctrl, const ViewTable* vt, unsigned int* lb,
-                      long long lb_tiles_cap, int items, int key_bytes, int num_sms, cudaStream_t st);
+                      long long lb_tiles_cap, int items, int key_bytes, bool wide, int num_sms, cudaStream_t st);
 void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned char* scratch, long long room_offset,
                   long long room_bytes, long long n_cells, long long n_tiles, int num_sms, cudaStream_t st);
 void launch_sort64(unsigned long long* k0, unsigned int* v0, unsigned long long* k1, unsigned int* v1,
@@ -205,14 +205,20 @@ void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRen
         launch_sort32(f.depth_keys[0], f.depth_order[0], f.depth_keys[1], f.depth_order[1], n_slots,
                       &ctrl->depth_sort, depth_lb, L.depth_tiles, &ctrl->error_flags, lc.depth_sort_items, 4, sms,
                       s);
-        launch_emit(vt, f, ctrl, emit_lb, cell_lb, 2 * L.sort_tiles, kSortThreads * lc.tile_sort_items,
-                    L.proj_blocks, persistent, sms, s);
+        /* 257 to 512 cells (1080p has 510): one pass over nine bits instead of
+         * two over eight and one. 1 M splats at 1080p: the emission and both
+         * passes 87 us, with one pass 74. A persistent launch knows only a
+         * bound of the cells. */
+        const bool wide = !persistent && n_cells > 256 && n_cells <= kWideCells;
+        launch_emit(vt, f, ctrl, emit_lb, cell_lb, 2 * L.sort_tiles,
+                    wide ? kWideCells * kWideItems : kSortThreads * lc.tile_sort_items, wide, L.proj_blocks, persistent,
+                    sms, s);
         /* the cell-sort region holds 4 passes of 2048-key tiles; cell ids
          * below n_cells (the batch's, or the bound a persistent launch is
          * sized for) vary in their low ceil(log2(n_cells) / 8) bytes only */
         int cell_bytes = 0;
         for (long long t = n_cells - 1; t > 0; t >>= 8) ++cell_bytes;
-        launch_cell_sort(f, ctrl, vt, cell_lb, 2 * L.sort_tiles, lc.tile_sort_items, cell_bytes, sms, s);
+        launch_cell_sort(f, ctrl, vt, cell_lb, 2 * L.sort_tiles, lc.tile_sort_items, cell_bytes, wide, sms, s);
     } else if (ev) {
         cudaEventRecord(ev[1], s);
     }

@@ -336,7 +336,7 @@ constexpr unsigned int kEmitLaneCells = 16;
 template <int kRounds>
 __global__ void __launch_bounds__(kEmitThreads, 6)
 emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, unsigned long long* lb,
-            unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys) {
+            unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys, bool wide) {
     chain_begin();
     __shared__ EmitSmem s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -348,6 +348,9 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
     const bool packed = n_cells <= kPackedCells;
     int nd = 0;
     for (long long t = n_cells - 1; t > 0 && nd < 4; t >>= 8) ++nd;
+    const unsigned int digit_mask = wide ? kWideCells - 1 : 0xFFu;
+    if (wide) nd = 1;   /* one digit of 9 bits, in two rows of counts */
+    const int rows = wide ? 2 : nd;
     for (int d = 0; d < 4; ++d) s.hist[d][tid] = 0u;
     if (int* ranges = cell_ranges(f, ctrl, vt)) {
         const long long nthreads = (long long)gridDim.x * blockDim.x;
@@ -462,7 +465,7 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
                 knot |= ~cell;
                 f.keys[0][pos] = key;
                 f.vals[0][pos] = vis;
-                for (int d = 0; d < nd; ++d) atomicAdd(&s.hist[d][(cell >> (8 * d)) & 0xFFu], 1u);
+                for (int d = 0; d < nd; ++d) atomicAdd(&s.hist[d][0] + ((cell >> (8 * d)) & digit_mask), 1u);
             };
             const unsigned int most = __reduce_max_sync(0xffffffffu, c.pairs);
             if (most <= kEmitLaneCells) {
@@ -507,13 +510,15 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
                 const unsigned int t0 = (i0 + tk - 1u) / tk;
                 unsigned int t1 = (i1 + tk - 1u) / tk;
                 if ((long long)t1 > sort_lb_tiles) t1 = (unsigned int)sort_lb_tiles;
+                const int row = wide ? kWideCells : 256;
                 for (int d = 0; d < nd; ++d) {
                     unsigned int* region = sort_lb + (size_t)d * (size_t)lookback_rows(sort_lb_tiles) * 256;
-                    for (unsigned int t = t0; t < t1; ++t) {
-                        region[(size_t)t * 256 + tid] = 0u;
-                        if (t % kLookbackGroup == 0)   /* its group's row */
-                            region[((size_t)sort_lb_tiles + t / kLookbackGroup) * 256 + tid] = 0u;
-                    }
+                    for (unsigned int t = t0; t < t1; ++t)
+                        for (int j = tid; j < row; j += kEmitThreads) {
+                            region[(size_t)t * row + j] = 0u;
+                            if (t % kLookbackGroup == 0)   /* its group's row */
+                                region[((size_t)sort_lb_tiles + t / kLookbackGroup) * row + j] = 0u;
+                        }
                 }
             }
             if (tid == 0) {
@@ -527,7 +532,7 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
         }
         __syncthreads();
     }
-    for (int d = 0; d < nd; ++d) {
+    for (int d = 0; d < rows; ++d) {
         const unsigned int n = s.hist[d][tid];
         if (n) atomicAdd(&ctrl->cell_sort.hist[d][tid], n);
     }
@@ -830,14 +835,14 @@ void launch_project(const ViewTable* vt, const LumenRenderOptions& opt, const Lu
 /* sort_lb: the cell sort's look-back region (sort_lb_tiles descriptor
  * tiles per digit) for digit passes of sort_tile_keys keys per tile. */
 void launch_emit(const ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned long long* lb,
-                 unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys, long long n_blocks,
+                 unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys, bool wide, long long n_blocks,
                  bool persistent, int num_sms, cudaStream_t st) {
     if (n_blocks <= 0) return;
     const long long resident = (long long)(g_emit_per_sm > 0 ? g_emit_per_sm : 1) * num_sms;
     auto run = [&](auto kernel, int rounds) {
         const long long blocks = (n_blocks * kProjThreads + rounds * kEmitThreads - 1) / (rounds * kEmitThreads);
         launch_chained(kernel, dim3((unsigned int)(persistent || blocks > resident ? resident : blocks)),
-                       dim3(kEmitThreads), 0, st, vt, f, ctrl, lb, sort_lb, sort_lb_tiles, sort_tile_keys);
+                       dim3(kEmitThreads), 0, st, vt, f, ctrl, lb, sort_lb, sort_lb_tiles, sort_tile_keys, wide);
     };
     if (n_blocks * kProjThreads >= 3ll * num_sms * kEmitMaxRounds * kEmitThreads)
         run(emit_kernel<kEmitMaxRounds>, kEmitMaxRounds);

@@ -126,16 +126,19 @@ histogram_kernel(const KeyT* __restrict__ keys, long long capacity, SortControl*
     }
 }
 
-template <typename KeyT, int kItems>
+/* kThreads: threads and digit values of the pass, 256 or 512 (the cell sort's
+ * single pass over 257 to 512 cells). */
+template <typename KeyT, int kItems, int kThreads = kSortThreads>
 struct PassSmem {
-    KeyT keys[kSortThreads * kItems];
-    unsigned int vals[kSortThreads * kItems];
-    unsigned int whist[kSortThreads / 32][256];
-    unsigned int match[2][kSortThreads / 32][256];   /* per item parity and warp: lanes holding each digit */
-    unsigned int digit_start[256];
-    long long gbase[256];
-    unsigned int goffset[256];
-    unsigned int warp_sums[kSortThreads / 32];
+    static constexpr int kSets = kThreads == 256 ? 2 : 1;
+    KeyT keys[kThreads * kItems];
+    unsigned int vals[kThreads * kItems];
+    unsigned int whist[kThreads / 32][kThreads];
+    unsigned int match[kSets][kThreads / 32][kThreads];   /* per item parity and warp: lanes holding each digit */
+    unsigned int digit_start[kThreads];
+    long long gbase[kThreads];
+    unsigned int goffset[kThreads];
+    unsigned int warp_sums[kThreads / 32];
     unsigned int tile;
 };
 
@@ -150,6 +153,7 @@ struct PassSmem {
 constexpr int kLookbackWindow = 4;
 constexpr unsigned int kGroupOne = 1u << 20;   /* 16 tiles of at most 6144 keys stay below */
 
+template <int kRow>
 __device__ __forceinline__ unsigned int lookback_digit(const unsigned int* lb, const unsigned int* groups, int tile,
                                                        int t, unsigned int* err) {
     unsigned int excl = 0;
@@ -159,7 +163,7 @@ __device__ __forceinline__ unsigned int lookback_digit(const unsigned int* lb, c
         unsigned int d[kLookbackWindow];
 #pragma unroll
         for (int w = 0; w < kLookbackWindow; ++w)
-            d[w] = j - w >= g0 * kLookbackGroup ? ld_volatile_u32(lb + (size_t)(j - w) * 256 + t) : 0u;
+            d[w] = j - w >= g0 * kLookbackGroup ? ld_volatile_u32(lb + (size_t)(j - w) * kRow + t) : 0u;
         bool stalled = false;
 #pragma unroll
         for (int w = 0; w < kLookbackWindow; ++w) {
@@ -186,8 +190,8 @@ __device__ __forceinline__ unsigned int lookback_digit(const unsigned int* lb, c
 #pragma unroll
         for (int w = 0; w < kLookbackWindow; ++w) {
             const int gw = g - w;
-            last[w] = gw >= 0 ? ld_volatile_u32(lb + ((size_t)gw * kLookbackGroup + kLookbackGroup - 1) * 256 + t) : 0u;
-            sum[w] = gw >= 0 ? ld_volatile_u32(groups + (size_t)gw * 256 + t) : 0u;
+            last[w] = gw >= 0 ? ld_volatile_u32(lb + ((size_t)gw * kLookbackGroup + kLookbackGroup - 1) * kRow + t) : 0u;
+            sum[w] = gw >= 0 ? ld_volatile_u32(groups + (size_t)gw * kRow + t) : 0u;
         }
         bool stalled = false;
 #pragma unroll
@@ -237,20 +241,28 @@ __device__ __forceinline__ void cell_edges(int* ranges, unsigned int id_mask, co
         atomicMax(ranges + 2 * (size_t)c + 1, (int)(pos + 1));
 }
 
-/* kItems keys per thread: tiles of 256 * kItems keys. */
-template <typename KeyT, int kItems>
-__global__ void __launch_bounds__(kSortThreads, sizeof(KeyT) == 4 ? (kItems <= 8 ? 4 : kItems <= 16 ? 3 : 2) : 2)
+/* Resident CTAs per SM of a pass. */
+template <typename KeyT, int kItems, int kThreads>
+constexpr int kPassCtas = sizeof(KeyT) == 4 && kThreads == 256 ? (kItems <= 8 ? 4 : kItems <= 16 ? 3 : 2) : 2;
+
+/* kItems keys per thread: tiles of kThreads * kItems keys. */
+template <typename KeyT, int kItems, int kThreads = kSortThreads>
+__global__ void __launch_bounds__(kThreads, (kPassCtas<KeyT, kItems, kThreads>))
 onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, long long capacity, SortControl* sc,
                      unsigned int* lb_all, long long lb_tiles_cap, unsigned int* err, int digit, CellSink sink) {
     chain_begin();
-    constexpr int kTileKeys = kSortThreads * kItems;
+    constexpr int kTileKeys = kThreads * kItems;
+    constexpr int kWarps = kThreads / 32;
+    constexpr unsigned int kDigit = kThreads - 1;   /* a digit's bits */
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PassSmem<KeyT, kItems>& s = *reinterpret_cast<PassSmem<KeyT, kItems>*>(smem_raw);
+    using Smem = PassSmem<KeyT, kItems, kThreads>;
+    Smem& s = *reinterpret_cast<Smem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     /* the digits that vary, from the producer's key statistics (the same
      * rule as the histogram kernel's, for sorts whose histogram the producer
      * counted) */
-    const unsigned int varying = sort_count(sc, capacity) > 1 ? varying_digits(sc, (int)sizeof(KeyT)) : 0u;
+    unsigned int varying = sort_count(sc, capacity) > 1 ? varying_digits(sc, (int)sizeof(KeyT)) : 0u;
+    if (kThreads != 256) varying = varying ? 1u : 0u;   /* one digit */
     if (blockIdx.x == 0 && tid == 0) {
         sc->varying = varying;
         sc->sorted_buffer = (unsigned int)(__popc(varying) & 1);
@@ -264,8 +276,8 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
     const long long K = sort_count(sc, capacity);
     const long long ntiles = (K + kTileKeys - 1) / kTileKeys;
     const int shift = 8 * digit;
-    unsigned int* lb = lb_all + (size_t)digit * (size_t)lookback_rows(lb_tiles_cap) * 256;
-    unsigned int* groups = lb + (size_t)lb_tiles_cap * 256;
+    unsigned int* lb = lb_all + (size_t)digit * (size_t)lookback_rows(lb_tiles_cap) * kThreads;
+    unsigned int* groups = lb + (size_t)lb_tiles_cap * kThreads;
     int* edges = nullptr;
     unsigned int id_mask = 0xFFFFFFFFu;
     if (sizeof(KeyT) == 4 && sink.ctrl && (varying >> digit) == 1u) {   /* the pass over the highest varying byte */
@@ -276,7 +288,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
 
     /* global exclusive offsets of this digit's buckets */
     {
-        const unsigned int c = sc->hist[digit][tid];
+        const unsigned int c = (&sc->hist[0][0])[digit * 256 + tid];
         unsigned int x = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -292,7 +304,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
     }
 
     /* the match masks start clear; each item's leaders clear what it set */
-    for (int j = tid; j < 2 * (kSortThreads / 32) * 256; j += kSortThreads) (&s.match[0][0][0])[j] = 0u;
+    for (int j = tid; j < Smem::kSets * kWarps * kThreads; j += kThreads) (&s.match[0][0][0])[j] = 0u;
 
     for (;;) {
         if (tid == 0) s.tile = atomicAdd(&sc->pass_ticket[digit], 1u);
@@ -312,7 +324,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
             v[it] = valid ? vin[idx] : 0u;
         }
         const long long wbase = base + warp * (kItems * 32);
-        for (int b = lane; b < 256; b += 32) s.whist[warp][b] = 0u;
+        for (int b = lane; b < kThreads; b += 32) s.whist[warp][b] = 0u;
         __syncwarp();
         /* the tile's digit counts come first (per-warp shared histograms; the
          * order of the increments does not matter), so that the tile's
@@ -320,20 +332,20 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
          * look-back chain of the tiles after it moves on sooner */
 #pragma unroll
         for (int it = 0; it < kItems; ++it)
-            if (wbase + it * 32 + lane < K) atomicAdd(&s.whist[warp][(unsigned int)((k[it] >> shift) & 0xFF)], 1u);
+            if (wbase + it * 32 + lane < K) atomicAdd(&s.whist[warp][(unsigned int)((k[it] >> shift) & kDigit)], 1u);
         __syncthreads();
         /* digit t: warp-exclusive offsets and the tile's count */
         const int t = tid;
         unsigned int run = 0;
 #pragma unroll
-        for (int w = 0; w < kSortThreads / 32; ++w) {
+        for (int w = 0; w < kWarps; ++w) {
             const unsigned int c = s.whist[w][t];
             s.whist[w][t] = run;
             run += c;
         }
         const unsigned int count = run;
-        st_volatile_u32(lb + (size_t)tile * 256 + t, (tile == 0 ? kDescIncl32 : kDescAgg32) | count);
-        atomicAdd(groups + (size_t)(tile / kLookbackGroup) * 256 + t, kGroupOne + count);
+        st_volatile_u32(lb + (size_t)tile * kThreads + t, (tile == 0 ? kDescIncl32 : kDescAgg32) | count);
+        atomicAdd(groups + (size_t)(tile / kLookbackGroup) * kThreads + t, kGroupOne + count);
         {
             unsigned int x = count;
 #pragma unroll
@@ -363,8 +375,8 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
 #pragma unroll
         for (int it = 0; it < kItems; ++it) {
             const bool valid = wbase + it * 32 + lane < K;
-            const unsigned int d = (unsigned int)((k[it] >> shift) & 0xFF);
-            unsigned int* mk = s.match[it & 1][warp];
+            const unsigned int d = (unsigned int)((k[it] >> shift) & kDigit);
+            unsigned int* mk = s.match[it % Smem::kSets][warp];
             if (valid) atomicOr(&mk[d], 1u << lane);
             __syncwarp();
             const unsigned int peers = valid ? mk[d] : 0u;
@@ -380,13 +392,14 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
                 s.keys[pos] = k[it];
                 s.vals[pos] = v[it];
             }
+            if (Smem::kSets == 1) __syncwarp();   /* the masks are clear before the next item sets them */
         }
         /* the look-back runs once the keys are in shared memory (their
          * registers are free for a wide window of descriptors) */
         unsigned int excl = 0;
         if (tile > 0) {
-            excl = lookback_digit(lb, groups, (int)tile, t, err);
-            st_volatile_u32(lb + (size_t)tile * 256 + t, kDescIncl32 | (excl + count));
+            excl = lookback_digit<kThreads>(lb, groups, (int)tile, t, err);
+            st_volatile_u32(lb + (size_t)tile * kThreads + t, kDescIncl32 | (excl + count));
         }
         s.gbase[t] = (long long)s.goffset[t] + (long long)excl - (long long)s.digit_start[t];
         __syncthreads();
@@ -394,18 +407,18 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
         if (nvalid == kTileKeys) {
 #pragma unroll
             for (int it = 0; it < kItems; ++it) {
-                const int j = it * kSortThreads + tid;
+                const int j = it * kThreads + tid;
                 const KeyT kk = s.keys[j];
-                const unsigned int d = (unsigned int)((kk >> shift) & 0xFF);
+                const unsigned int d = (unsigned int)((kk >> shift) & kDigit);
                 const long long out = s.gbase[d] + j;
                 kout[out] = kk;
                 vout[out] = s.vals[j];
                 if (edges) cell_edges(edges, id_mask, s.keys, j, kTileKeys, kk, out);
             }
         } else {
-            for (int j = tid; j < nvalid; j += kSortThreads) {
+            for (int j = tid; j < nvalid; j += kThreads) {
                 const KeyT kk = s.keys[j];
-                const unsigned int d = (unsigned int)((kk >> shift) & 0xFF);
+                const unsigned int d = (unsigned int)((kk >> shift) & kDigit);
                 const long long out = s.gbase[d] + j;
                 kout[out] = kk;
                 vout[out] = s.vals[j];
@@ -638,19 +651,18 @@ __global__ void sorted_keys64_kernel(const unsigned int* k0, const unsigned int*
 /* key_bytes: the low bytes that can vary at all (a pass per byte is
  * launched; among those, passes over bytes that turn out constant exit at
  * once). */
-template <typename KeyT, int kItems>
+template <typename KeyT, int kItems, int kThreads = kSortThreads>
 void launch_sort_impl(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, long long capacity, SortControl* sc,
                       unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int key_bytes, int num_sms,
                       cudaStream_t st, const CellSink* sink = nullptr) {
     if (!sink)
         launch_chained(histogram_kernel<KeyT>, dim3(num_sms * 4), dim3(256), 0, st, (const KeyT*)k0, capacity, sc, lb,
                        lb_tiles_cap, kSortThreads * kItems);
-    const size_t smem = sizeof(PassSmem<KeyT, kItems>);
-    /* matches __launch_bounds__: all CTAs resident */
-    const int ctas_per_sm = sizeof(KeyT) == 4 ? (kItems <= 8 ? 4 : kItems <= 16 ? 3 : 2) : 2;
+    const size_t smem = sizeof(PassSmem<KeyT, kItems, kThreads>);
+    const int ctas_per_sm = kPassCtas<KeyT, kItems, kThreads>;   /* all CTAs resident */
     const int nd = key_bytes < (int)sizeof(KeyT) ? key_bytes : (int)sizeof(KeyT);
     for (int d = 0; d < nd; ++d)
-        launch_chained(onesweep_pass_kernel<KeyT, kItems>, dim3(num_sms * ctas_per_sm), dim3(kSortThreads), smem, st,
+        launch_chained(onesweep_pass_kernel<KeyT, kItems, kThreads>, dim3(num_sms * ctas_per_sm), dim3(kThreads), smem, st,
                        k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, d, sink ? *sink : CellSink{});
 }
 
@@ -688,8 +700,14 @@ void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigne
  * the look-back tiles and filled the cells' ranges with -1, so only the digit
  * passes run, the last of which writes the ranges. */
 void launch_cell_sort(const LumenGpuFrame& f, Control* ctrl, const ViewTable* vt, unsigned int* lb,
-                      long long lb_tiles_cap, int items, int key_bytes, int num_sms, cudaStream_t st) {
+                      long long lb_tiles_cap, int items, int key_bytes, bool wide, int num_sms, cudaStream_t st) {
     const CellSink sink{ctrl, vt, f};
+    if (wide) {
+        launch_sort_impl<unsigned int, kWideItems, kWideCells>(
+            f.keys[0], f.vals[0], f.keys[1], f.vals[1], f.instance_capacity, &ctrl->cell_sort, lb, lb_tiles_cap,
+            &ctrl->error_flags, 1, num_sms, st, &sink);
+        return;
+    }
     launch_sort_items(f.keys[0], f.vals[0], f.keys[1], f.vals[1], f.instance_capacity, &ctrl->cell_sort, lb,
                       lb_tiles_cap, &ctrl->error_flags, items, key_bytes, &sink, num_sms, st);
 }
@@ -721,6 +739,9 @@ void configure_sort_kernels() {
                          (int)sizeof(PassSmem<unsigned int, 8>));
     cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(PassSmem<unsigned int, 16>));
+    cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, kWideItems, kWideCells>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(PassSmem<unsigned int, kWideItems, kWideCells>));
     cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, 24>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(PassSmem<unsigned int, 24>));
     cudaFuncSetAttribute(onesweep_pass_kernel<unsigned long long, kSort64Items>,

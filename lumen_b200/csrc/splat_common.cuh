@@ -85,6 +85,10 @@ __device__ __forceinline__ long long tile_in_line(const Control* ctrl, long long
  * covers in the upper half. With more cells the key is the id alone and the
  * mask is formed again from the rectangle. */
 constexpr int kCellSide = 4;
+/* From 257 to 512 cells the cell sort is one wide pass, by 512 threads with 8
+ * keys each. */
+constexpr int kWideCells = 512;
+constexpr int kWideItems = 8;
 constexpr long long kPackedCells = 1ll << 16;
 
 /* Resident CTAs per SM the compositor is compiled for (72 registers per

@@ -61,6 +61,13 @@ def test_lists_around_a_segment(n):
     _check(_scene(n, n, spread=(0.3, 0.3)), _cam(64, 64))
 
 
+@pytest.mark.parametrize("size", [(1024, 1024), (257 * 64 - 3, 40), (2048, 1024), (1728, 1210)])
+@pytest.mark.parametrize("n", [5, 3000])
+def test_cell_sort_in_one_pass(n, size):
+    """256, 257, 512 and 513 cells: 257 to 512 are sorted in one pass over nine bits."""
+    _check(_scene(n, size[0] + n, scale=(0.01, 0.4)), _cam(*size))
+
+
 # 2040 cells: the notes of 80 B per cell do not fit the scratch of so few instances, and the cells'
 # ranges do not fit the depth keys of 300 splats
 @pytest.mark.parametrize("n", [300, 5000])
