@@ -430,15 +430,18 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
                 block_pairs += s.warp_pairs[q][w];
                 block_tiles += s.warp_tiles[q][w];
             }
-            s.rect[tid] = r;
-            s.run[tid] = make_uint4(excl, c.cw, cell0, cells_x);
-            s.aux[tid] = make_uint2(__float_as_uint(1.0f / (float)c.cw), v);
-            __syncwarp();
             const unsigned int tile_base = (unsigned int)(base >> 31) & 0x7FFFFFFFu;
             const unsigned int pair_base = (unsigned int)base & 0x7FFFFFFFu;
             /* the capacity is reached in this block or before it */
             const bool over = tile_base + min(block_tiles, kSaturated) > cap;
             unsigned int kept_pairs = block_pairs, cut = kEmitThreads;
+            const bool lanes = !over && __reduce_max_sync(0xffffffffu, c.pairs) <= kEmitLaneCells;
+            if (!lanes) {
+                s.rect[tid] = r;
+                s.run[tid] = make_uint4(excl, c.cw, cell0, cells_x);
+                s.aux[tid] = make_uint2(__float_as_uint(1.0f / (float)c.cw), v);
+                __syncwarp();
+            }
             if (over) {
                 __syncthreads();
                 if (tid == 0) {
@@ -449,35 +452,37 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
                 kept_pairs = s.kept;
                 cut = s.cut;
             }
-            /* one pair of splat lo (rectangle rect, first tile of the cell's column and row), block-relative index j */
-            auto store = [&](unsigned int lo, unsigned long long rect, unsigned int cx, unsigned int cy, unsigned int cell,
-                             unsigned int vis, unsigned int j) {
-                unsigned int key = cell;
-                if (packed) {
-                    const int x = (int)cx * kCellSide, y = (int)cy * kCellSide;
-                    unsigned int mask = cell_mask(rect, x, y);
-                    if (over && lo == cut) mask = emit_cut_mask(rect, x, y, mask, s.cut_tiles);
-                    key |= mask << 16;
-                }
-                const unsigned int pos = pair_base + j;   /* below the capacity, like the instances */
-                if (pos >= cap) return;
+            auto count = [&](unsigned int cell) {
                 kor |= cell;
                 knot |= ~cell;
-                f.keys[0][pos] = key;
-                f.vals[0][pos] = vis;
-                for (int d = 0; d < nd; ++d) atomicAdd(&s.hist[d][0] + ((cell >> (8 * d)) & digit_mask), 1u);
+                atomicAdd(&s.hist[0][0] + (cell & digit_mask), 1u);
+                for (int d = 1; d < nd; ++d) atomicAdd(&s.hist[d][(cell >> (8 * d)) & 0xFFu], 1u);
             };
-            const unsigned int most = __reduce_max_sync(0xffffffffu, c.pairs);
-            if (most <= kEmitLaneCells) {
-                unsigned int col = 0u, row = 0u;
-                for (unsigned int k = 0; k < most; ++k) {
-                    if (k < c.pairs && excl + k < kept_pairs)
-                        store((unsigned int)tid, r, c.cx + col, c.cy + row, cell0 + row * cells_x + col, v, excl + k);
+            if (lanes) {
+                /* A cell's mask is what the rectangle's four sides leave of
+                 * it; a side matters in its own row or column of cells only. */
+                const unsigned int left = 0x1111u * ((0xFu << (rect_min_tx(r) % kCellSide)) & 0xFu);
+                const unsigned int right = 0x1111u * (0xFu >> (kCellSide - 1 - rect_max_tx(r) % kCellSide));
+                const unsigned int top = (0xFFFFu << (4 * (rect_min_ty(r) % kCellSide))) & 0xFFFFu;
+                const unsigned int bottom = 0xFFFFu >> (4 * (kCellSide - 1 - rect_max_ty(r) % kCellSide));
+                const unsigned int last_row = (unsigned int)rect_max_ty(r) / kCellSide - c.cy;
+                unsigned int cell = cell0, col = 0u, row = 0u;
+                unsigned int* key = f.keys[0] + pair_base + excl;
+                unsigned int* val = f.vals[0] + pair_base + excl;
+                for (unsigned int k = 0; k < c.pairs; ++k) {
+                    const unsigned int mask = (col == 0u ? left : 0xFFFFu) & (col + 1u == c.cw ? right : 0xFFFFu) &
+                                              (row == 0u ? top : 0xFFFFu) & (row == last_row ? bottom : 0xFFFFu);
+                    key[k] = packed ? mask * (unsigned int)kPackedCells + cell : cell;
+                    val[k] = v;
+                    count(cell);
+                    ++cell;
                     if (++col == c.cw) {
                         col = 0u;
                         ++row;
+                        cell += cells_x - c.cw;
                     }
                 }
+                __syncwarp();
             } else {
                 /* The warp's pairs (those of its 32 splats, consecutive in the
                  * block's order), kEmitWindow at a time. Each splat marks the
@@ -496,8 +501,20 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
                         unsigned int column;
                         const unsigned int row = emit_row(s, lo, rn, a + jj, &column);
                         const unsigned long long rect = s.rect[lo];
-                        store((unsigned int)lo, rect, rect_min_tx(rect) / kCellSide + column,
-                              rect_min_ty(rect) / kCellSide + row, rn.z + row * rn.w + column, s.aux[lo].y, a + jj);
+                        const unsigned int cell = rn.z + row * rn.w + column;
+                        const unsigned int pos = pair_base + a + jj;   /* below the capacity, like the instances */
+                        if (pos >= cap) continue;
+                        unsigned int key = cell;
+                        if (packed) {
+                            const int x = (int)(rect_min_tx(rect) / kCellSide + column) * kCellSide;
+                            const int y = (int)(rect_min_ty(rect) / kCellSide + row) * kCellSide;
+                            unsigned int mask = cell_mask(rect, x, y);
+                            if (over && (unsigned int)lo == cut) mask = emit_cut_mask(rect, x, y, mask, s.cut_tiles);
+                            key |= mask << 16;
+                        }
+                        f.keys[0][pos] = key;
+                        f.vals[0][pos] = s.aux[lo].y;
+                        count(cell);
                     }
                     __syncwarp();
                 }
