@@ -84,9 +84,11 @@ typedef struct {
  * The reference sorts 64-bit (tile << 32 | depth key) instance keys with a
  * stable LSD sort over emission order (pipeline.mojo:152-166). The same
  * permutation is produced here in two smaller sorts: the visible splats are
- * stably sorted by depth key (depth_keys/depth_order), instances are emitted
- * in that order with 32-bit tile-id keys, and those are stably sorted by
- * tile (keys/vals). Within a tile both orders are (depth key, visible index).
+ * stably sorted by depth key (depth_keys/depth_order), one pair per cell of
+ * 4x4 tiles that a splat touches is emitted in that order and stably sorted by
+ * cell, and each cell's list is split over its tiles (keys/vals). Within a tile
+ * both orders are (depth key, visible index). The depth buffers that the depth
+ * sort left unsorted are used as scratch after it.
  *
  * Per Gaussian (n_gaussians entries each): records, visible_ids, radii,
  * rects (tile rectangle of each visible splat: min_tx | min_ty << 16 |
@@ -210,8 +212,9 @@ LumenStatus lumen_gpu_stage_timer_read(LumenGpuStageTimer* timer, float stage_ms
 /* Launch parameters of the forward; none of them changes any output.
  * composite_chunk: sorted instances the compositor stages per round (128,
  * 256 or 512); *_sort_items: keys per thread in a digit pass of the depth
- * and tile sorts (depth: 8 or 16; tile: 8, 16 or 24 — tiles of 2048, 4096
- * or 6144 keys). Defaults 512, 16, 16. */
+ * and cell sorts (depth: 8 or 16; cell: 8, 16 or 24 — tiles of 2048, 4096
+ * or 6144 keys); sorts of up to 131072 depth keys and cell sorts of 257 to
+ * 512 cells have one form only. Defaults 256, 16, 16. */
 typedef struct {
     int32_t composite_chunk;
     int32_t depth_sort_items;
@@ -227,9 +230,9 @@ LumenStatus lumen_gpu_render_forward_ex(const LumenGpuGaussians* gaussians, cons
 
 /* ---------------------------------------------------------------- batches
  * Several views rendered by one pipeline: one projection over all views'
- * Gaussians, one depth sort, one tile sort whose 32-bit keys are batch-wide
- * tile ids (the view's first tile id + ty * tiles_x + tx, so the view id is
- * the key's high part), one range pass and one persistent compositor. A
+ * Gaussians, one depth sort, one cell sort whose lists are split over
+ * batch-wide tile ids (the view's first tile id + ty * tiles_x + tx) and one
+ * compositor. A
  * view's image is identical to rendering it alone: within a (view, tile) the
  * instances are ordered by (depth key, visible index) either way, and the
  * visible indices of a view keep its Gaussian order.

@@ -11,17 +11,15 @@
  *    batch while the batch fits a slot's work buffers (projection slots,
  *    tiles, an instance estimate learned per scene and resolution, output
  *    pixels) and max_views_per_batch, and while its tiles number at most
- *    65 536 (unless one view alone has more): batch-wide tile ids then sort
- *    in two digit passes, where one tile more would add a third pass over
- *    every instance of the batch;
+ *    65 536 (unless one view alone has more);
  *  - up to max_batches_in_flight batches are on the device at once, each on
  *    its own stream with its own buffers, so a batch admitted while others
  *    run overlaps with them; a slot is reused as soon as its batch is done;
  *  - a batch is rendered by the multi-view pipeline (lumen_gpu_render_batch
- *    semantics: every view equals rendering it alone) as one launch of a
+ *    semantics: every view equals rendering it alone): one launch of a
  *    captured CUDA graph whose persistent kernels read the batch from a
- *    device view table, then each view's bytes are copied to its request's
- *    host buffer;
+ *    device view table, then the compositor view by view, each view's bytes
+ *    leaving for its request's host buffer while the next is composited;
  *  - the compositor chunk and the digit-pass tile size of each batch are
  *    chosen by an autotuner that times the variants on live batches (they
  *    do not change any result) per batch size class;

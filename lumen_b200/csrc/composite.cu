@@ -5,8 +5,7 @@
  * src/raster/pipeline.mojo:172-229, with compute_gaussian_pixel_alpha and
  * PixelAccumulator.blend/finalize, src/raster/compositor.mojo:10-89.
  *
- * One CTA of 128 threads per 16x16 tile (or persistent CTAs taking tiles in
- * ticket order). A group of 8 lanes shades a 4x4 block of pixels, a lane two
+ * One CTA of 128 threads per 16x16 tile. A group of 8 lanes shades a 4x4 block of pixels, a lane two
  * pixels one above the other, so a warp holds four blocks (an 8x8 quadrant)
  * that walk four lists of their own in step. The tile's sorted instances are
  * processed in chunks of 128, 256 or 512 (a launch parameter the autotuner
@@ -444,29 +443,6 @@ composite_kernel(const ViewTable* __restrict__ vt, int n_views, const LumenSplat
                                    in_line ? tile_in_line(ctrl, blockIdx.x) : tile_offset + blockIdx.x);
 }
 
-/* Persistent form for a grid fixed in advance (a captured graph replayed
- * for batches of any size): CTAs take tiles in ticket order. */
-template <int kChunk, bool kTrack>
-__global__ void __launch_bounds__(kCompositeThreads, kCompositeBlocksPerSm)
-composite_persistent_kernel(const ViewTable* __restrict__ vt, const LumenSplatRecord* __restrict__ records,
-                            LumenGpuFrame f, long long capacity, Control* __restrict__ ctrl, LumenRenderOptions opt,
-                            float t_stop, float minus_one) {
-    chain_begin();
-    __shared__ CompositeSmem<kChunk> s;
-    init_padding_splat(s);
-    const long long total = vt->hdr.total_tiles;
-    const int n_views = vt->hdr.n_views;
-    for (;;) {
-        if (threadIdx.x == 0) s.ticket = atomicAdd(&ctrl->composite_ticket, 1u);
-        __syncthreads();
-        const long long t = s.ticket;
-        if (t >= total) break;
-        composite_tile<kChunk, kTrack>(s, vt, records, f, capacity, ctrl, opt, t_stop, splat2(minus_one), n_views,
-                                       tile_in_line(ctrl, t));
-        __syncthreads();
-    }
-}
-
 /* The transmittance at or below which a blend stops its pixel. Termination
  * mode 0 compares T with the threshold itself (compositor.mojo:53); mode 1
  * stops when 1 - T, rounded, reaches the threshold, which holds for every T
@@ -492,35 +468,28 @@ static float stop_transmittance(const LumenRenderOptions& opt) {
 template <int kChunk, bool kTrack>
 static void launch_composite_chunk(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
                                    const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
-                                   bool persistent, int num_sms, cudaStream_t st) {
-    if (persistent) {
-        launch_chained(composite_persistent_kernel<kChunk, kTrack>, dim3(kCompositeBlocksPerSm * num_sms),
-                       dim3(kCompositeThreads), 0, st, vt, (const LumenSplatRecord*)f.records, f,
-                       (long long)f.instance_capacity, ctrl, opt, stop_transmittance(opt),
-                       -1.0f);
-    } else {
-        launch_chained(composite_kernel<kChunk, kTrack>, dim3((unsigned int)n_tiles), dim3(kCompositeThreads), 0, st, vt,
-                       n_views, (const LumenSplatRecord*)f.records, f, (long long)f.instance_capacity, ctrl, opt,
-                       tile_offset, whole, stop_transmittance(opt), -1.0f);
-    }
+                                   int num_sms, cudaStream_t st) {
+    launch_chained(composite_kernel<kChunk, kTrack>, dim3((unsigned int)n_tiles), dim3(kCompositeThreads), 0, st, vt,
+                   n_views, (const LumenSplatRecord*)f.records, f, (long long)f.instance_capacity, ctrl, opt,
+                   tile_offset, whole, stop_transmittance(opt), -1.0f);
 }
 
 template <int kChunk>
 static void launch_composite_track(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
                                    const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
-                                   bool persistent, bool track, int num_sms, cudaStream_t st) {
+                                   bool track, int num_sms, cudaStream_t st) {
     if (track)
-        launch_composite_chunk<kChunk, true>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, num_sms, st);
+        launch_composite_chunk<kChunk, true>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, num_sms, st);
     else
-        launch_composite_chunk<kChunk, false>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, num_sms, st);
+        launch_composite_chunk<kChunk, false>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, num_sms, st);
 }
 
-/* chunk: instances staged per round, one of kCompositeChunks. Plain
- * launches shade tiles [tile_offset, tile_offset + n_tiles) of the batch;
- * persistent launches take every tile of the table by ticket. track: some
- * view's image asks for contributor counts or last-visited offsets. */
+/* Shades tiles [tile_offset, tile_offset + n_tiles) of the batch. whole: these
+ * are all its tiles, so they may go longest list first. chunk: instances
+ * staged per round, one of kCompositeChunks. track: some view's image asks for
+ * contributor counts or last-visited offsets. */
 void launch_composite(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
-                      const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole, bool persistent,
+                      const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
                       int chunk, bool track, int num_sms, cudaStream_t st) {
     if (n_tiles <= 0) return;
     /* Not chained: blocks that are resident before the list kernel ends are
@@ -531,15 +500,15 @@ void launch_composite(const ViewTable* vt, int n_views, const LumenGpuFrame& f, 
     ChainedLaunches chained(false);
     switch (chunk) {
         case 128:
-            launch_composite_track<128>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, track, num_sms,
+            launch_composite_track<128>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, track, num_sms,
                                         st);
             break;
         case 512:
-            launch_composite_track<512>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, track, num_sms,
+            launch_composite_track<512>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, track, num_sms,
                                         st);
             break;
         default:
-            launch_composite_track<256>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, persistent, track, num_sms,
+            launch_composite_track<256>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, track, num_sms,
                                         st);
             break;
     }

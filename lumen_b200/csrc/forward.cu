@@ -51,7 +51,7 @@ void launch_key_stats64(const unsigned long long* keys, long long n, SortControl
 void launch_sorted_keys64(const LumenGpuFrame& f, const Control* ctrl, int key_mode, unsigned long long* out,
                           int num_sms, cudaStream_t st);
 void launch_composite(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
-                      const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole, bool persistent,
+                      const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
                       int chunk, bool track, int num_sms, cudaStream_t st);
 void configure_sort_kernels();
 
@@ -227,7 +227,7 @@ void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRen
                  n_cells, n_tiles, sms, s);
     if (ev) cudaEventRecord(ev[3], s);
     if (!with_composite) return;
-    launch_composite(vt, n_views, f, ctrl, opt, 0, n_tiles, true, persistent, lc.composite_chunk, lc.track != 0, sms, s);
+    launch_composite(vt, n_views, f, ctrl, opt, 0, n_tiles, true, lc.composite_chunk, lc.track != 0, sms, s);
     if (ev) cudaEventRecord(ev[4], s);
 }
 
@@ -327,7 +327,7 @@ LumenStatus forward_banded(const LumenGpuGaussians* g, const LumenViewCamera* ca
     if (n_bands > tiles_y) n_bands = tiles_y;
     for (int b = 0; b < n_bands; ++b) {
         const int r0 = (int)((long long)tiles_y * b / n_bands), r1 = (int)((long long)tiles_y * (b + 1) / n_bands);
-        launch_composite(vt, 1, *f, ctrl, *opt, (long long)r0 * tiles_x, (long long)(r1 - r0) * tiles_x, false, false,
+        launch_composite(vt, 1, *f, ctrl, *opt, (long long)r0 * tiles_x, (long long)(r1 - r0) * tiles_x, false,
                          kDefaultLaunch.composite_chunk, img->n_contrib || img->last_idx, sms, s);
         const int y0 = r0 * kTile, y1 = r1 * kTile < cam->height ? r1 * kTile : cam->height;
         if (after_band) after_band(ctx, y0, y1, s);

@@ -60,10 +60,10 @@ struct Control {
     unsigned int proj_ticket;            /* block order of the project look-back */
     unsigned int cells_by_sort;          /* 1: the cell sort's last digit pass wrote the cells' ranges */
     unsigned int emit_ticket;            /* block order of the emit look-back */
-    unsigned int composite_ticket;       /* tile order of the compositor */
     unsigned int count_ticket;           /* unit order of the batch visibility count */
     unsigned int offsets_ticket;         /* tile order of the batch offset scan */
     unsigned int n_segments;             /* of the cells' sorted pairs (lists.cu) */
+    unsigned int pad;
     unsigned int order_offset;           /* where the tiles' order starts, in 256 bytes from here, or 0 */
     unsigned int group_total[kTileGroups];   /* instances per group of tiles */
     unsigned int class_total[kTileClasses], class_taken[kTileClasses];   /* tiles per class of list length */
