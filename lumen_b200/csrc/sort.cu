@@ -439,16 +439,19 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
  * A sort of so few keys is bound by latency: with the histogram and a launch
  * per digit, most of it went to launches (2.5 us each on the device, 4 us to
  * issue) and the passes' fixed 7 to 10 us. The sort of the depth keys, before
- * and after: 512 splats 27 -> 11 us, 50 k 34 -> 22, 100 k 40 -> 30, and four
- * launches fewer. Eight CTAs is the largest portable cluster and 16 keys per
- * thread what the shared memory holds, hence the limit; up to 1024 keys one
- * CTA does. */
+ * and after: 512 splats 27 -> 11 us, 50 k 34 -> 20, 100 k 40 -> 24, and four
+ * launches fewer. Up to 1024 keys one CTA does, up to 8192 eight (a key per
+ * thread; the largest portable cluster), beyond them sixteen where the device
+ * takes such a cluster (100 k keys: 24 us against 31 with eight). At 250 k keys
+ * the digit passes over the whole GPU are faster (65 us against 89), and eight
+ * CTAs hold 131072 keys (16 per thread), hence the limit. */
 constexpr int kClusterThreads = 1024;
 constexpr int kClusterItems = 16;
 constexpr int kClusterCtas = 8;
 constexpr int kClusterKeys = kClusterThreads * kClusterItems;   /* per CTA */
 constexpr int kClusterWarps = kClusterThreads / 32;
 constexpr int kCountParts = kClusterThreads / 256;
+static int g_cluster_ctas = kClusterCtas;   /* for more than a key per thread of eight CTAs */
 
 struct ClusterSmem {
     unsigned int keys[kClusterKeys], vals[kClusterKeys];
@@ -694,9 +697,11 @@ void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigne
                    SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int items,
                    int key_bytes, int num_sms, cudaStream_t st) {
     if (capacity <= (long long)kClusterCtas * kClusterKeys && key_bytes >= 4) {
-        const bool one = capacity <= kClusterThreads;
-        launch_chained_cluster(cluster_sort_kernel, one ? 1 : kClusterCtas, dim3(one ? 1 : kClusterCtas),
-                               dim3(kClusterThreads), sizeof(ClusterSmem), st, k0, v0, k1, v1, capacity, sc);
+        const int ctas = capacity <= kClusterThreads                  ? 1
+                         : capacity <= kClusterCtas * kClusterThreads ? kClusterCtas
+                                                                      : g_cluster_ctas;
+        launch_chained_cluster(cluster_sort_kernel, ctas, dim3(ctas), dim3(kClusterThreads), sizeof(ClusterSmem), st,
+                               k0, v0, k1, v1, capacity, sc);
         return;
     }
     launch_sort_items(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, items, key_bytes, nullptr, num_sms, st);
@@ -741,6 +746,23 @@ void launch_sorted_keys64(const LumenGpuFrame& f, const Control* ctrl, int key_m
 
 void configure_sort_kernels() {
     cudaFuncSetAttribute(cluster_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterSmem));
+    /* a cluster of 16 where the device can hold one */
+    cudaFuncSetAttribute(cluster_sort_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * kClusterCtas);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = sizeof(ClusterSmem);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2 * kClusterCtas;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, cluster_sort_kernel, &cfg) == cudaSuccess && clusters > 0)
+        g_cluster_ctas = 2 * kClusterCtas;
+    else
+        cudaGetLastError();
     cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(PassSmem<unsigned int, 8>));
     cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
