@@ -214,7 +214,7 @@ LumenStatus lumen_gpu_stage_timer_read(LumenGpuStageTimer* timer, float stage_ms
  * 256 or 512); *_sort_items: keys per thread in a digit pass of the depth
  * and cell sorts (depth: 8 or 16; cell: 8, 16 or 24 — tiles of 2048, 4096
  * or 6144 keys); sorts of up to 131072 depth keys and cell sorts of 257 to
- * 512 cells have one form only. Defaults 256, 16, 16. */
+ * 512 cells have one form only. Defaults 256, 16, 16 (8 for smaller frames). */
 typedef struct {
     int32_t composite_chunk;
     int32_t depth_sort_items;

@@ -245,6 +245,19 @@ void launch_init(const ScratchLayout& L, unsigned char* base, const BatchHeader*
                    (ViewTable*)(base + L.table_off), h, v, (int)(v0 != nullptr));
 }
 
+/* The launch parameters for so many projection slots. Digit passes run with
+ * smaller tiles where tiles of 4096 keys would leave SMs idle. The depth sort,
+ * up to three of those per SM: 250 k splats 227 -> 220 us per frame, 1 M 392.4
+ * -> 390.8, 2 M (beyond) 731.5 -> 732. The cell sort, whose pairs the host does
+ * not know, up to the slots of a one-kernel projection: 50 k splats 96.2 ->
+ * 93.4, 250 k (beyond) 220 -> 222. */
+static LaunchConfig default_launch(long long n_slots) {
+    LaunchConfig lc = kDefaultLaunch;
+    if (n_slots <= 3ll * device_sm_count() * kSortTile) lc.depth_sort_items = 8;
+    if (n_slots <= kOnePassBlocks * kProjThreads) lc.tile_sort_items = 8;
+    return lc;
+}
+
 static bool launch_ok(const LaunchConfig& lc) {
     return (lc.composite_chunk == 128 || lc.composite_chunk == 256 || lc.composite_chunk == 512) &&
            (lc.depth_sort_items == 8 || lc.depth_sort_items == 16) &&
@@ -275,7 +288,8 @@ static void single_view_table(const LumenGpuGaussians* g, const LumenViewCamera*
 
 static LumenStatus forward_impl(const LumenGpuGaussians* g, const LumenViewCamera* cam, const LumenRenderOptions* opt,
                                 LumenGpuFrame* f, LumenGpuImage* img, cudaEvent_t* ev, void* stream,
-                                LaunchConfig lc = kDefaultLaunch) {
+                                const LaunchConfig* chosen = nullptr) {
+    LaunchConfig lc = chosen ? *chosen : default_launch(g ? g->count : 0);
     if (!launch_ok(lc)) return LUMEN_ERROR_INVALID_ARGUMENT;
     if (img) lc.track = img->n_contrib || img->last_idx;
     LumenStatus st = check_inputs(g, cam, opt);
@@ -319,7 +333,8 @@ LumenStatus forward_banded(const LumenGpuGaussians* g, const LumenViewCamera* ca
     ViewDesc v{};
     single_view_table(g, cam, img, L, tiles, &hdr, &v);
     launch_init(L, base, &hdr, &v, s);
-    launch_pipeline(L, base, *opt, *f, g->count, tiles, hdr.total_cells, 1, false, kDefaultLaunch, nullptr, s, false,
+    const LaunchConfig lc = default_launch(g->count);
+    launch_pipeline(L, base, *opt, *f, g->count, tiles, hdr.total_cells, 1, false, lc, nullptr, s, false,
                     hdr.total_units);
     Control* ctrl = (Control*)(base + L.control_off);
     const ViewTable* vt = (const ViewTable*)(base + L.table_off);
@@ -328,7 +343,7 @@ LumenStatus forward_banded(const LumenGpuGaussians* g, const LumenViewCamera* ca
     for (int b = 0; b < n_bands; ++b) {
         const int r0 = (int)((long long)tiles_y * b / n_bands), r1 = (int)((long long)tiles_y * (b + 1) / n_bands);
         launch_composite(vt, 1, *f, ctrl, *opt, (long long)r0 * tiles_x, (long long)(r1 - r0) * tiles_x, false,
-                         kDefaultLaunch.composite_chunk, img->n_contrib || img->last_idx, sms, s);
+                         lc.composite_chunk, img->n_contrib || img->last_idx, sms, s);
         const int y0 = r0 * kTile, y1 = r1 * kTile < cam->height ? r1 * kTile : cam->height;
         if (after_band) after_band(ctx, y0, y1, s);
     }
@@ -401,7 +416,7 @@ static LumenStatus batch_impl(const LumenGpuBatchView* views, int n_views, const
     cudaError_t e = cudaMemcpyAsync(base + L.table_off, host.data(), host.size(), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return map_cuda(e);
     launch_init(L, base, nullptr, nullptr, s);
-    LaunchConfig lc = kDefaultLaunch;
+    LaunchConfig lc = default_launch(slots);
     lc.track = 0;
     for (int v = 0; v < n_views; ++v)
         if (views[v].image.n_contrib || views[v].image.last_idx) lc.track = 1;
@@ -438,9 +453,9 @@ LumenStatus lumen_gpu_render_forward_ex(const LumenGpuGaussians* g, const LumenV
                                         LumenGpuFrame* f, LumenGpuImage* img, LumenGpuStageTimer* t, void* stream) {
     if (!launch) return LUMEN_ERROR_INVALID_ARGUMENT;
     const LaunchConfig lc = {launch->composite_chunk, launch->depth_sort_items, launch->tile_sort_items, 1};
-    if (!t) return forward_impl(g, cam, opt, f, img, nullptr, stream, lc);
+    if (!t) return forward_impl(g, cam, opt, f, img, nullptr, stream, &lc);
     if (t->next >= t->max_frames) return LUMEN_ERROR_INVALID_ARGUMENT;
-    LumenStatus st = forward_impl(g, cam, opt, f, img, t->ev + (size_t)t->next * 5, stream, lc);
+    LumenStatus st = forward_impl(g, cam, opt, f, img, t->ev + (size_t)t->next * 5, stream, &lc);
     if (st == LUMEN_SUCCESS) t->next++;
     return st;
 }

@@ -119,11 +119,9 @@ struct LaunchConfig {
     int track;             /* 1: some view's image asks for contributor counts or last-visited
                               offsets (the compositor then keeps them); set by the host */
 };
-/* measured on B200 at 1080p with 1 M Gaussians: 256-instance compositor
- * chunks (0.156 against 0.157 ms for 128 and 0.175 for 512, which stages more
- * instances behind the pixels' last splat); 4096-key tiles
- * for both sorts (sort stage 0.1955 ms, against 0.1978 with 2048-key depth
- * tiles, 0.2002 with 6144-key and 0.2232 with 2048-key tile-sort tiles) */
+/* 256-instance compositor chunks (1 M Gaussians at 1080p: 0.152 ms against 0.153
+ * for 128 and 0.170 for 512, which stages more instances behind the pixels'
+ * last splat) and, for large frames, 4096-key tiles in both sorts */
 constexpr LaunchConfig kDefaultLaunch = {256, 16, 16, 1};
 
 __host__ __device__ constexpr inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
