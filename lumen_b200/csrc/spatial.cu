@@ -12,7 +12,9 @@
  *   K1 bbox_kernel      the cloud's box: per-axis min and max of the positions
  *                       (NaN skipped, as add_gaussian's comparisons skip it),
  *                       reduced with atomicMax on order-preserving bit keys
- *   K2 morton_kernel    one 30-bit code per Gaussian, index as the value
+ *   K2 morton_kernel    one 30-bit code per Gaussian, index as the value, and
+ *                       which bits of the codes vary (the sort skips digits
+ *                       that do not; a kernel of its own for this took 5 us)
  *   K3 the library's stable onesweep radix sort (32-bit keys, 4 digit passes)
  *   K4 bvh_levels_kernel, once per ten levels: a block writes 1024 leaves
  *                       (or loads 1024 nodes of the level reached so far)
@@ -42,7 +44,6 @@ LumenStatus map_cuda(cudaError_t e);
 LumenStatus status_from_flags(unsigned int flags);
 int device_sm_count();
 void configure_once();
-void launch_key_stats32(const unsigned int* keys, long long n, SortControl* sc, int num_sms, cudaStream_t st);
 void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1, long long capacity,
                    SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int items,
                    int key_bytes, int num_sms, cudaStream_t st);
@@ -51,7 +52,6 @@ namespace {
 
 constexpr int kMaxLevels = 40;        /* 2^30 leaves need 31 levels */
 constexpr int kRayStack = 64;         /* a traversal holds at most levels + 1 entries */
-constexpr int kBvhSortItems = 16;     /* 4096-key sort tiles */
 
 struct BvhControl {
     SortControl sort;
@@ -98,14 +98,14 @@ long long node_count_of(long long n) {
 
 BvhLayout make_layout(long long n) {
     BvhLayout B;
-    B.sort_tiles = (n + 256 * kBvhSortItems - 1) / (256 * kBvhSortItems);
+    B.sort_tiles = (n + kSortTileMin - 1) / kSortTileMin;
     B.control_off = 0;
     B.keys0_off = align_up(sizeof(BvhControl), 256);
     B.vals0_off = align_up(B.keys0_off + (size_t)n * 4, 256);
     B.keys1_off = align_up(B.vals0_off + (size_t)n * 4, 256);
     B.vals1_off = align_up(B.keys1_off + (size_t)n * 4, 256);
     B.lb_off = align_up(B.vals1_off + (size_t)n * 4, 256);
-    B.total = align_up(B.lb_off + (size_t)8 * (size_t)lookback_rows(B.sort_tiles > 0 ? B.sort_tiles : 1) * 256 * 4, 256);
+    B.total = align_up(B.lb_off + (size_t)4 * (size_t)lookback_rows(B.sort_tiles > 0 ? B.sort_tiles : 1) * 256 * 4, 256);
     return B;
 }
 
@@ -182,7 +182,7 @@ __device__ __forceinline__ unsigned int morton3(float nx, float ny, float nz) {
 }
 
 __global__ void __launch_bounds__(256)
-morton_kernel(const float* __restrict__ means, long long n, const BvhControl* __restrict__ ctrl,
+morton_kernel(const float* __restrict__ means, long long n, BvhControl* __restrict__ ctrl,
               unsigned int* __restrict__ keys, unsigned int* __restrict__ vals) {
     /* the box as add_gaussian leaves it: min from 1e9, max from -1e9 */
     float mn[3], inv[3];
@@ -202,14 +202,34 @@ morton_kernel(const float* __restrict__ means, long long n, const BvhControl* __
         mn[c] = lo;
         inv[c] = 1.0f / (extent > (float)0.001 ? extent : 1.0f);
     }
+    unsigned int key_or = 0u, key_or_not = 0u;
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const float nx = (means[i * 3 + 0] - mn[0]) * inv[0];                /* bvh.mojo:64-72 */
         const float ny = (means[i * 3 + 1] - mn[1]) * inv[1];
         const float nz = (means[i * 3 + 2] - mn[2]) * inv[2];
-        keys[i] = morton3(nx, ny, nz);
+        const unsigned int code = morton3(nx, ny, nz);
+        keys[i] = code;
         vals[i] = (unsigned int)i;
+        key_or |= code;
+        key_or_not |= ~code;
     }
+    /* the sort's key statistics, one atomic per block and word */
+    __shared__ unsigned int block_or, block_or_not;
+    if (threadIdx.x == 0) block_or = block_or_not = 0u;
+    __syncthreads();
+    key_or = __reduce_or_sync(0xffffffffu, key_or);
+    key_or_not = __reduce_or_sync(0xffffffffu, key_or_not);
+    if ((threadIdx.x & 31) == 0) {
+        atomicOr(&block_or, key_or);
+        atomicOr(&block_or_not, key_or_not);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicOr(&ctrl->sort.key_or, (unsigned long long)block_or);
+        atomicOr(&ctrl->sort.key_or_not, (unsigned long long)block_or_not);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->sort.n = (unsigned long long)n;
 }
 
 struct Box {
@@ -774,8 +794,9 @@ LumenStatus lumen_gpu_bvh_build(const LumenGpuGaussians* g, LumenGpuBvh* bvh, vo
     if (grid > (long long)sms * 8) grid = (long long)sms * 8;
     bbox_kernel<<<(unsigned int)grid, 256, 0, s>>>(g->means, n, ctrl);
     morton_kernel<<<(unsigned int)grid, 256, 0, s>>>(g->means, n, ctrl, k0, v0);
-    launch_key_stats32(k0, n, &ctrl->sort, sms, s);
-    launch_sort32(k0, v0, k1, v1, n, &ctrl->sort, lb, B.sort_tiles, &ctrl->error_flags, kBvhSortItems, 4, sms, s);
+    /* 2048-key tiles while 4096-key ones would leave SMs idle */
+    const int items = n <= 3ll * sms * kSortTile ? 8 : 16;
+    launch_sort32(k0, v0, k1, v1, n, &ctrl->sort, lb, B.sort_tiles, &ctrl->error_flags, items, 4, sms, s);
     for (int L0 = 0; L0 + 1 < lv.n_levels; L0 += kRefitSpan) {
         const long long blocks = (lv.count[L0] + kRefitNodes - 1) / kRefitNodes;
         bvh_levels_kernel<<<(unsigned int)blocks, kRefitThreads, 0, s>>>(g->means, g->scales, n, ctrl, v0, v1,
