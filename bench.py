@@ -39,21 +39,24 @@ METRIC = "1080p frames/s and p99 latency, served vs per-call render; fwd+bwd ste
 UNIT = "frames/s"
 N_GAUSSIANS = 1_000_000
 WIDTH, HEIGHT = 1920, 1080
-# DRAM bytes (read + write) of one composite_kernel<512> launch at the 1 M-Gaussian
+# DRAM bytes (read + write) of one composite_kernel launch at the 1 M-Gaussian
 # 1080p workload, from an ncu capture (profiles/forward_config1_kernels.md)
 COMPOSITE_DRAM_BYTES = 43.5e6
-def kernels_per_frame(n_tiles: int) -> int:
-    """Kernels one forward frame launches: init; the projection's count,
-    offset scan and projection; the depth sort's histogram and 4 digit
-    passes; the emission (which also counts the tile sort's digits); one
-    tile-sort digit pass per byte a tile id can vary in; tile ranges;
-    composite."""
-    tile_bytes = 0
-    t = n_tiles - 1
-    while t > 0:
-        tile_bytes += 1
-        t >>= 8
-    return 1 + 3 + (1 + 4) + 1 + tile_bytes + 1 + 1
+def cells_of(width: int, height: int) -> int:
+    """Cells of 4x4 tiles (64x64 pixels) of a view."""
+    return ((width + 63) // 64) * ((height + 63) // 64)
+
+
+def kernels_per_frame(slots: int, cells: int, views: int = 1) -> int:
+    """Kernels one forward frame or batch launches: init; the projection (one
+    kernel for a view of up to 131072 Gaussians, else count, offset scan and
+    projection); the depth sort (one kernel for as many, else a histogram and 4
+    digit passes); the emission (which also counts the cell sort's digits); one
+    cell-sort digit pass per byte a cell id can vary in, or one nine-bit pass
+    for 257 to 512 cells; the lists' count, scan and write; composite."""
+    cell_passes = 1 if 256 < cells <= 512 else ((cells - 1).bit_length() + 7) // 8
+    small = slots <= 131072
+    return 1 + (1 if small and views == 1 else 3) + (1 if small else 5) + 1 + cell_passes + 3 + 1
 
 
 def parse():
@@ -688,7 +691,7 @@ def multiview_leg(dev, steps, warmup, hbm_peak):
             "per_call_views_per_s": n_views * 1000.0 / ms_single, "per_call_ms_for_64": ms_single,
             "stages_ms": {k: round(v / steps, 4) for k, v in zip(["project", "sort", "tile_ranges", "composite"],
                                                                  stage)},
-            "visible": V, "instances": K, "tiles": T, "digit_passes": p, "gpu_launches_per_batch": kernels_per_frame(T),
+            "visible": V, "instances": K, "tiles": T, "digit_passes": p, "gpu_launches_per_batch": kernels_per_frame(n * n_views, n_views * cells_of(W, H), n_views),
             "roofline": {"bytes": b, "achieved": b / (ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                          "frac": b / (ms * 1e-3) / 1e9 / hbm_peak}}
 
@@ -1118,7 +1121,7 @@ def main():
             "ms_per_step": ms_max, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32", "data": "synthetic",
             "config": workload_config({"parallelism": f"replicas x{world}" if world > 1 else "single GPU"}),
-            "gpu_launches": kernels_per_frame(T) * steps,
+            "gpu_launches": kernels_per_frame(N_GAUSSIANS, cells_of(WIDTH, HEIGHT)) * steps,
             "clocks": clk.summary(),
             "stages_ms": {n: round(v, 4) for n, v in zip(names, stage_ms)},
             "stages_timing": "a second run of the K frames with CUDA events between the stages",

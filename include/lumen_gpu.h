@@ -156,7 +156,7 @@ typedef struct {
 size_t lumen_gpu_scratch_bytes(int64_t n_gaussians, int64_t instance_capacity, int64_t n_tiles);
 
 /* Enqueue the whole forward on `stream`: project + cull + SH + compacting
- * scan + key emit, histogram, stable LSD digit passes, tile ranges,
+ * scan, depth sort, emission and sort by cells, the tiles' lists and ranges,
  * compositing. Does not wait. */
 LumenStatus lumen_gpu_render_forward(const LumenGpuGaussians* gaussians, const LumenViewCamera* camera,
                                      const LumenRenderOptions* options, LumenGpuFrame* frame,
@@ -194,8 +194,8 @@ LumenStatus lumen_gpu_sort_pairs(uint64_t* keys0, uint32_t* vals0, uint64_t* key
 
 /* Stage timing with CUDA events on the render stream. A timer holds events
  * for up to max_frames frames; each lumen_gpu_render_forward_timed call
- * records 5 events (before K1, after K1, after the sort, after the ranges,
- * after compositing) into the next frame slot without waiting.
+ * records 5 events (before K1, after K1, after the sort, after the tiles'
+ * lists, after compositing) into the next frame slot without waiting.
  * lumen_gpu_stage_timer_read waits for the last event and returns the summed
  * milliseconds of the 4 stages over the recorded frames, then resets.
  * No counterpart in the reference (its timers are perf_counter_ns and clock(),

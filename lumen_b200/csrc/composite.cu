@@ -5,11 +5,11 @@
  * src/raster/pipeline.mojo:172-229, with compute_gaussian_pixel_alpha and
  * PixelAccumulator.blend/finalize, src/raster/compositor.mojo:10-89.
  *
- * One CTA of 128 threads per 16x16 tile. A group of 8 lanes shades a 4x4 block of pixels, a lane two
- * pixels one above the other, so a warp holds four blocks (an 8x8 quadrant)
- * that walk four lists of their own in step. The tile's sorted instances are
- * processed in chunks of 128, 256 or 512 (a launch parameter the autotuner
- * picks): the threads gather the chunk's 48-byte records (through the sorted
+ * One CTA of 128 threads per 16x16 tile. A group of 8 lanes shades a 4x4
+ * block of pixels, a lane two pixels one above the other, so a warp holds
+ * four blocks (an 8x8 quadrant) that walk four lists of their own in step.
+ * The tile's sorted instances are processed in chunks of 128, 256 or 512 (a
+ * launch parameter the autotuner picks): the threads gather the chunk's 48-byte records (through the sorted
  * visible index) into shared memory and compute which blocks each splat can
  * reach at all (reach_blocks); each warp then builds its four lists and walks
  * them in sorted order, so each pixel blends exactly the reference's

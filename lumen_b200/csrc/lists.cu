@@ -23,9 +23,9 @@
  * and moves 8 B per instance five times. A splat covers about 7 tiles but 2
  * cells, so the ranked pairs are 3 to 4 times fewer, and the split needs no
  * ranking. The instances are written once. From the depth order to the ranges,
- * emission included, this took (us, before -> after): 1 M splats at
- * 1080p 160 -> 130, 2 M at 4K 455 -> 260, 64 views of 300 k at 720p
- * 2400 -> 1330, 512 splats at 800x600 34 -> 32.
+ * emission included, this took (us, before -> after): 1 M splats at 1080p
+ * 160 -> 115, 2 M at 4K 455 -> 235, 64 views of 300 k at 720p 2400 -> 1320,
+ * 512 splats at 800x600 34 -> 32.
  */
 #include "splat_common.cuh"
 
