@@ -41,7 +41,7 @@ N_GAUSSIANS = 1_000_000
 WIDTH, HEIGHT = 1920, 1080
 # DRAM bytes (read + write) of one composite_kernel launch at the 1 M-Gaussian
 # 1080p workload, from an ncu capture (profiles/forward_config1_kernels.md)
-COMPOSITE_DRAM_BYTES = 43.5e6
+COMPOSITE_DRAM_BYTES = 51.7e6
 def cells_of(width: int, height: int) -> int:
     """Cells of 4x4 tiles (64x64 pixels) of a view."""
     return ((width + 63) // 64) * ((height + 63) // 64)
@@ -911,7 +911,7 @@ def serving_leg(dev, n_requests, hbm_budget):
                 "requeued_batches": s1["requeued_batches"] - s0["requeued_batches"],
                 "explored_batches_in_timed_runs": s1["explored_batches"] - s0["explored_batches"]}
     # the bound: what a batch of 1080p views of the 1M scene costs per view, by stage, at the
-    # server's largest batch of such views (8: 65 280 tiles; a ninth view adds a tile-sort pass)
+    # server's largest batch of such views (8: 65 280 tiles)
     ceil = _batch_ceiling(dev, dscenes[sizes.index(1_000_000)], lib, opt, 8)
     per_view_unshared = ceil["sort"] + ceil["tile_ranges"] + ceil["composite"]
     out["ceiling_1080p_1M"] = {
@@ -1110,7 +1110,7 @@ def main():
            "composite": 40 * K + 16 * P}
     # the dominant kernel: composite_kernel, the largest share of the frame's
     # launch list (profiles/forward_config1_launches.md); the sort stage is
-    # nine kernels, none above an eighth of the frame
+    # seven kernels, none above a tenth of the frame
     dom = names.index("composite")
     dname = names[dom]
     achieved = alg[dname] / (stage_ms[dom] * 1e-3) / 1e9

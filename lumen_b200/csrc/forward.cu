@@ -605,7 +605,7 @@ LumenStatus lumen_gpu_sort_pairs(uint64_t* keys0, uint32_t* vals0, uint64_t* key
     unsigned long long* k0 = reinterpret_cast<unsigned long long*>(keys0);
     unsigned long long* k1 = reinterpret_cast<unsigned long long*>(keys1);
     launch_key_stats64(k0, n, &ctrl->cell_sort, sms, s);
-    /* the tile-sort look-back region holds 8 digits x tiles x 256 entries */
+    /* the cell sort's look-back region holds 8 digits x tiles x 256 entries */
     launch_sort64(k0, vals0, k1, vals1, n, &ctrl->cell_sort, (unsigned int*)(base + L.tile_lb_off), L.sort_tiles,
                   &ctrl->error_flags, sms, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return map_cuda(e);

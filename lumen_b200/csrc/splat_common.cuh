@@ -155,7 +155,7 @@ struct ViewDesc {
     long long block_begin;
     long long tile_begin;
     long long cell_begin;     /* batch-wide id of the view's cell 0 */
-    long long inst_begin;     /* first tile-sorted instance of the view, or -1
+    long long inst_begin;     /* first instance of the view in the lists, or -1
                                  (written on the device by the list scan) */
     long long unit_begin;     /* batch projection: the first unit of the view's scene group
                                  when the view leads the group (units of the views before it
