@@ -41,7 +41,8 @@ void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigne
                    SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int items,
                    int key_bytes, int num_sms, cudaStream_t st);
 void launch_cell_sort(const LumenGpuFrame& f, Control* ctrl, const ViewTable* vt, unsigned int* lb,
-                      long long lb_tiles_cap, int items, int key_bytes, bool wide, int num_sms, cudaStream_t st);
+                      long long lb_tiles_cap, int items, CellDigits digits, bool wide, bool persistent, int num_sms,
+                      cudaStream_t st);
 void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned char* scratch, long long room_offset,
                   long long room_bytes, long long n_cells, long long n_tiles, int num_sms, cudaStream_t st);
 void launch_sort64(unsigned long long* k0, unsigned int* v0, unsigned long long* k1, unsigned int* v1,
@@ -215,10 +216,9 @@ void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRen
                     sms, s);
         /* the cell-sort region holds 4 passes of 2048-key tiles; cell ids
          * below n_cells (the batch's, or the bound a persistent launch is
-         * sized for) vary in their low ceil(log2(n_cells) / 8) bytes only */
-        int cell_bytes = 0;
-        for (long long t = n_cells - 1; t > 0; t >>= 8) ++cell_bytes;
-        launch_cell_sort(f, ctrl, vt, cell_lb, 2 * L.sort_tiles, lc.tile_sort_items, cell_bytes, wide, sms, s);
+         * sized for) have that many digits at most */
+        launch_cell_sort(f, ctrl, vt, cell_lb, 2 * L.sort_tiles, lc.tile_sort_items, CellDigits(n_cells), wide,
+                         persistent, sms, s);
     } else if (ev) {
         cudaEventRecord(ev[1], s);
     }

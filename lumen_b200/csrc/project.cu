@@ -343,13 +343,12 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
     const long long V = ctrl->n_visible;
     const unsigned int* order = ctrl->depth_sort.sorted_buffer ? f.depth_order[1] : f.depth_order[0];
     const unsigned int cap = (unsigned int)f.instance_capacity;   /* below 2^30 */
-    /* the cell-id bytes that can vary: ids are below the batch's cell count */
+    /* the digits of the cell ids, which are below the batch's cell count */
     const long long n_cells = vt->hdr.total_cells;
     const bool packed = n_cells <= kPackedCells;
-    int nd = 0;
-    for (long long t = n_cells - 1; t > 0 && nd < 4; t >>= 8) ++nd;
-    const unsigned int digit_mask = wide ? kWideCells - 1 : 0xFFu;
-    if (wide) nd = 1;   /* one digit of 9 bits, in two rows of counts */
+    const CellDigits digits(n_cells);
+    const int nd = wide ? 1 : digits.n, bits = wide ? 9 : digits.bits;   /* nine bits: in two rows of counts */
+    const unsigned int digit_mask = (1u << bits) - 1u;
     const int rows = wide ? 2 : nd;
     for (int d = 0; d < 4; ++d) s.hist[d][tid] = 0u;
     if (int* ranges = cell_ranges(f, ctrl, vt)) {
@@ -456,7 +455,7 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
                 kor |= cell;
                 knot |= ~cell;
                 atomicAdd(&s.hist[0][0] + (cell & digit_mask), 1u);
-                for (int d = 1; d < nd; ++d) atomicAdd(&s.hist[d][(cell >> (8 * d)) & 0xFFu], 1u);
+                for (int d = 1; d < nd; ++d) atomicAdd(&s.hist[d][(cell >> (bits * d)) & digit_mask], 1u);
             };
             if (lanes) {
                 /* A cell's mask is what the rectangle's four sides leave of

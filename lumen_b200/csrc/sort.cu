@@ -26,11 +26,11 @@
 
 namespace lumen {
 
-__device__ __forceinline__ unsigned int varying_digits(const SortControl* c, int nbytes) {
+__device__ __forceinline__ unsigned int varying_digits(const SortControl* c, int nbytes, int bits = 8) {
     const unsigned long long v = c->key_or & c->key_or_not;
     unsigned int m = 0;
     for (int d = 0; d < nbytes; ++d)
-        if ((v >> (8 * d)) & 0xFFull) m |= 1u << d;
+        if ((v >> (bits * d)) & ((1ull << bits) - 1ull)) m |= 1u << d;
     return m;
 }
 
@@ -245,15 +245,18 @@ __device__ __forceinline__ void cell_edges(int* ranges, unsigned int id_mask, co
 template <typename KeyT, int kItems, int kThreads>
 constexpr int kPassCtas = sizeof(KeyT) == 4 && kThreads == 256 ? (kItems <= 8 ? 4 : kItems <= 16 ? 3 : 2) : 2;
 
-/* kItems keys per thread: tiles of kThreads * kItems keys. */
-template <typename KeyT, int kItems, int kThreads = kSortThreads>
+/* kItems keys per thread: tiles of kThreads * kItems keys. kCellDigits: digits
+ * of the width that CellDigits gives (a constant width where it is 8: the
+ * depth passes of 250 k splats are 1 us faster each). */
+template <typename KeyT, int kItems, int kThreads = kSortThreads, bool kCellDigits = false>
 __global__ void __launch_bounds__(kThreads, (kPassCtas<KeyT, kItems, kThreads>))
 onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, long long capacity, SortControl* sc,
                      unsigned int* lb_all, long long lb_tiles_cap, unsigned int* err, int digit, CellSink sink) {
     chain_begin();
     constexpr int kTileKeys = kThreads * kItems;
     constexpr int kWarps = kThreads / 32;
-    constexpr unsigned int kDigit = kThreads - 1;   /* a digit's bits */
+    const int bits = kThreads != 256 ? 9 : kCellDigits ? CellDigits(sink.vt->hdr.total_cells).bits : 8;
+    const unsigned int digit_mask = (1u << bits) - 1u;   /* a digit's bits */
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using Smem = PassSmem<KeyT, kItems, kThreads>;
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
@@ -261,7 +264,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
     /* the digits that vary, from the producer's key statistics (the same
      * rule as the histogram kernel's, for sorts whose histogram the producer
      * counted) */
-    unsigned int varying = sort_count(sc, capacity) > 1 ? varying_digits(sc, (int)sizeof(KeyT)) : 0u;
+    unsigned int varying = sort_count(sc, capacity) > 1 ? varying_digits(sc, (int)sizeof(KeyT), kThreads == 256 ? bits : 8) : 0u;
     if (kThreads != 256) varying = varying ? 1u : 0u;   /* one digit */
     if (blockIdx.x == 0 && tid == 0) {
         sc->varying = varying;
@@ -275,7 +278,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
     unsigned int* __restrict__ vout = src ? v0 : v1;
     const long long K = sort_count(sc, capacity);
     const long long ntiles = (K + kTileKeys - 1) / kTileKeys;
-    const int shift = 8 * digit;
+    const int shift = bits * digit;
     unsigned int* lb = lb_all + (size_t)digit * (size_t)lookback_rows(lb_tiles_cap) * kThreads;
     unsigned int* groups = lb + (size_t)lb_tiles_cap * kThreads;
     int* edges = nullptr;
@@ -332,7 +335,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
          * look-back chain of the tiles after it moves on sooner */
 #pragma unroll
         for (int it = 0; it < kItems; ++it)
-            if (wbase + it * 32 + lane < K) atomicAdd(&s.whist[warp][(unsigned int)((k[it] >> shift) & kDigit)], 1u);
+            if (wbase + it * 32 + lane < K) atomicAdd(&s.whist[warp][(unsigned int)((k[it] >> shift) & digit_mask)], 1u);
         __syncthreads();
         /* digit t: warp-exclusive offsets and the tile's count */
         const int t = tid;
@@ -375,7 +378,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
 #pragma unroll
         for (int it = 0; it < kItems; ++it) {
             const bool valid = wbase + it * 32 + lane < K;
-            const unsigned int d = (unsigned int)((k[it] >> shift) & kDigit);
+            const unsigned int d = (unsigned int)((k[it] >> shift) & digit_mask);
             unsigned int* mk = s.match[it % Smem::kSets][warp];
             if (valid) atomicOr(&mk[d], 1u << lane);
             __syncwarp();
@@ -409,7 +412,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
             for (int it = 0; it < kItems; ++it) {
                 const int j = it * kThreads + tid;
                 const KeyT kk = s.keys[j];
-                const unsigned int d = (unsigned int)((kk >> shift) & kDigit);
+                const unsigned int d = (unsigned int)((kk >> shift) & digit_mask);
                 const long long out = s.gbase[d] + j;
                 kout[out] = kk;
                 vout[out] = s.vals[j];
@@ -418,7 +421,7 @@ onesweep_pass_kernel(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lon
         } else {
             for (int j = tid; j < nvalid; j += kThreads) {
                 const KeyT kk = s.keys[j];
-                const unsigned int d = (unsigned int)((kk >> shift) & kDigit);
+                const unsigned int d = (unsigned int)((kk >> shift) & digit_mask);
                 const long long out = s.gbase[d] + j;
                 kout[out] = kk;
                 vout[out] = s.vals[j];
@@ -654,7 +657,7 @@ __global__ void sorted_keys64_kernel(const unsigned int* k0, const unsigned int*
 /* key_bytes: the low bytes that can vary at all (a pass per byte is
  * launched; among those, passes over bytes that turn out constant exit at
  * once). */
-template <typename KeyT, int kItems, int kThreads = kSortThreads>
+template <typename KeyT, int kItems, int kThreads = kSortThreads, bool kCellDigits = false>
 void launch_sort_impl(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, long long capacity, SortControl* sc,
                       unsigned int* lb, long long lb_tiles_cap, unsigned int* err, int key_bytes, int num_sms,
                       cudaStream_t st, const CellSink* sink = nullptr) {
@@ -671,26 +674,22 @@ void launch_sort_impl(KeyT* k0, unsigned int* v0, KeyT* k1, unsigned int* v1, lo
     const int ctas_per_sm = kPassCtas<KeyT, kItems, kThreads>;   /* all CTAs resident */
     const int nd = key_bytes < (int)sizeof(KeyT) ? key_bytes : (int)sizeof(KeyT);
     for (int d = 0; d < nd; ++d)
-        launch_chained(onesweep_pass_kernel<KeyT, kItems, kThreads>, dim3(num_sms * ctas_per_sm), dim3(kThreads), smem, st,
+        launch_chained(onesweep_pass_kernel<KeyT, kItems, kThreads, kCellDigits>, dim3(num_sms * ctas_per_sm), dim3(kThreads), smem, st,
                        k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, d, sink ? *sink : CellSink{});
 }
 
 /* items: keys per thread of a digit pass, 8, 16 or 24 (tiles of 2048, 4096
  * or 6144 keys); lb_tiles_cap must hold ceil(capacity / (256 * items))
  * tiles. */
+template <bool kCellDigits>
 static void launch_sort_items(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1,
                               long long capacity, SortControl* sc, unsigned int* lb, long long lb_tiles_cap,
                               unsigned int* err, int items, int key_bytes, const CellSink* sink, int num_sms,
                               cudaStream_t st) {
-    if (items == 8)
-        launch_sort_impl<unsigned int, 8>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, key_bytes, num_sms, st,
-                                          sink);
-    else if (items == 24)
-        launch_sort_impl<unsigned int, 24>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, key_bytes, num_sms,
-                                           st, sink);
-    else
-        launch_sort_impl<unsigned int, 16>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, key_bytes, num_sms,
-                                           st, sink);
+    auto run = [&](auto kernel) { kernel(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, key_bytes, num_sms, st, sink); };
+    if (items == 8) run(launch_sort_impl<unsigned int, 8, kSortThreads, kCellDigits>);
+    else if (items == 24) run(launch_sort_impl<unsigned int, 24, kSortThreads, kCellDigits>);
+    else run(launch_sort_impl<unsigned int, 16, kSortThreads, kCellDigits>);
 }
 
 void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigned int* v1, long long capacity,
@@ -704,14 +703,16 @@ void launch_sort32(unsigned int* k0, unsigned int* v0, unsigned int* k1, unsigne
                                k0, v0, k1, v1, capacity, sc);
         return;
     }
-    launch_sort_items(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, items, key_bytes, nullptr, num_sms, st);
+    launch_sort_items<false>(k0, v0, k1, v1, capacity, sc, lb, lb_tiles_cap, err, items, key_bytes, nullptr, num_sms,
+                             st);
 }
 
 /* The frame's cell sort: the emission has counted the pairs' digits, cleared
  * the look-back tiles and filled the cells' ranges with -1, so only the digit
  * passes run, the last of which writes the ranges. */
 void launch_cell_sort(const LumenGpuFrame& f, Control* ctrl, const ViewTable* vt, unsigned int* lb,
-                      long long lb_tiles_cap, int items, int key_bytes, bool wide, int num_sms, cudaStream_t st) {
+                      long long lb_tiles_cap, int items, CellDigits digits, bool wide, bool persistent, int num_sms,
+                      cudaStream_t st) {
     const CellSink sink{ctrl, vt, f};
     if (wide) {
         launch_sort_impl<unsigned int, kWideItems, kWideCells>(
@@ -719,8 +720,10 @@ void launch_cell_sort(const LumenGpuFrame& f, Control* ctrl, const ViewTable* vt
             &ctrl->error_flags, 1, num_sms, st, &sink);
         return;
     }
-    launch_sort_items(f.keys[0], f.vals[0], f.keys[1], f.vals[1], f.instance_capacity, &ctrl->cell_sort, lb,
-                      lb_tiles_cap, &ctrl->error_flags, items, key_bytes, &sink, num_sms, st);
+    /* persistent launches learn the cells, and with them the width, on the device */
+    auto run = persistent || digits.bits != 8 ? launch_sort_items<true> : launch_sort_items<false>;
+    run(f.keys[0], f.vals[0], f.keys[1], f.vals[1], f.instance_capacity, &ctrl->cell_sort, lb, lb_tiles_cap,
+        &ctrl->error_flags, items, digits.n, &sink, num_sms, st);
 }
 
 void launch_sort64(unsigned long long* k0, unsigned int* v0, unsigned long long* k1, unsigned int* v1,
@@ -759,15 +762,18 @@ void configure_sort_kernels() {
         g_cluster_ctas = 2 * kClusterCtas;
     else
         cudaGetLastError();
-    cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(PassSmem<unsigned int, 8>));
-    cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(PassSmem<unsigned int, 16>));
+    auto allow = [](auto kernel, size_t smem) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    };
+    allow(onesweep_pass_kernel<unsigned int, 8>, sizeof(PassSmem<unsigned int, 8>));
+    allow(onesweep_pass_kernel<unsigned int, 16>, sizeof(PassSmem<unsigned int, 16>));
+    allow(onesweep_pass_kernel<unsigned int, 24>, sizeof(PassSmem<unsigned int, 24>));
+    allow(onesweep_pass_kernel<unsigned int, 8, kSortThreads, true>, sizeof(PassSmem<unsigned int, 8>));
+    allow(onesweep_pass_kernel<unsigned int, 16, kSortThreads, true>, sizeof(PassSmem<unsigned int, 16>));
+    allow(onesweep_pass_kernel<unsigned int, 24, kSortThreads, true>, sizeof(PassSmem<unsigned int, 24>));
     cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, kWideItems, kWideCells>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(PassSmem<unsigned int, kWideItems, kWideCells>));
-    cudaFuncSetAttribute(onesweep_pass_kernel<unsigned int, 24>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(PassSmem<unsigned int, 24>));
     cudaFuncSetAttribute(onesweep_pass_kernel<unsigned long long, kSort64Items>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(PassSmem<unsigned long long, kSort64Items>));

@@ -68,6 +68,12 @@ def test_cell_sort_in_one_pass(n, size):
     _check(_scene(n, size[0] + n, scale=(0.01, 0.4)), _cam(*size))
 
 
+@pytest.mark.parametrize("width", [52416, 52432])
+def test_cell_digits_of_equal_width(width):
+    """4095 cells (12 bits) are sorted as six and six bits, 4100 (13) as eight and five."""
+    _check(_scene(2000, width, scale=(0.0005, 0.1), spread=(1.0, 0.004)), _cam(width, 320))
+
+
 # 2040 cells: the notes of 80 B per cell do not fit the scratch of so few instances, and the cells'
 # ranges do not fit the depth keys of 300 splats
 @pytest.mark.parametrize("n", [300, 5000])
