@@ -26,22 +26,32 @@
  *
  * The work is split as in the compositor: two pixels per lane in packed FP32,
  * groups of 8 lanes with a 4x4 block and a splat list of their own. A splat's
- * 10 gradients are sums over the block's pixels of two scalars, s = dL/dpower
- * and w = alpha T: s times 1, dx, dy, dx^2, dx dy, dy^2 (the centre, the conic
- * and, divided by the opacity, the opacity) and w times the pixel's upstream
- * gradient (colour and depth). So a lane only forms s and w for its pixels and
- * leaves them in shared memory; after eight list steps every lane takes one
- * of the warp's 32 (splat, block) entries, reads its 16 pixels and forms the
- * sums, with dx per column and dy per row, and adds them to the Gaussian with
- * three vector atomics.
+ * 10 gradients are sums over the block's pixels of two scalars, s =
+ * -dL/dopacity and w = alpha T: s times the opacity is dL/dpower, which goes
+ * with dx^2, dx dy, dy^2 to the conic and with the power's derivatives to the
+ * centre; w goes with the pixel's upstream gradient to colour and depth. So a
+ * lane only forms s and w for its pixels and leaves them in shared memory;
+ * after eight list steps every lane takes one of the warp's 32 (splat, block)
+ * entries, reads its 16 pixels, forms the sums, with dx per column and dy per
+ * row, and adds them to the warp's sums for the splat. At a chunk's end a
+ * thread per splat adds the four warps' sums and sends the tile's to the
+ * Gaussian with three vector atomics.
  *
- * Bound by what shared memory delivers (its pipe 73% busy at 500 k Gaussians
- * and 1080p; issue 56%, FMA 23%, ALU 38%), so staged splats are read as 10
- * words and the rows lie without bank conflicts. Measured there on a B200:
- * 0.428 ms with one pixel per thread, 10 values per pixel summed over the
- * warp by a transpose and over the CTA by shared atomics (356 M warp
- * instructions); 0.227 ms in this form (145 M), of which staging and lists
- * take 0.09, the walk 0.09, the sums 0.03 and the atomics 0.015.
+ * A Gaussian's gradients are thus sums over tiles of sums that do not depend
+ * on the order of the warps. Sent block by block, the running sums took 16
+ * times as many additions, and their error went into the rotations of needles
+ * (the conic's way back to the covariance cancels three to four digits): over
+ * 500 k Gaussians at 1080p single quaternion gradients then scattered by 8e-4
+ * of the typical one where they now do by 2.5e-4, and a splat over the whole
+ * screen could lose 2e-3 of its colour's gradient.
+ *
+ * Bound by what shared memory delivers, so staged splats are read as 10 words
+ * and the rows lie without bank conflicts, and by the four CTAs per SM that its
+ * sums leave room for. Measured on a B200 at 500 k Gaussians and 1080p: 0.425
+ * ms with one pixel per thread, 10 values per pixel summed over the warp by a
+ * transpose and over the CTA by shared atomics; 0.300 ms in this form (0.230
+ * with an atomic per block and six CTAs; the warps' sums by shared atomics,
+ * which need a quarter of the room: 0.343).
  *
  * K7 project_backward_kernel: per Gaussian, the chain rule through the
  * conic inverse, the EWA product T Sigma T^T with T = J W, the projective
@@ -81,8 +91,10 @@ struct BackwardSmem {
     float4 col[kBwdChunk + 1];    /* g, b, depth, - */
     __align__(16) unsigned short mask[kBwdChunk];
     unsigned short list[kBlocks][kBwdChunk + 8];   /* byte offsets (16 x slot), as in the forward */
-    unsigned int gid[kBwdChunk + 1];
     ulonglong2 rows[kBwdThreads / 32][2 * kRowsW];
+    /* per warp and slot: the sums over the warp's pixels, in the order of splat2d */
+    float4 acc0[kBwdThreads / 32][kBwdChunk], acc1[kBwdThreads / 32][kBwdChunk];
+    float2 acc2[kBwdThreads / 32][kBwdChunk];
     /* per group and channel: dL/d(r, g, b, depth) of its pixels, 16 values in 4 units */
     ulonglong2 grad[kBwdThreads / 32][4][4 * kChannels + 1];
     int tile_last;
@@ -101,7 +113,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 template <bool kDepth>
 __device__ __forceinline__ bool stage_chunk(BackwardSmem<kDepth>& s, const LumenSplatRecord* __restrict__ records,
                                             const unsigned int* __restrict__ vals, unsigned int& next,
-                                            const unsigned int* __restrict__ visible_ids, unsigned int n_visible,
+                                            const unsigned int* __restrict__ visible_ids, unsigned int& gid,
+                                            unsigned int n_visible,
                                             Control* ctrl, int cs, int end, float tile_x0, float tile_y0) {
     static_assert(kBwdChunk == kBwdThreads, "one slot per thread");
     int high = 0;
@@ -127,7 +140,7 @@ __device__ __forceinline__ bool stage_chunk(BackwardSmem<kDepth>& s, const Lumen
                 s.geo[slot] = make_float4(geo.x, -geo.y, -0.5f * con.x, con.y);
                 s.con[slot] = make_float4(0.5f * con.z, geo.w, -fminf(4.5f, faint + 1e-3f), col.x);
                 s.col[slot] = make_float4(col.y, col.z, geo.z, 0.0f);
-                s.gid[slot] = visible_ids[v];
+                gid = visible_ids[v];
                 bool finite;
                 m = reach_blocks(geo, con, tile_x0, tile_y0, &finite);
                 finite = finite && fabsf(col.x) + fabsf(col.y) + fabsf(col.z) + fabsf(geo.z) < 1e15f;
@@ -204,16 +217,16 @@ __device__ __forceinline__ float fast_rcp(float x) {
     return r;
 }
 
-/* A lane's two pixels: the transmittance, R = G . C - g_tail - G . P (what
- * the splats behind contribute) and the negated upstream gradient, as packed
- * pairs; end: 16 x the chunk slot of the last splat each pixel visited. */
+/* A lane's two pixels: the transmittance, R = G . C - g_tail, the running
+ * -G . P and the negated upstream gradient, as packed pairs; end: 16 x the
+ * chunk slot of the last splat each pixel visited. */
 struct GradPair {
-    f32x2 T, R, nr, ng, nb, nd;
+    f32x2 T, R, nP, nr, ng, nb, nd;
     int end[2];
 };
 
-/* One list entry for the lane's two pixels: s = dL/dpower and w = alpha T of
- * each, zero where the pixel did not blend the splat. Every staged value and
+/* One list entry for the lane's two pixels: s = -dL/dopacity and w = alpha T
+ * of each, zero where the pixel did not blend the splat. Every staged value and
  * upstream gradient is finite. */
 template <bool kClamp, bool kDepth>
 __device__ __forceinline__ void backward_step(const BackwardSmem<kDepth>& sm, unsigned int off, float pxc, f32x2 pyc,
@@ -245,27 +258,32 @@ __device__ __forceinline__ void backward_step(const BackwardSmem<kDepth>& sm, un
         if (unsure0) b0 = !(__fmul_rn(op, lumen_expf_core(x0)) < min_alpha());
         if (unsure1) b1 = !(__fmul_rn(op, lumen_expf_core(x1)) < min_alpha());
     }
-    float a0 = op * fast_exp(x0), a1 = op * fast_exp(x1);
+    float e0 = fast_exp(x0), e1 = fast_exp(x1);
+    if (kClamp) {
+        /* near the 0.99 clamp likewise */
+        if (fabsf(__fmul_rn(op, e0) - (float)0.99) <= 4e-6f) e0 = lumen_expf_core(x0);
+        if (fabsf(__fmul_rn(op, e1) - (float)0.99) <= 4e-6f) e1 = lumen_expf_core(x1);
+    }
+    const f32x2 e = pack2(b0 ? e0 : 0.0f, b1 ? e1 : 0.0f);
+    f32x2 alpha = mul2(splat2(op), e);
     bool c0 = false, c1 = false;
     if (kClamp) {
-        /* near the 0.99 clamp likewise; a clamped alpha passes no gradient on */
-        if (fabsf(a0 - (float)0.99) <= 4e-6f) a0 = __fmul_rn(op, lumen_expf_core(x0));
-        if (fabsf(a1 - (float)0.99) <= 4e-6f) a1 = __fmul_rn(op, lumen_expf_core(x1));
+        /* a clamped alpha passes no gradient on */
+        float a0, a1;
+        unpack2(alpha, a0, a1);
         c0 = a0 > (float)0.99;
         c1 = a1 > (float)0.99;
-        a0 = fminf(a0, (float)0.99);
-        a1 = fminf(a1, (float)0.99);
+        alpha = pack2(fminf(a0, (float)0.99), fminf(a1, (float)0.99));
     }
-    const f32x2 alpha = pack2(b0 ? a0 : 0.0f, b1 ? a1 : 0.0f);
     const f32x2 w = mul2(alpha, p.T);
-    f32x2 ngcol = fma2(splat2(c.w), p.nr, fma2(splat2(k.x), p.ng, mul2(splat2(k.y), p.nb)));
+    f32x2 ngcol = fma2(splat2(k.y), p.nb, fma2(splat2(c.w), p.nr, mul2(splat2(k.x), p.ng)));
     if (kDepth) ngcol = fma2(splat2(*reinterpret_cast<const float*>(at_col + 8)), p.nd, ngcol);
-    p.R = fma2(w, ngcol, p.R);
+    p.nP = fma2(w, ngcol, p.nP);
     const f32x2 om = fma2(alpha, splat2(-1.0f), splat2(1.0f));
     float o0, o1;
     unpack2(om, o0, o1);
-    const f32x2 ndalpha = fma2(p.T, ngcol, mul2(p.R, pack2(fast_rcp(o0), fast_rcp(o1))));
-    f32x2 sv = mul2(ndalpha, alpha);
+    const f32x2 ndalpha = fma2(p.T, ngcol, mul2(add2(p.R, p.nP), pack2(fast_rcp(o0), fast_rcp(o1))));
+    f32x2 sv = mul2(ndalpha, e);
     if (kClamp) {
         float s0, s1;
         unpack2(sv, s0, s1);
@@ -277,16 +295,17 @@ __device__ __forceinline__ void backward_step(const BackwardSmem<kDepth>& sm, un
 }
 
 /* The same for a tile with a value that is not finite: one pixel at a time,
- * nothing computed for a pixel that skips. */
+ * nothing computed for a pixel that skips (as above). */
 template <bool kDepth>
 __device__ __forceinline__ void backward_step_general(const BackwardSmem<kDepth>& sm, unsigned int off, float pxc,
                                                       float pyc0, GradPair& p, f32x2& s_out, f32x2& w_out) {
     const unsigned int j = off >> 4;
     const float4 g = sm.geo[j], c = sm.con[j], k = sm.col[j];
     const float op = c.y;
-    float T[2], R[2], nr[2], ng[2], nb[2], nd[2], s[2] = {0.0f, 0.0f}, w[2] = {0.0f, 0.0f};
+    float T[2], R[2], nP[2], nr[2], ng[2], nb[2], nd[2], s[2] = {0.0f, 0.0f}, w[2] = {0.0f, 0.0f};
     unpack2(p.T, T[0], T[1]);
     unpack2(p.R, R[0], R[1]);
+    unpack2(p.nP, nP[0], nP[1]);
     unpack2(p.nr, nr[0], nr[1]);
     unpack2(p.ng, ng[0], ng[1]);
     unpack2(p.nb, nb[0], nb[1]);
@@ -299,34 +318,39 @@ __device__ __forceinline__ void backward_step_general(const BackwardSmem<kDepth>
                             __fmul_rn(__fmul_rn(c.x, dy), dy));
         if (x > 0.0f) x = 0.0f;
         if (x < c.z) continue;
-        float alpha = op * fast_exp(x);
-        if (fabsf(alpha - min_alpha()) <= 4e-6f * min_alpha() || fabsf(alpha - (float)0.99) <= 4e-6f)
-            alpha = __fmul_rn(op, lumen_expf_core(x));
+        float e = fast_exp(x), alpha = __fmul_rn(op, e);
+        if (fabsf(alpha - min_alpha()) <= 4e-6f * min_alpha() || fabsf(alpha - (float)0.99) <= 4e-6f) {
+            e = lumen_expf_core(x);
+            alpha = __fmul_rn(op, e);
+        }
         const bool clamped = alpha > (float)0.99;
         if (clamped) alpha = (float)0.99;
         if (alpha < min_alpha()) continue;
-        w[h] = alpha * T[h];
-        float ngcol = c.w * nr[h] + k.x * ng[h] + k.y * nb[h];
-        if (kDepth) ngcol += k.z * nd[h];
-        R[h] += w[h] * ngcol;
+        const float wh = alpha * T[h];
+        float ngcol = __fmaf_rn(k.y, nb[h], __fmaf_rn(c.w, nr[h], __fmul_rn(k.x, ng[h])));
+        if (kDepth) ngcol = __fmaf_rn(k.z, nd[h], ngcol);
+        nP[h] = __fmaf_rn(wh, ngcol, nP[h]);
         const float om = 1.0f - alpha;
-        if (!clamped) s[h] = (T[h] * ngcol + R[h] * fast_rcp(om)) * alpha;
+        const float ndalpha = __fmaf_rn(T[h], ngcol, __fmul_rn(__fadd_rn(R[h], nP[h]), fast_rcp(om)));
+        if (!clamped) s[h] = __fmul_rn(ndalpha, e);
         T[h] *= om;
+        w[h] = wh;
     }
     p.T = pack2(T[0], T[1]);
-    p.R = pack2(R[0], R[1]);
+    p.nP = pack2(nP[0], nP[1]);
     s_out = pack2(s[0], s[1]);
     w_out = pack2(w[0], w[1]);
 }
 
 /* The sums of a batch: lane e takes entry e (list position t0 + e / 4 of
  * group e % 4), reads the group's 16 values of s and w from its row and adds
- * its 10 gradients to the splat's Gaussian with three vector atomics. Rows
- * hold the pixels in the order (row pair, column, row within the pair), so
- * the packed halves are the two rows of a pair. */
+ * its 10 gradients to the warp's sums for the splat, group by group (a group's
+ * entries are different splats, so no two lanes add to one). Rows hold the
+ * pixels in the order (row pair, column, row within the pair), so the packed
+ * halves are the two rows of a pair. */
 template <bool kDepth>
-__device__ __forceinline__ void backward_flush(const BackwardSmem<kDepth>& sm, int warp, int lane, int t0,
-                                               float quad_x, float quad_y, float* __restrict__ grad2d) {
+__device__ __forceinline__ void backward_flush(BackwardSmem<kDepth>& sm, int warp, int lane, int t0, float quad_x,
+                                               float quad_y) {
     const int g = lane & 3, u = lane >> 2;
     const unsigned int off = sm.list[4 * warp + g][t0 + u];
     const float4 geo = *reinterpret_cast<const float4*>(reinterpret_cast<const char*>(sm.geo) + off);
@@ -339,63 +363,76 @@ __device__ __forceinline__ void backward_flush(const BackwardSmem<kDepth>& sm, i
     for (int x = 0; x < 4; ++x) dx[x] = (bx + (float)x) - geo.x;
     constexpr int kCh = BackwardSmem<kDepth>::kChannels;
     const f32x2 zero = splat2(0.0f);
-    f32x2 S = zero, Sx = zero, Sxx = zero, Sy = zero, Sxy = zero, Syy = zero, c[kCh];
+    f32x2 So = zero, Gx = zero, Gy = zero, Sxx = zero, Sxy = zero, Syy = zero, c[kCh];
 #pragma unroll
     for (int ch = 0; ch < kCh; ++ch) c[ch] = zero;
+    const f32x2 op = splat2(con.y), na = splat2(2.0f * geo.z), nb = splat2(-geo.w), nc = splat2(-2.0f * con.x);
 #pragma unroll
     for (int yp = 0; yp < 2; ++yp) {
-        f32x2 r0 = zero, r1 = zero, r2 = zero;
+        const f32x2 dy = add2(pack2(by + (float)(2 * yp), by + (float)(2 * yp + 1)), splat2(geo.y));
+        const f32x2 nbdy = mul2(nb, dy), ncdy = mul2(nc, dy);
+        f32x2 r0 = zero, r1 = zero;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            const ulonglong2 s2 = row[2 * yp + q], w2 = row[kRowsW + 2 * yp + q];
+            ulonglong2 s2 = row[2 * yp + q];
+            const ulonglong2 w2 = row[kRowsW + 2 * yp + q];
+            So = add2(So, add2(s2.x, s2.y));
+            s2 = make_ulonglong2(mul2(s2.x, op), mul2(s2.y, op));   /* dL/dpower */
             const f32x2 d0 = splat2(dx[2 * q]), d1 = splat2(dx[2 * q + 1]);
+            Gx = fma2(fma2(na, d0, nbdy), s2.x, fma2(fma2(na, d1, nbdy), s2.y, Gx));
+            Gy = fma2(fma2(nb, d0, ncdy), s2.x, fma2(fma2(nb, d1, ncdy), s2.y, Gy));
             r0 = add2(r0, add2(s2.x, s2.y));
             const f32x2 e0 = mul2(s2.x, d0), e1 = mul2(s2.y, d1);
             r1 = add2(r1, add2(e0, e1));
-            r2 = fma2(e0, d0, fma2(e1, d1, r2));
+            Sxx = fma2(e0, d0, fma2(e1, d1, Sxx));
 #pragma unroll
             for (int ch = 0; ch < kCh; ++ch) {
                 const ulonglong2 G = gr[4 * ch + 2 * yp + q];
                 c[ch] = fma2(w2.x, G.x, fma2(w2.y, G.y, c[ch]));
             }
         }
-        const f32x2 dy = add2(pack2(by + (float)(2 * yp), by + (float)(2 * yp + 1)), splat2(geo.y));
-        const f32x2 r0y = mul2(r0, dy);
-        S = add2(S, r0);
-        Sx = add2(Sx, r1);
-        Sxx = add2(Sxx, r2);
-        Sy = add2(Sy, r0y);
         Sxy = fma2(r1, dy, Sxy);
-        Syy = fma2(r0y, dy, Syy);
+        Syy = fma2(r0, mul2(dy, dy), Syy);
     }
     auto both = [](f32x2 v) {
         float a, b;
         unpack2(v, a, b);
         return a + b;
     };
-    const float s0 = both(S), sx = both(Sx), sy = both(Sy);
-    const float ga = 0.5f * both(Sxx), gb = both(Sxy), gc = 0.5f * both(Syy);
-    const float cr = both(c[0]), cg = both(c[1]), cb = both(c[2]), cd = kDepth ? both(c[kCh - 1]) : 0.0f;
-    float* dst = grad2d + (size_t)sm.gid[off >> 4] * kGrad2DStride;
-    if (s0 != 0.0f || sx != 0.0f || sy != 0.0f || ga != 0.0f || gb != 0.0f)
-        atomicAdd(reinterpret_cast<float4*>(dst), make_float4(2.0f * geo.z * sx - geo.w * sy,
-                                                              -geo.w * sx - 2.0f * con.x * sy, ga, gb));
-    if (s0 != 0.0f || gc != 0.0f || cr != 0.0f || cg != 0.0f)   /* a padding entry has opacity 0, and zeros only */
-        atomicAdd(reinterpret_cast<float4*>(dst + 4), make_float4(gc, -s0 / con.y, cr, cg));
-    if (cb != 0.0f || cd != 0.0f) atomicAdd(reinterpret_cast<float2*>(dst + 8), make_float2(cb, cd));
+    const unsigned int slot = off >> 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (g == k && slot < (unsigned int)kBwdChunk) {   /* not a padding entry */
+            float4 a = sm.acc0[warp][slot], b = sm.acc1[warp][slot];
+            float2 d = sm.acc2[warp][slot];
+            a.x += both(Gx);
+            a.y += both(Gy);
+            a.z += 0.5f * both(Sxx);
+            a.w += both(Sxy);
+            b.x += 0.5f * both(Syy);
+            b.y -= both(So);
+            b.z += both(c[0]);
+            b.w += both(c[1]);
+            d.x += both(c[2]);
+            if (kDepth) d.y += both(c[kCh - 1]);
+            sm.acc0[warp][slot] = a;
+            sm.acc1[warp][slot] = b;
+            sm.acc2[warp][slot] = d;
+        }
+        __syncwarp();
+    }
 }
 
 /* The lists' n entries of one staged chunk, kBwdSteps at a time. */
 template <int kWay, bool kDepth>   /* kWay 0: general, 1: no clamp, 2: clamp */
 __device__ __forceinline__ void backward_walk(BackwardSmem<kDepth>& sm, int warp, int lane, int n, float pxc,
-                                              float pyc, f32x2 minus_one, float quad_x, float quad_y, GradPair& p,
-                                              float* __restrict__ grad2d) {
+                                              float pyc, f32x2 minus_one, float quad_x, float quad_y, GradPair& p) {
     const int group = lane >> 3;
     const unsigned short* lst = sm.list[4 * warp + group];
     const f32x2 pyc2 = pack2(pyc, pyc + 1.0f);
     f32x2* row = reinterpret_cast<f32x2*>(sm.rows[warp] + row_unit(0, group)) + (lane & 7);
     for (int t0 = 0; t0 < n; t0 += kBwdSteps) {
-#pragma unroll 4
+#pragma unroll 2
         for (int u = 0; u < kBwdSteps; ++u) {
             f32x2 s, w;
             const unsigned int off = lst[t0 + u];
@@ -405,16 +442,14 @@ __device__ __forceinline__ void backward_walk(BackwardSmem<kDepth>& sm, int warp
             row[2 * (row_unit(u, 0) + kRowsW)] = w;
         }
         __syncwarp();
-        backward_flush<kDepth>(sm, warp, lane, t0, quad_x, quad_y, grad2d);
-        __syncwarp();
+        backward_flush<kDepth>(sm, warp, lane, t0, quad_x, quad_y);
     }
 }
 
-/* 6 CTAs per SM (80 registers, 33 KB of shared memory): with the clearing of
- * the sums 0.234 ms at 500 k Gaussians and 1080p, against 0.245 for 5, 0.237
- * for 7 and 0.244 for 8. kDepth: there is an upstream depth gradient. */
+/* 4 CTAs per SM (128 registers, 53 KB of shared memory). kDepth: there is an
+ * upstream depth gradient. */
 template <bool kDepth>
-__global__ void __launch_bounds__(kBwdThreads, 6)
+__global__ void __launch_bounds__(kBwdThreads, 4)
 composite_backward_kernel(const LumenSplatRecord* __restrict__ records, LumenGpuFrame f, Control* ctrl,
                           int width, int height, int tiles_x, LumenRenderOptions opt,
                           const float* __restrict__ out_rgb, const float* __restrict__ out_depth,
@@ -422,7 +457,8 @@ composite_backward_kernel(const LumenSplatRecord* __restrict__ records, LumenGpu
                           const float* __restrict__ grad_rgb, const float* __restrict__ grad_depth,
                           const float* __restrict__ grad_alpha, float* __restrict__ grad2d, float minus_one) {
     chain_begin();
-    __shared__ BackwardSmem<kDepth> s;
+    extern __shared__ float4 bwd_smem[];
+    BackwardSmem<kDepth>& s = *reinterpret_cast<BackwardSmem<kDepth>*>(bwd_smem);
     const int tile = (int)tile_in_line(ctrl, blockIdx.x);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = tile % tiles_x, ty = tile / tiles_x;
@@ -449,7 +485,11 @@ composite_backward_kernel(const LumenSplatRecord* __restrict__ records, LumenGpu
         s.geo[kBwdChunk] = make_float4(0.0f, 0.0f, -1e30f, 0.0f);   /* out of every pixel's reach */
         s.con[kBwdChunk] = make_float4(1e30f, 0.0f, -4.5f, 0.0f);
         s.col[kBwdChunk] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        s.gid[kBwdChunk] = 0u;
+    }
+#pragma unroll
+    for (int w = 0; w < kBwdThreads / 32; ++w) {
+        s.acc0[w][tid] = s.acc1[w][tid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        s.acc2[w][tid] = make_float2(0.0f, 0.0f);
     }
     __syncthreads();
     /* the pixels' upstream gradients and the forward's outputs */
@@ -498,6 +538,7 @@ composite_backward_kernel(const LumenSplatRecord* __restrict__ records, LumenGpu
         }
         p.T = splat2(1.0f);
         p.R = pack2(R[0], R[1]);
+        p.nP = splat2(0.0f);
         p.nr = pack2(nr[0], nr[1]);
         p.ng = pack2(ng[0], ng[1]);
         p.nb = pack2(nb[0], nb[1]);
@@ -519,9 +560,10 @@ composite_backward_kernel(const LumenSplatRecord* __restrict__ records, LumenGpu
 
     const float pxc = (float)px + 0.5f, pyc = (float)py + 0.5f;
     const float quad_x = tile_x0 + (float)(8 * (warp & 1)) + 0.5f, quad_y = tile_y0 + (float)(8 * (warp >> 1)) + 0.5f;
-    unsigned int next = rs + tid < end ? vals[rs + tid] : 0u;
+    unsigned int next = rs + tid < end ? vals[rs + tid] : 0u, gid = 0u;
     for (int cs = rs; cs < end; cs += kBwdChunk) {
-        const bool clamp = stage_chunk<kDepth>(s, records, vals, next, f.visible_ids, n_visible, ctrl, cs, end, tile_x0, tile_y0);
+        const bool clamp = stage_chunk<kDepth>(s, records, vals, next, f.visible_ids, gid, n_visible, ctrl, cs, end,
+                                               tile_x0, tile_y0);
         if (warp_last >= cs) {
             const int limit[4] = {ends[0] - cs, ends[1] - cs, ends[2] - cs, ends[3] - cs};
             const int n = build_backward_lists<kDepth>(s, warp, lane, limit);
@@ -529,11 +571,32 @@ composite_backward_kernel(const LumenSplatRecord* __restrict__ records, LumenGpu
             p.end[1] = 16 * min(last[1] - cs, kBwdChunk);
             if (last[0] < cs) p.end[0] = -1;
             if (last[1] < cs) p.end[1] = -1;
-            if (s.special) backward_walk<0, kDepth>(s, warp, lane, n, pxc, pyc, splat2(minus_one), quad_x, quad_y, p, grad2d);
-            else if (clamp) backward_walk<2, kDepth>(s, warp, lane, n, pxc, pyc, splat2(minus_one), quad_x, quad_y, p, grad2d);
-            else backward_walk<1, kDepth>(s, warp, lane, n, pxc, pyc, splat2(minus_one), quad_x, quad_y, p, grad2d);
+            if (s.special) backward_walk<0, kDepth>(s, warp, lane, n, pxc, pyc, splat2(minus_one), quad_x, quad_y, p);
+            else if (clamp) backward_walk<2, kDepth>(s, warp, lane, n, pxc, pyc, splat2(minus_one), quad_x, quad_y, p);
+            else backward_walk<1, kDepth>(s, warp, lane, n, pxc, pyc, splat2(minus_one), quad_x, quad_y, p);
         }
         __syncthreads();
+        /* thread t: the tile's sums of the chunk's splat t, over the warps */
+        float4 a = s.acc0[0][tid], b = s.acc1[0][tid];
+        float2 d = s.acc2[0][tid];
+#pragma unroll
+        for (int w = 1; w < kBwdThreads / 32; ++w) {
+            const float4 a1 = s.acc0[w][tid], b1 = s.acc1[w][tid];
+            const float2 d1 = s.acc2[w][tid];
+            a = make_float4(a.x + a1.x, a.y + a1.y, a.z + a1.z, a.w + a1.w);
+            b = make_float4(b.x + b1.x, b.y + b1.y, b.z + b1.z, b.w + b1.w);
+            d = make_float2(d.x + d1.x, d.y + d1.y);
+        }
+        float* dst = grad2d + (size_t)gid * kGrad2DStride;
+        if (a.x != 0.0f || a.y != 0.0f || a.z != 0.0f || a.w != 0.0f) atomicAdd(reinterpret_cast<float4*>(dst), a);
+        if (b.x != 0.0f || b.y != 0.0f || b.z != 0.0f || b.w != 0.0f) atomicAdd(reinterpret_cast<float4*>(dst + 4), b);
+        if (d.x != 0.0f || d.y != 0.0f) atomicAdd(reinterpret_cast<float2*>(dst + 8), d);
+        if (cs + kBwdChunk >= end) break;
+#pragma unroll
+        for (int w = 0; w < kBwdThreads / 32; ++w) {
+            s.acc0[w][tid] = s.acc1[w][tid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            s.acc2[w][tid] = make_float2(0.0f, 0.0f);
+        }
     }
 }
 
@@ -901,10 +964,12 @@ namespace lumen {
 /* Six 33 KB CTAs of the compositing adjoint per SM need the largest
  * shared-memory carveout; set per device by configure_once. */
 void configure_backward_kernels() {
-    cudaFuncSetAttribute(composite_backward_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         (int)cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(composite_backward_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         (int)cudaSharedmemCarveoutMaxShared);
+    auto allow = [](auto kernel, size_t smem) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    };
+    allow(composite_backward_kernel<false>, sizeof(BackwardSmem<false>));
+    allow(composite_backward_kernel<true>, sizeof(BackwardSmem<true>));
 }
 
 void configure_once();
@@ -946,8 +1011,9 @@ static LumenStatus backward_impl(const LumenGpuGaussians* g, const LumenViewCame
     const int tiles_x = (cam->width + kTile - 1) / kTile;
     const int tiles = tiles_x * ((cam->height + kTile - 1) / kTile);
     /* without an upstream depth gradient the sweep and its sums leave the depth out */
-    launch_chained(grad_depth && opt->compute_depth ? composite_backward_kernel<true> : composite_backward_kernel<false>,
-                   dim3(tiles), dim3(kBwdThreads), 0, s,
+    const bool depth = grad_depth && opt->compute_depth;
+    launch_chained(depth ? composite_backward_kernel<true> : composite_backward_kernel<false>, dim3(tiles),
+                   dim3(kBwdThreads), depth ? sizeof(BackwardSmem<true>) : sizeof(BackwardSmem<false>), s,
                    (const LumenSplatRecord*)f->records, *f, ctrl, cam->width, cam->height, tiles_x, *opt,
                    (const float*)fwd->rgb, (const float*)fwd->depth, (const float*)fwd->alpha,
                    (const int*)fwd->last_idx, grad_rgb, grad_depth, grad_alpha, out->splat2d, -1.0f);
