@@ -21,8 +21,9 @@
  * 4.5, alpha below 1/255, the 0.99 clamp) are taken exactly as the forward
  * took them: the power is formed with separately rounded operations in the
  * forward's order, and an alpha near a threshold is recomputed with the
- * shared exponential. (A power that rounds below 0 is clamped to 0 as in the
- * forward; its gradient is that of the true power, which is not negative.)
+ * shared exponential. A power that rounds below 0 (or is, of a conic that is
+ * not positive definite) is a constant 0 in the forward: the centre and the
+ * conic get nothing from that pixel.
  *
  * The work is split as in the compositor: two pixels per lane in packed FP32,
  * groups of 8 lanes with a 4x4 block and a splat list of their own. A splat's
@@ -225,11 +226,17 @@ struct GradPair {
     int end[2];
 };
 
+/* A mark in a batch's w (which is never negative itself), read by the marked
+ * form of backward_flush: -w where the forward clamped a power below 0 to 0, so
+ * that the pixel's s belongs to the opacity only. */
+__device__ __forceinline__ float marked(float w) { return __uint_as_float(__float_as_uint(w) | 0x80000000u); }
+__device__ __forceinline__ bool is_marked(float w) { return (__float_as_uint(w) & 0x80000000u) != 0u; }
+
 /* One list entry for the lane's two pixels: s = -dL/dopacity and w = alpha T
  * of each, zero where the pixel did not blend the splat. Every staged value and
- * upstream gradient is finite. */
+ * upstream gradient is finite. Returns whether a w is marked. */
 template <bool kClamp, bool kDepth>
-__device__ __forceinline__ void backward_step(const BackwardSmem<kDepth>& sm, unsigned int off, float pxc, f32x2 pyc,
+__device__ __forceinline__ bool backward_step(const BackwardSmem<kDepth>& sm, unsigned int off, float pxc, f32x2 pyc,
                                               f32x2 minus_one, GradPair& p, f32x2& s_out, f32x2& w_out) {
     /* 10 words per lane (12 with the depth): the kernel is bound by what
      * shared memory delivers */
@@ -244,10 +251,9 @@ __device__ __forceinline__ void backward_step(const BackwardSmem<kDepth>& sm, un
     const f32x2 q = fma2(mul2(mul2(splat2(c.x), dy), dy), minus_one,
                          fma2(mul2(splat2(__fmul_rn(g.w, dx)), dy), minus_one,
                               splat2(__fmul_rn(__fmul_rn(g.z, dx), dx))));
-    float x0, x1;
-    unpack2(q, x0, x1);
-    x0 = fminf(x0, 0.0f);
-    x1 = fminf(x1, 0.0f);
+    float q0, q1;
+    unpack2(q, q0, q1);
+    const float x0 = fminf(q0, 0.0f), x1 = fminf(q1, 0.0f);
     const int at = (int)off;
     bool b0 = !(x0 < skip) && at <= p.end[0];
     bool b1 = !(x1 < skip) && at <= p.end[1];
@@ -292,17 +298,24 @@ __device__ __forceinline__ void backward_step(const BackwardSmem<kDepth>& sm, un
     p.T = mul2(p.T, om);
     s_out = sv;
     w_out = w;
+    const bool below0 = q0 > 0.0f && b0, below1 = q1 > 0.0f && b1;
+    if (!(below0 || below1)) return false;
+    float w0, w1;
+    unpack2(w, w0, w1);
+    w_out = pack2(below0 ? marked(w0) : w0, below1 ? marked(w1) : w1);
+    return true;
 }
 
 /* The same for a tile with a value that is not finite: one pixel at a time,
  * nothing computed for a pixel that skips (as above). */
 template <bool kDepth>
-__device__ __forceinline__ void backward_step_general(const BackwardSmem<kDepth>& sm, unsigned int off, float pxc,
+__device__ __forceinline__ bool backward_step_general(const BackwardSmem<kDepth>& sm, unsigned int off, float pxc,
                                                       float pyc0, GradPair& p, f32x2& s_out, f32x2& w_out) {
     const unsigned int j = off >> 4;
     const float4 g = sm.geo[j], c = sm.con[j], k = sm.col[j];
     const float op = c.y;
     float T[2], R[2], nP[2], nr[2], ng[2], nb[2], nd[2], s[2] = {0.0f, 0.0f}, w[2] = {0.0f, 0.0f};
+    bool any_below = false;
     unpack2(p.T, T[0], T[1]);
     unpack2(p.R, R[0], R[1]);
     unpack2(p.nP, nP[0], nP[1]);
@@ -316,7 +329,8 @@ __device__ __forceinline__ void backward_step_general(const BackwardSmem<kDepth>
         const float dx = __fsub_rn(pxc, g.x), dy = __fadd_rn(pyc0 + (float)h, g.y);
         float x = __fsub_rn(__fsub_rn(__fmul_rn(__fmul_rn(g.z, dx), dx), __fmul_rn(__fmul_rn(g.w, dx), dy)),
                             __fmul_rn(__fmul_rn(c.x, dy), dy));
-        if (x > 0.0f) x = 0.0f;
+        const bool below = x > 0.0f;
+        if (below) x = 0.0f;
         if (x < c.z) continue;
         float e = fast_exp(x), alpha = __fmul_rn(op, e);
         if (fabsf(alpha - min_alpha()) <= 4e-6f * min_alpha() || fabsf(alpha - (float)0.99) <= 4e-6f) {
@@ -334,12 +348,14 @@ __device__ __forceinline__ void backward_step_general(const BackwardSmem<kDepth>
         const float ndalpha = __fmaf_rn(T[h], ngcol, __fmul_rn(__fadd_rn(R[h], nP[h]), fast_rcp(om)));
         if (!clamped) s[h] = __fmul_rn(ndalpha, e);
         T[h] *= om;
-        w[h] = wh;
+        w[h] = below ? marked(wh) : wh;
+        any_below |= below;
     }
     p.T = pack2(T[0], T[1]);
     p.nP = pack2(nP[0], nP[1]);
     s_out = pack2(s[0], s[1]);
     w_out = pack2(w[0], w[1]);
+    return any_below;
 }
 
 /* The sums of a batch: lane e takes entry e (list position t0 + e / 4 of
@@ -347,8 +363,8 @@ __device__ __forceinline__ void backward_step_general(const BackwardSmem<kDepth>
  * its 10 gradients to the warp's sums for the splat, group by group (a group's
  * entries are different splats, so no two lanes add to one). Rows hold the
  * pixels in the order (row pair, column, row within the pair), so the packed
- * halves are the two rows of a pair. */
-template <bool kDepth>
+ * halves are the two rows of a pair. kMarked: some w of the batch is marked. */
+template <bool kDepth, bool kMarked>
 __device__ __forceinline__ void backward_flush(BackwardSmem<kDepth>& sm, int warp, int lane, int t0, float quad_x,
                                                float quad_y) {
     const int g = lane & 3, u = lane >> 2;
@@ -374,9 +390,23 @@ __device__ __forceinline__ void backward_flush(BackwardSmem<kDepth>& sm, int war
         f32x2 r0 = zero, r1 = zero;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            ulonglong2 s2 = row[2 * yp + q];
-            const ulonglong2 w2 = row[kRowsW + 2 * yp + q];
+            ulonglong2 s2 = row[2 * yp + q], w2 = row[kRowsW + 2 * yp + q];
             So = add2(So, add2(s2.x, s2.y));
+            if (kMarked) {
+                float s[4], w[4];
+                unpack2(s2.x, s[0], s[1]);
+                unpack2(s2.y, s[2], s[3]);
+                unpack2(w2.x, w[0], w[1]);
+                unpack2(w2.y, w[2], w[3]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (!is_marked(w[i])) continue;
+                    w[i] = -w[i];
+                    s[i] = 0.0f;
+                }
+                s2 = make_ulonglong2(pack2(s[0], s[1]), pack2(s[2], s[3]));
+                w2 = make_ulonglong2(pack2(w[0], w[1]), pack2(w[2], w[3]));
+            }
             s2 = make_ulonglong2(mul2(s2.x, op), mul2(s2.y, op));   /* dL/dpower */
             const f32x2 d0 = splat2(dx[2 * q]), d1 = splat2(dx[2 * q + 1]);
             Gx = fma2(fma2(na, d0, nbdy), s2.x, fma2(fma2(na, d1, nbdy), s2.y, Gx));
@@ -432,17 +462,19 @@ __device__ __forceinline__ void backward_walk(BackwardSmem<kDepth>& sm, int warp
     const f32x2 pyc2 = pack2(pyc, pyc + 1.0f);
     f32x2* row = reinterpret_cast<f32x2*>(sm.rows[warp] + row_unit(0, group)) + (lane & 7);
     for (int t0 = 0; t0 < n; t0 += kBwdSteps) {
+        bool any_marked = false;
 #pragma unroll 2
         for (int u = 0; u < kBwdSteps; ++u) {
             f32x2 s, w;
             const unsigned int off = lst[t0 + u];
-            if (kWay == 0) backward_step_general<kDepth>(sm, off, pxc, pyc, p, s, w);
-            else backward_step<kWay == 2, kDepth>(sm, off, pxc, pyc2, minus_one, p, s, w);
+            if (kWay == 0) any_marked |= backward_step_general<kDepth>(sm, off, pxc, pyc, p, s, w);
+            else any_marked |= backward_step<kWay == 2, kDepth>(sm, off, pxc, pyc2, minus_one, p, s, w);
             row[2 * row_unit(u, 0)] = s;
             row[2 * (row_unit(u, 0) + kRowsW)] = w;
         }
         __syncwarp();
-        backward_flush<kDepth>(sm, warp, lane, t0, quad_x, quad_y);
+        if (__any_sync(0xffffffffu, any_marked)) backward_flush<kDepth, true>(sm, warp, lane, t0, quad_x, quad_y);
+        else backward_flush<kDepth, false>(sm, warp, lane, t0, quad_x, quad_y);
     }
 }
 

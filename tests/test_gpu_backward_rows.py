@@ -92,3 +92,22 @@ def test_rows_of_large_and_needle_like_splats():
     scale = torch.stack([(size * v).sum(1) for v in abs_geo] + [(w * G[:, k].abs()).sum(1) for k in range(4)], 1)
     err = (got[order] - want).abs() / scale.clamp_min(1e-12)
     assert float(err.max()) <= 6e-5, err.amax(0).tolist()
+
+
+def test_a_power_clamped_at_zero_moves_neither_centre_nor_conic():
+    """Needles without a low pass, whose conics come out indefinite: where the
+    power is below 0 the forward takes the constant 0, so a splat that is
+    blended at such pixels alone gets a gradient for its opacity and none for
+    its centre and conic."""
+    n, cam, opt = 40, _cam(37, 26), RenderOptions(term_threshold=0.0, lowpass=0.0)
+    scene = _scene(n, 21, (0.05, 0.5))
+    scene[1][:, 0] = 2.0
+    scene[1][:, 1:] = 1e-5
+    r, got = _splat2d(scene, cam, opt, *_grads(cam, 21, False, False))
+    got = got[r.frame.visible_ids[:r.n_visible].long()]
+    py, px = torch.meshgrid(torch.arange(cam.height, device="cuda") + 0.5, torch.arange(cam.width, device="cuda") + 0.5,
+                            indexing="ij")
+    power = _forward_power(r.records, px, py)
+    only_clamped = (power < 0.0).any(1) & ~((power >= 0.0) & (power <= 4.5)).any(1)
+    assert int(only_clamped.sum()) >= 5
+    assert bool((got[only_clamped][:, :5] == 0.0).all()) and bool((got[only_clamped][:, 5] != 0.0).all())
