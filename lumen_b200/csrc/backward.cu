@@ -226,9 +226,11 @@ struct GradPair {
     int end[2];
 };
 
-/* A mark in a batch's w (which is never negative itself), read by the marked
+/* Marks in a batch's w (which is never negative itself), read by the marked
  * form of backward_flush: -w where the forward clamped a power below 0 to 0, so
- * that the pixel's s belongs to the opacity only. */
+ * that the pixel's s belongs to the opacity only; -0 where the pixel did not
+ * blend the splat, so that an upstream gradient that is not finite stays out
+ * of its colour. */
 __device__ __forceinline__ float marked(float w) { return __uint_as_float(__float_as_uint(w) | 0x80000000u); }
 __device__ __forceinline__ bool is_marked(float w) { return (__float_as_uint(w) & 0x80000000u) != 0u; }
 
@@ -307,15 +309,14 @@ __device__ __forceinline__ bool backward_step(const BackwardSmem<kDepth>& sm, un
 }
 
 /* The same for a tile with a value that is not finite: one pixel at a time,
- * nothing computed for a pixel that skips (as above). */
+ * nothing computed for a pixel that skips (its w is marked). */
 template <bool kDepth>
-__device__ __forceinline__ bool backward_step_general(const BackwardSmem<kDepth>& sm, unsigned int off, float pxc,
+__device__ __forceinline__ void backward_step_general(const BackwardSmem<kDepth>& sm, unsigned int off, float pxc,
                                                       float pyc0, GradPair& p, f32x2& s_out, f32x2& w_out) {
     const unsigned int j = off >> 4;
     const float4 g = sm.geo[j], c = sm.con[j], k = sm.col[j];
     const float op = c.y;
-    float T[2], R[2], nP[2], nr[2], ng[2], nb[2], nd[2], s[2] = {0.0f, 0.0f}, w[2] = {0.0f, 0.0f};
-    bool any_below = false;
+    float T[2], R[2], nP[2], nr[2], ng[2], nb[2], nd[2], s[2] = {0.0f, 0.0f}, w[2] = {-0.0f, -0.0f};
     unpack2(p.T, T[0], T[1]);
     unpack2(p.R, R[0], R[1]);
     unpack2(p.nP, nP[0], nP[1]);
@@ -349,13 +350,11 @@ __device__ __forceinline__ bool backward_step_general(const BackwardSmem<kDepth>
         if (!clamped) s[h] = __fmul_rn(ndalpha, e);
         T[h] *= om;
         w[h] = below ? marked(wh) : wh;
-        any_below |= below;
     }
     p.T = pack2(T[0], T[1]);
     p.nP = pack2(nP[0], nP[1]);
     s_out = pack2(s[0], s[1]);
     w_out = pack2(w[0], w[1]);
-    return any_below;
 }
 
 /* The sums of a batch: lane e takes entry e (list position t0 + e / 4 of
@@ -392,6 +391,7 @@ __device__ __forceinline__ void backward_flush(BackwardSmem<kDepth>& sm, int war
         for (int q = 0; q < 2; ++q) {
             ulonglong2 s2 = row[2 * yp + q], w2 = row[kRowsW + 2 * yp + q];
             So = add2(So, add2(s2.x, s2.y));
+            bool skip[4] = {false, false, false, false};
             if (kMarked) {
                 float s[4], w[4];
                 unpack2(s2.x, s[0], s[1]);
@@ -402,6 +402,7 @@ __device__ __forceinline__ void backward_flush(BackwardSmem<kDepth>& sm, int war
                 for (int i = 0; i < 4; ++i) {
                     if (!is_marked(w[i])) continue;
                     w[i] = -w[i];
+                    skip[i] = w[i] == 0.0f;
                     s[i] = 0.0f;
                 }
                 s2 = make_ulonglong2(pack2(s[0], s[1]), pack2(s[2], s[3]));
@@ -417,7 +418,15 @@ __device__ __forceinline__ void backward_flush(BackwardSmem<kDepth>& sm, int war
             Sxx = fma2(e0, d0, fma2(e1, d1, Sxx));
 #pragma unroll
             for (int ch = 0; ch < kCh; ++ch) {
-                const ulonglong2 G = gr[4 * ch + 2 * yp + q];
+                ulonglong2 G = gr[4 * ch + 2 * yp + q];
+                if (kMarked) {
+                    float G0[4];
+                    unpack2(G.x, G0[0], G0[1]);
+                    unpack2(G.y, G0[2], G0[3]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) G0[i] = skip[i] ? 0.0f : G0[i];
+                    G = make_ulonglong2(pack2(G0[0], G0[1]), pack2(G0[2], G0[3]));
+                }
                 c[ch] = fma2(w2.x, G.x, fma2(w2.y, G.y, c[ch]));
             }
         }
@@ -462,12 +471,12 @@ __device__ __forceinline__ void backward_walk(BackwardSmem<kDepth>& sm, int warp
     const f32x2 pyc2 = pack2(pyc, pyc + 1.0f);
     f32x2* row = reinterpret_cast<f32x2*>(sm.rows[warp] + row_unit(0, group)) + (lane & 7);
     for (int t0 = 0; t0 < n; t0 += kBwdSteps) {
-        bool any_marked = false;
+        bool any_marked = kWay == 0;
 #pragma unroll 2
         for (int u = 0; u < kBwdSteps; ++u) {
             f32x2 s, w;
             const unsigned int off = lst[t0 + u];
-            if (kWay == 0) any_marked |= backward_step_general<kDepth>(sm, off, pxc, pyc, p, s, w);
+            if (kWay == 0) backward_step_general<kDepth>(sm, off, pxc, pyc, p, s, w);
             else any_marked |= backward_step<kWay == 2, kDepth>(sm, off, pxc, pyc2, minus_one, p, s, w);
             row[2 * row_unit(u, 0)] = s;
             row[2 * (row_unit(u, 0) + kRowsW)] = w;

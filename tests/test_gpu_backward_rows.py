@@ -111,3 +111,21 @@ def test_a_power_clamped_at_zero_moves_neither_centre_nor_conic():
     only_clamped = (power < 0.0).any(1) & ~((power >= 0.0) & (power <= 4.5)).any(1)
     assert int(only_clamped.sum()) >= 5
     assert bool((got[only_clamped][:, :5] == 0.0).all()) and bool((got[only_clamped][:, 5] != 0.0).all())
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_an_upstream_value_that_is_not_finite_stays_with_the_splats_its_pixel_blends(value):
+    """A splat that reaches the upper left 4x4 block but not its first pixel
+    (2.8 pixels away; a 3-sigma radius of 1.65): that pixel's gradient is none
+    of its business."""
+    cam, opt = _cam(16, 16), RenderOptions(term_threshold=0.0)
+    scene = [t.cuda().contiguous() for t in (
+        torch.tensor([[(2.5 - 8) / 60 * 4, (2.5 - 8) / 60 * 4, 4.0]]), torch.full((1, 3), 1e-4),
+        torch.tensor([[1.0, 0.0, 0.0, 0.0]]), torch.tensor([0.5]), torch.full((1, 48), 0.1))]
+    up = _grads(cam, 4, True, False)
+    r, clean = _splat2d(scene, cam, opt, *up)
+    assert int(r.n_contrib[0, 0]) == 0 and int(r.n_contrib[2, 2]) == 1
+    up[0][0, 0, 1] = value
+    up[1][0, 0] = value
+    got = _splat2d(scene, cam, opt, *up)[1]
+    assert float(((got - clean).abs() / clean.abs().amax().clamp_min(1e-12)).max()) <= 2e-5
