@@ -75,7 +75,9 @@ LumenStatus lumen_gpu_bvh_build(const LumenGpuGaussians* gaussians, LumenGpuBvh*
                                 size_t scratch_bytes, void* stream);
 
 /* The closest Gaussian along each of n_rays rays (device arrays). The
- * hierarchy must have been built over these gaussians. Does not wait. */
+ * hierarchy must have been built over these gaussians; where they or its nodes
+ * have changed since, the hits are those of the reference's traversal of the
+ * nodes as they are, found more slowly. Does not wait. */
 LumenStatus lumen_gpu_raycast(const LumenGpuBvh* bvh, const LumenGpuGaussians* gaussians, const LumenRay* rays,
                               int64_t n_rays, float max_dist, LumenRayHit* hits, void* stream);
 

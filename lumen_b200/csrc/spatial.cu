@@ -30,8 +30,9 @@
  * Casts: eight lanes per ray walk the hierarchy three levels at a time, the
  * nearest nodes first (cast_ray); the hits are those of the reference's
  * depth-first order bit for bit, ties included. Rays for which that order
- * could show, and hierarchies with NaN boxes, are cast in that order by one
- * thread (cast_ray_in_order).
+ * could show, and hierarchies that are not as the build leaves them for the
+ * Gaussians as they are now (check_nodes_kernel), are cast in that order by
+ * one thread (cast_ray_in_order).
  *
  * Memory: the build reads 24 B per Gaussian twice and writes 32 B per node
  * (n + ceil(n / 2) + ceil(n / 4) + ... nodes, about 64 MB for 1M Gaussians) plus the sort's traffic.
@@ -250,6 +251,22 @@ __device__ __forceinline__ void store_node(LumenBvhNode* node, const Box& b, int
     __stcg(p + 1, make_float4(b.mx[0], b.mx[1], b.mx[2], __int_as_float(right)));
 }
 
+/* A leaf's box: position +- 3 x the largest scale (bvh.mojo:78-93). */
+__device__ __forceinline__ Box leaf_box(const float* __restrict__ means, const float* __restrict__ scales, long long g) {
+    float r = scales[g * 3 + 0];
+    if (scales[g * 3 + 1] > r) r = scales[g * 3 + 1];
+    if (scales[g * 3 + 2] > r) r = scales[g * 3 + 2];
+    const float r3 = r * 3.0f;
+    Box leaf;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float pc = means[g * 3 + c];
+        leaf.mn[c] = pc - r3;
+        leaf.mx[c] = pc + r3;
+    }
+    return leaf;
+}
+
 /* AABB3f.expand_point, aabb.mojo:47-54 */
 __device__ __forceinline__ void expand_point(Box& b, const float p[3]) {
 #pragma unroll
@@ -286,18 +303,7 @@ bvh_levels_kernel(const float* __restrict__ means, const float* __restrict__ sca
         for (int k = tid; k < m0; k += kRefitThreads) {
             const long long i = first + k;
             const long long g = perm[i];
-            /* leaf: position +- 3 x the largest scale (bvh.mojo:78-93) */
-            float r = scales[g * 3 + 0];
-            if (scales[g * 3 + 1] > r) r = scales[g * 3 + 1];
-            if (scales[g * 3 + 2] > r) r = scales[g * 3 + 2];
-            const float r3 = r * 3.0f;
-            Box leaf;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float pc = means[g * 3 + c];
-                leaf.mn[c] = pc - r3;
-                leaf.mx[c] = pc + r3;
-            }
+            const Box leaf = leaf_box(means, scales, g);
             store_node(nodes + i, leaf, -1, -1);
             splat_index[i] = (int)g;
             cur[k] = leaf;
@@ -508,8 +514,9 @@ struct CastEntry {
  * to 6.1 ms in the reference's order with one thread per ray, 0.56 to 1.43
  * with the nearer child first, 0.37 to 0.83 with eight lanes per ray.
  *
- * The result is the reference's bit for bit. Boxes of finite numbers contain
- * their children's, and float subtraction and multiplication are monotone,
+ * The result is the reference's bit for bit, where the nodes are as the build
+ * leaves them for the Gaussians as they are now (check_nodes_kernel). Their
+ * boxes contain their children's, and float subtraction and multiplication are monotone,
  * so a leaf whose box passes has ancestors that pass. A leaf with a hit at
  * t_proj normally has t_enter <= t_proj (its box contains the hit point), and
  * then the reference keeps it exactly when t_proj is below the best so far:
@@ -520,8 +527,7 @@ struct CastEntry {
  * depends on its order. Such a leaf is never pruned here before it is seen,
  * as t_near is below t_proj, and when one with t_proj up to the best so far
  * is seen, the whole ray is cast in the reference's order. So is a ray whose
- * origin or reciprocals are not ordinary numbers; a hierarchy with NaN boxes
- * (which do not contain their children) never comes here (nan_boxes_kernel).
+ * origin or reciprocals are not ordinary numbers.
  *
  * Every lane of the group returns its hit (`active` false: none). */
 __device__ __forceinline__ LumenRayHit cast_ray(const CastArgs& A, const CastLevels& lv, const float origin[3],
@@ -629,11 +635,13 @@ __device__ __forceinline__ LumenRayHit cast_ray(const CastArgs& A, const CastLev
     return best;
 }
 
-/* Whether some leaf's box holds a NaN (a NaN position or scale, or an
- * infinite one of both): a NaN box does not contain its children, so rays are
- * then cast in the reference's order. Nothing but the hits is at hand to
- * carry that to the cast, so a block that finds one marks every hit record;
- * a record that holds the mark by chance only costs its ray the slower way. */
+/* What cast_ray rests on is checked before every cast: the Gaussians may have
+ * moved since the build, and the nodes are the caller's memory. Rays through
+ * nodes that do not pass are cast in the reference's order, which follows the
+ * links and the boxes whatever they hold. Nothing but the hits is at hand to
+ * carry the finding to the cast, so a block that finds such a node marks every
+ * hit record, unless a block before it has come to the last; a record that holds
+ * the mark by chance only costs its ray the slower way. */
 __device__ __forceinline__ uint4 in_order_mark() {
     return make_uint4(0x7A3C91E5u, 0x1D80F24Bu, 0xC5E76A03u, 0x3B9F58D2u);
 }
@@ -644,16 +652,43 @@ __device__ __forceinline__ bool marked_in_order(const LumenRayHit* hit) {
     return w[0] == m.x && w[1] == m.y && w[2] == m.z && w[3] == m.w;
 }
 
+/* Whether node i is as the build leaves it: a leaf holds the box of its
+ * Gaussian; a parent the links to its two children (or one) of the level
+ * below, and a box that contains theirs. A NaN passes no comparison. */
+__device__ __forceinline__ bool node_as_built(const CastArgs& A, const CastLevels& lv, long long i) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(A.nodes + i));
+    const float4 b = __ldg(reinterpret_cast<const float4*>(A.nodes + i) + 1);
+    const int left = __float_as_int(a.w), right = __float_as_int(b.w);
+    if (i < A.n_leaves) {
+        const int g = A.splat_index[i];
+        if (g < 0 || (long long)g >= A.n_gauss) return false;
+        const Box box = leaf_box(A.means, A.scales, g);
+        return left == -1 && right == -1 && a.x == box.mn[0] && a.y == box.mn[1] && a.z == box.mn[2] &&
+               b.x == box.mx[0] && b.y == box.mx[1] && b.z == box.mx[2];
+    }
+    int level = 1;
+    while (level + 1 < lv.n_levels && i >= (long long)lv.start[level + 1]) ++level;
+    const long long first = 2 * (i - (long long)lv.start[level]);
+    const long long child = (long long)lv.start[level - 1] + first;
+    const bool two = first + 1 < (long long)lv.count[level - 1];
+    if ((long long)left != child || right != (two ? left + 1 : -1)) return false;
+    for (int k = 0; k < (two ? 2 : 1); ++k) {
+        const float4 c = __ldg(reinterpret_cast<const float4*>(A.nodes + child + k));
+        const float4 d = __ldg(reinterpret_cast<const float4*>(A.nodes + child + k) + 1);
+        if (!(a.x <= c.x && a.y <= c.y && a.z <= c.z && b.x >= d.x && b.y >= d.y && b.z >= d.z)) return false;
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(256)
-nan_boxes_kernel(const LumenBvhNode* __restrict__ nodes, long long n_leaves, LumenRayHit* __restrict__ hits,
-                 long long n_rays) {
+check_nodes_kernel(CastArgs A, BvhLevels levels, LumenRayHit* __restrict__ hits, long long n_rays) {
+    __shared__ CastLevels lv;
+    copy_levels(lv, levels);
     const long long stride = (long long)gridDim.x * blockDim.x;
     int found = 0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < 2 * n_leaves; i += stride) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(nodes) + i);
-        found |= !(v.x == v.x && v.y == v.y && v.z == v.z);
-    }
-    if (!__syncthreads_or(found)) return;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < A.node_count; i += stride)
+        found |= !node_as_built(A, lv, i);
+    if (!__syncthreads_or(found) || marked_in_order(hits + n_rays - 1)) return;
     for (long long i = threadIdx.x; i < n_rays; i += blockDim.x) {
         unsigned int* w = reinterpret_cast<unsigned int*>(hits + i);
         const uint4 m = in_order_mark();
@@ -736,12 +771,12 @@ int ray_grid(long long n) {
     return (int)(g < 1 ? 1 : g);
 }
 
-void launch_nan_boxes(const LumenGpuBvh* bvh, long long n_rays, LumenRayHit* hits, cudaStream_t s) {
-    if (bvh->leaf_count <= 0) return;
-    long long g = (2 * bvh->leaf_count + 2047) / 2048;
+void launch_check_nodes(const CastArgs& A, const BvhLevels& lv, long long n_rays, LumenRayHit* hits, cudaStream_t s) {
+    if (A.node_count <= 0) return;
+    long long g = (A.node_count + 255) / 256;
     const long long cap = (long long)device_sm_count() * 8;
     if (g > cap) g = cap;
-    nan_boxes_kernel<<<(unsigned int)g, 256, 0, s>>>(bvh->nodes, bvh->leaf_count, hits, n_rays);
+    check_nodes_kernel<<<(unsigned int)g, 256, 0, s>>>(A, lv, hits, n_rays);
 }
 
 bool bvh_ok(const LumenGpuBvh* b, const LumenGpuGaussians* g) {
@@ -823,8 +858,9 @@ LumenStatus lumen_gpu_raycast(const LumenGpuBvh* bvh, const LumenGpuGaussians* g
     if (!rays || !hits) return LUMEN_ERROR_INVALID_ARGUMENT;
     const CastArgs A{bvh->nodes, bvh->splat_index, bvh->node_count, bvh->root_index, g->count, bvh->leaf_count,
                      g->means, g->scales, max_dist};
-    launch_nan_boxes(bvh, n_rays, hits, (cudaStream_t)stream);
-    raycast_kernel<<<ray_grid(n_rays), kCastThreads, 0, (cudaStream_t)stream>>>(A, make_levels(bvh->leaf_count), rays, n_rays, hits);
+    const BvhLevels lv = make_levels(bvh->leaf_count);
+    launch_check_nodes(A, lv, n_rays, hits, (cudaStream_t)stream);
+    raycast_kernel<<<ray_grid(n_rays), kCastThreads, 0, (cudaStream_t)stream>>>(A, lv, rays, n_rays, hits);
     return map_cuda(cudaGetLastError());
 }
 
@@ -836,8 +872,9 @@ LumenStatus lumen_gpu_pick_pixels(const LumenGpuBvh* bvh, const LumenGpuGaussian
     if (!pixels_xy || !hits) return LUMEN_ERROR_INVALID_ARGUMENT;
     const CastArgs A{bvh->nodes, bvh->splat_index, bvh->node_count, bvh->root_index, g->count, bvh->leaf_count,
                      g->means, g->scales, max_dist};
-    launch_nan_boxes(bvh, n, hits, (cudaStream_t)stream);
-    pick_kernel<<<ray_grid(n), kCastThreads, 0, (cudaStream_t)stream>>>(A, make_levels(bvh->leaf_count), *cam, pixels_xy, n, rays, hits);
+    const BvhLevels lv = make_levels(bvh->leaf_count);
+    launch_check_nodes(A, lv, n, hits, (cudaStream_t)stream);
+    pick_kernel<<<ray_grid(n), kCastThreads, 0, (cudaStream_t)stream>>>(A, lv, *cam, pixels_xy, n, rays, hits);
     return map_cuda(cudaGetLastError());
 }
 
