@@ -63,3 +63,20 @@ def test_nodes_of_the_callers_own(what):
         raw.view(np.float32)[0:n:20, 0:3] += 0.05
     bvh.nodes.copy_(torch.from_numpy(raw).cuda())
     _same(bvh, raw.reshape(-1).view(nodes.dtype), idx, root, means, scales, rays)
+
+
+@pytest.mark.parametrize("n", [1, 256, 257, 4096, 4097, 8193])
+def test_many_rays_at_once_hit_what_few_do(n):
+    """A thread per ray and eight lanes per ray, by the numbers of Gaussians and of rays."""
+    from lumen_b200 import spatial as S
+    from lumen_b200.types import ViewCamera
+    means, scales, rays = _random(n, 33_000, n)
+    means[n // 2] = means[0]
+    bvh, rays = S.LBVH(_t(means), _t(scales)), _t(rays)
+    few = torch.cat([bvh.raycast(rays[k:k + 3000], max_dist=40.0) for k in range(0, rays.shape[0], 3000)])
+    assert torch.equal(bvh.raycast(rays, max_dist=40.0), few)
+    cam = ViewCamera.from_fov(200, 200, 60.0, position=(0.0, 0.0, -9.0))
+    px = torch.rand((140_000, 2), device="cuda", generator=torch.Generator("cuda").manual_seed(n)) * 200.0
+    made, made_few = torch.empty((140_000, 6), device="cuda"), torch.empty((140_000, 6), device="cuda")
+    few = torch.cat([bvh.pick(cam, px[k:k + 20_000], rays_out=made_few[k:k + 20_000]) for k in range(0, 140_000, 20_000)])
+    assert torch.equal(bvh.pick(cam, px, rays_out=made), few) and torch.equal(made, made_few)
