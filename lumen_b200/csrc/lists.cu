@@ -242,14 +242,15 @@ list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ct
                               (int)(c.tile_begin + (long long)c.y * c.tiles_x + c.x), c.tiles_x);
             }
         }
-        if (tid < kCellTiles) {
-            const long long t = c.tile(tid);
+        if (warp == 0) {
+            const long long t = lane < kCellTiles ? c.tile(lane) : -1;
+            const unsigned int tiles = __ballot_sync(0xffffffffu, t >= 0);
             if (t >= 0) {
                 f.ranges[2 * t + 1] = (int)base;
                 if (base) atomicAdd(&ctrl->group_total[t / group], base);
                 if (order) {
                     const int cls = length_class(base);
-                    const unsigned int same = __match_any_sync(__activemask(), cls);
+                    const unsigned int same = __match_any_sync(tiles, cls);
                     if (lane == __ffs(same) - 1) atomicAdd(&ctrl->class_total[cls], (unsigned int)__popc(same));
                 }
             }
