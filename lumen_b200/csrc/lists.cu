@@ -85,11 +85,6 @@ __device__ __forceinline__ int first_of_cell(const unsigned int* __restrict__ ke
     return lo;
 }
 
-/* The tile mask of a sorted pair of the cell whose first tile is (x, y). */
-__device__ __forceinline__ unsigned int pair_mask(bool packed, unsigned int key, unsigned int v,
-                                                  const uint64_t* __restrict__ rects, int x, int y) {
-    return packed ? key >> 16 : cell_mask(rects[v], x, y);
-}
 
 /* Tiles per scan group: at most kTileGroups groups. */
 __device__ __forceinline__ long long tile_group_size(long long n_tiles) {
@@ -103,14 +98,25 @@ struct SortedPairs {
     const unsigned int* vals;
     int n;
     bool packed;
+    unsigned int cut_splat, cut_tiles;   /* of the control block */
 };
+
+/* The tile mask of a sorted pair of the cell whose first tile is (x, y). */
+__device__ __forceinline__ unsigned int pair_mask(const SortedPairs& in, unsigned int key, unsigned int v,
+                                                  const uint64_t* __restrict__ rects, int x, int y) {
+    if (in.packed) return key >> 16;
+    const unsigned long long rect = rects[v];
+    const unsigned int mask = cell_mask(rect, x, y);
+    return v + 1u == in.cut_splat ? cut_mask(rect, x, y, mask, in.cut_tiles) : mask;
+}
 
 __device__ __forceinline__ SortedPairs sorted_pairs(const LumenGpuFrame& f, const Control* ctrl,
                                                     const ViewTable* vt) {
     const unsigned int b = ctrl->cell_sort.sorted_buffer;
     const long long n = (long long)ctrl->cell_sort.n;
     return {b ? f.keys[1] : f.keys[0], b ? f.vals[1] : f.vals[0],
-            (int)(n < f.instance_capacity ? n : f.instance_capacity), vt->hdr.total_cells <= kPackedCells};
+            (int)(n < f.instance_capacity ? n : f.instance_capacity), vt->hdr.total_cells <= kPackedCells,
+            ctrl->cut_splat, ctrl->cut_tiles};
 }
 
 /* A segment: up to 256 consecutive pairs of one cell, as the count kernel
@@ -203,7 +209,7 @@ list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ct
 #pragma unroll
             for (int u = 0; u < kReads; ++u) {
                 const int i = first + seg * kSegment + 32 * u + lane;
-                m[u] = i < end ? pair_mask(in.packed, in.keys[i], in.packed ? 0u : in.vals[i], f.rects, c.x, c.y) : 0u;
+                m[u] = i < end ? pair_mask(in, in.keys[i], in.packed ? 0u : in.vals[i], f.rects, c.x, c.y) : 0u;
             }
         };
         read(warp);
@@ -404,7 +410,7 @@ list_write_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ct
             for (int g = 0; g < kSegment / 32; ++g) {
                 const int i = i0 + g * 32 + lane;
                 v[g] = i < end ? in.vals[i] : 0u;
-                m[g] = i < end ? pair_mask(in.packed, in.keys[i], v[g], f.rects, cx, cy) : 0u;
+                m[g] = i < end ? pair_mask(in, in.keys[i], v[g], f.rects, cx, cy) : 0u;
             }
             unsigned int written = 0u;   /* lane k: the segment's instances of tile k */
             bool fits = true;

@@ -272,18 +272,6 @@ __device__ __noinline__ void emit_cut(EmitSmem& s, unsigned int room, int n) {
     }
 }
 
-/* The tiles of the cell whose first tile is (x, y) among the first `left`
- * of the rectangle's, row-major. */
-__device__ __noinline__ unsigned int emit_cut_mask(unsigned long long r, int x, int y, unsigned int mask,
-                                                   unsigned int left) {
-    const int w = rect_max_tx(r) - rect_min_tx(r) + 1;
-    for (int k = 0; k < 16; ++k) {
-        const long long q = (long long)(y + k / 4 - rect_min_ty(r)) * w + (x + k % 4 - rect_min_tx(r));
-        if (q >= (long long)left) mask &= ~(1u << k);
-    }
-    return mask;
-}
-
 /* A splat's rectangle in cells, and its tile and cell counts. */
 struct CellRect {
     unsigned int tiles;   /* below 2^24, so that 256 of them fit 32 bits */
@@ -446,6 +434,10 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
                 if (tid == 0) {
                     const long long left = V - p0 - q * kEmitThreads;
                     emit_cut(s, tile_base < cap ? cap - tile_base : 0u, (int)(left < kEmitThreads ? left : kEmitThreads));
+                    if (s.cut_tiles) {   /* keys without masks: the lists form them again */
+                        ctrl->cut_splat = s.aux[s.cut].y + 1u;
+                        ctrl->cut_tiles = s.cut_tiles;
+                    }
                 }
                 __syncthreads();
                 kept_pairs = s.kept;
@@ -508,7 +500,7 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
                             const int x = (int)(rect_min_tx(rect) / kCellSide + column) * kCellSide;
                             const int y = (int)(rect_min_ty(rect) / kCellSide + row) * kCellSide;
                             unsigned int mask = cell_mask(rect, x, y);
-                            if (over && (unsigned int)lo == cut) mask = emit_cut_mask(rect, x, y, mask, s.cut_tiles);
+                            if (over && (unsigned int)lo == cut) mask = cut_mask(rect, x, y, mask, s.cut_tiles);
                             key |= mask << 16;
                         }
                         f.keys[0][pos] = key;

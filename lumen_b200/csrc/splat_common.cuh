@@ -63,8 +63,10 @@ struct Control {
     unsigned int count_ticket;           /* unit order of the batch visibility count */
     unsigned int offsets_ticket;         /* tile order of the batch offset scan */
     unsigned int n_segments;             /* of the cells' sorted pairs (lists.cu) */
-    unsigned int pad;
     unsigned int order_offset;           /* where the tiles' order starts, in 256 bytes from here, or 0 */
+    unsigned int cut_splat, cut_tiles;   /* at the instance capacity: 1 + the visible index of the splat
+                                            that fits only in part (or 0), and how many of its tiles do */
+    unsigned int pad;
     unsigned int group_total[kTileGroups];   /* instances per group of tiles */
     unsigned int class_total[kTileClasses], class_taken[kTileClasses];   /* tiles per class of list length */
     SortControl depth_sort;              /* visible splats by depth key */
@@ -294,6 +296,17 @@ __device__ __forceinline__ unsigned int cell_mask(unsigned long long rect, int x
     const unsigned int columns = (0xFu >> (3 - x1)) & (0xFu << x0);
     const unsigned int rows = (0xFFFFu >> (4 * (3 - y1))) & (0xFFFFu << (4 * y0));
     return (columns * 0x1111u) & rows;
+}
+
+/* Of mask, the tiles of the cell whose first tile is (x, y) that are among the
+ * first `left` of the rectangle's, row-major. */
+__device__ inline unsigned int cut_mask(unsigned long long rect, int x, int y, unsigned int mask, unsigned int left) {
+    const int w = rect_max_tx(rect) - rect_min_tx(rect) + 1;
+    for (int k = 0; k < kCellSide * kCellSide; ++k) {
+        const long long q = (long long)(y + k / kCellSide - rect_min_ty(rect)) * w + (x + k % kCellSide - rect_min_tx(rect));
+        if (q >= (long long)left) mask &= ~(1u << k);
+    }
+    return mask;
 }
 
 /* The scene group that owns batch projection unit u: the last view with
