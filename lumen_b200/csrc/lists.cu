@@ -11,8 +11,8 @@
  * depth order, and the cell sort keeps that order within a cell. Here each
  * cell's list is split over its 16 tiles by the pairs' tile masks, in order:
  *
- *   list_count_kernel   per segment of 256 pairs of a cell: the instances of
- *                       each of its tiles before it
+ *   list_count_kernel   per segment of 256 pairs of a cell (or of a part of a
+ *                       long cell): the instances of each of its tiles before it
  *   list_scan_kernel    an exclusive scan of the tiles' counts: the ranges, the
  *                       touched tiles, each view's first instance
  *   list_write_kernel   per segment: a vote per tile and 32 pairs gives every
@@ -40,6 +40,8 @@ constexpr int kWriteThreads = 128;
 constexpr int kWriteWarps = kWriteThreads / 32;
 constexpr int kWriteCtas = 6;                   /* per SM */
 constexpr int kSegment = 256;                   /* pairs of a cell that a warp counts and writes at a time */
+constexpr int kLongCell = 8192;                 /* cells of more pairs are counted in parts, */
+constexpr int kWindow = 16384;                  /* cut at multiples of so many sorted pairs */
 constexpr int kCellTiles = kCellSide * kCellSide;
 
 /* A cell in its view. */
@@ -119,21 +121,23 @@ __device__ __forceinline__ SortedPairs sorted_pairs(const LumenGpuFrame& f, cons
             ctrl->cut_splat, ctrl->cut_tiles};
 }
 
-/* A segment: up to 256 consecutive pairs of one cell, as the count kernel
- * leaves it for the write kernel. They lie in the cell sort's look-back rows,
- * which nothing reads once it is done (2 B per instance that the frame can
- * hold, against 80 B per 256 pairs and per cell). Without enough room, a warp
- * writes a whole cell. */
+/* A segment: up to 256 consecutive pairs of one part of a cell, as the count
+ * kernel leaves it for the write kernel. They lie in the cell sort's look-back
+ * rows, which nothing reads once it is done (2 B per instance that the frame can
+ * hold, against 80 B per 256 pairs and per part, and 64 B per part). Without
+ * enough room, a warp writes a whole cell. */
 struct Segment {
-    int first, n;               /* its pairs */
+    int first;
+    unsigned int n_part;        /* its pairs (10 bits), and its part's number in the cell */
     unsigned int tile0;         /* the cell's first tile, and the view's tiles per row */
     int tiles_x;
-    unsigned int before[kCellTiles];   /* per tile, its instances in the cell's pairs before */
+    unsigned int before[kCellTiles];   /* per tile, its instances in the part's pairs before */
 };
 static_assert(sizeof(Segment) == 80, "16-byte aligned");
 
 /* Scratch after the cell sort: the tiles' order (u32 per tile), if there is to
- * be one, then the segments. offset: of p in the frame's scratch. */
+ * be one, then the parts' totals, then the segments. offset: of p in the
+ * frame's scratch. */
 struct Room {
     unsigned char* p;
     long long bytes, offset;
@@ -145,14 +149,26 @@ __device__ __forceinline__ bool has_order(const Room& room, const ViewTable* vt)
     return n >= room.order_min && n <= room.order_max && n * 4 <= room.bytes;
 }
 
+/* The work items of the count: a cell, or (from n_cells on) a window of
+ * sorted pairs that lies in a long cell which starts before it. Part 0 of a
+ * cell is the cell's item; part k the window k after the one that the cell starts
+ * in. total: per item and tile, the part's instances. */
 struct SegmentRoom {
+    unsigned int (*total)[kCellTiles];
     Segment* p;
     long long n;
 };
 
-__device__ __forceinline__ SegmentRoom segment_room(const Room& room, const ViewTable* vt) {
+__device__ __forceinline__ long long count_items(const ViewTable* vt, int n_pairs) {
+    return vt->hdr.total_cells + (n_pairs + kWindow - 1) / kWindow;
+}
+
+__device__ __forceinline__ SegmentRoom segment_room(const Room& room, const ViewTable* vt, int n_pairs) {
     const long long order = has_order(room, vt) ? (vt->hdr.total_tiles * 4 + 15) / 16 * 16 : 0;
-    return {reinterpret_cast<Segment*>(room.p + order), max(room.bytes - order, 0ll) / (long long)sizeof(Segment)};
+    const long long totals = count_items(vt, n_pairs) * (long long)sizeof(unsigned int[kCellTiles]);
+    return {reinterpret_cast<unsigned int(*)[kCellTiles]>(room.p + order),
+            reinterpret_cast<Segment*>(room.p + order + totals),
+            max(room.bytes - order - totals, 0ll) / (long long)sizeof(Segment)};
 }
 
 /* Class of a tile's list length n: higher for longer lists. */
@@ -162,7 +178,7 @@ __device__ __forceinline__ int length_class(unsigned int n) {
 }
 
 __device__ __forceinline__ bool has_room(const SegmentRoom& room, const ViewTable* vt, int n_pairs) {
-    return n_pairs / kSegment + vt->hdr.total_cells <= room.n;
+    return n_pairs / kSegment + count_items(vt, n_pairs) <= room.n;
 }
 
 /* The cell's range among the sorted pairs to bounds[0], bounds[1]: as the
@@ -179,13 +195,17 @@ __device__ __forceinline__ void find_bounds(int* bounds, const SortedPairs& in, 
     }
 }
 
-/* One CTA per cell, eight segments at a time (a warp each, all its keys'
+/* One CTA per item, eight segments at a time (a warp each, all its keys'
  * reads in flight, the next eight's before these are counted). Bound by the
- * latency of those reads (4 B per pair, once). */
+ * latency of those reads (4 B per pair, once), about 0.6 us per step of 2048
+ * pairs: a cell of 2 M pairs alone took 590 us (2 M splats in a 64x64 image: the
+ * frame 1.81 ms, against 1.22 with the instances sorted by tile), so long cells
+ * are counted in parts by as many CTAs. A part's counts start at 0 (the write
+ * kernel adds the totals of the parts before); the tiles' totals are added up by
+ * atomics, and the last part to arrive knows them. */
 __global__ void __launch_bounds__(kCountThreads)
 list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, Room scratch) {
     chain_begin();
-    const SegmentRoom room = segment_room(scratch, vt);
     const bool order = has_order(scratch, vt);
     constexpr int kReads = kSegment / 32;
     __shared__ int bounds[2];
@@ -193,15 +213,38 @@ list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ct
     __shared__ unsigned int count[2][kCountWarps][kCellTiles];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const SortedPairs in = sorted_pairs(f, ctrl, vt);
+    const SegmentRoom room = segment_room(scratch, vt, in.n);
     const bool noted = has_room(room, vt, in.n);
     const int* cells = ctrl->cells_by_sort ? cell_ranges(f, ctrl, vt) : nullptr;
     const long long n_cells = vt->hdr.total_cells, group = tile_group_size(vt->hdr.total_tiles);
+    const long long n_items = count_items(vt, in.n);
+    const unsigned int id_mask = in.packed ? (unsigned int)(kPackedCells - 1) : 0xFFFFFFFFu;
     const int n_views = vt->hdr.n_views;
-    for (long long cell = blockIdx.x; cell < n_cells; cell += gridDim.x) {
+    for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
+        const int window = item < n_cells ? -1 : (int)(item - n_cells);
+        const long long cell = window < 0 ? item : (long long)(in.keys[(long long)window * kWindow] & id_mask);
+        if (cell >= n_cells) {   /* self-check: a key that names no cell */
+            if (tid == 0) atomicOr(&ctrl->error_flags, LUMEN_GPU_ERR_BOUNDS);
+            continue;
+        }
         find_bounds(bounds, in, cells, cell);
         const Cell c = find_cell(vt, n_views, cell);
         __syncthreads();
-        const int first = bounds[0], end = bounds[1];
+        const int cell_first = bounds[0], cell_end = bounds[1];
+        const bool in_parts = cell_end - cell_first > kLongCell;
+        /* the item's pairs */
+        int first = cell_first, end = cell_end;
+        unsigned int part = 0u;
+        if (window >= 0) {
+            first = window * kWindow;
+            part = (unsigned int)(window - cell_first / kWindow);
+            if (!in_parts || cell_first >= first) first = end;   /* the cell's own item has them */
+        }
+        if (in_parts) end = (int)min((long long)end, ((long long)first / kWindow + 1) * kWindow);
+        if (window >= 0 && first >= end) {
+            __syncthreads();
+            continue;
+        }
         const int n_seg = first < end ? (end - first + kSegment - 1) / kSegment : 0;
         if (tid == 0 && n_seg) slot_s = noted ? atomicAdd(&ctrl->n_segments, (unsigned int)n_seg) : 0u;
         unsigned int m[kReads], base = 0u;   /* base: lane k < 16, tile k's instances so far */
@@ -243,19 +286,35 @@ list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ct
                 if (noted && seg < n_seg) room.p[slot_s + seg].before[lane] = before;
             } else if (lane == kCellTiles && noted && seg < n_seg) {
                 const int i0 = first + seg * kSegment;
+                const unsigned int n = end - i0 < kSegment ? (unsigned int)(end - i0) : (unsigned int)kSegment;
                 *reinterpret_cast<int4*>(room.p + slot_s + seg) =
-                    make_int4(i0, end - i0 < kSegment ? end - i0 : kSegment,
-                              (int)(c.tile_begin + (long long)c.y * c.tiles_x + c.x), c.tiles_x);
+                    make_int4(i0, (int)(n | part << 10), (int)(c.tile_begin + (long long)c.y * c.tiles_x + c.x), c.tiles_x);
             }
         }
         if (warp == 0) {
             const long long t = lane < kCellTiles ? c.tile(lane) : -1;
-            const unsigned int tiles = __ballot_sync(0xffffffffu, t >= 0);
-            if (t >= 0) {
-                f.ranges[2 * t + 1] = (int)base;
-                if (base) atomicAdd(&ctrl->group_total[t / group], base);
-                if (order) {
-                    const int cls = length_class(base);
+            if (t >= 0 && base) atomicAdd(&ctrl->group_total[t / group], base);
+            unsigned int total = base;
+            bool known = true;
+            if (!in_parts) {
+                if (t >= 0) f.ranges[2 * t + 1] = (int)base;
+            } else {
+                if (noted && lane < kCellTiles) room.total[item][lane] = base;
+                /* the emission has zeroed the ranges; the first tile's other
+                 * word counts the parts that have arrived */
+                if (t >= 0) atomicAdd(f.ranges + 2 * t + 1, (int)base);
+                __threadfence();
+                __syncwarp();
+                int arrived = lane == 0 ? atomicAdd(f.ranges + 2 * t, 1) : 0;
+                arrived = __shfl_sync(0xffffffffu, arrived, 0);
+                known = arrived == (cell_end - 1) / kWindow - cell_first / kWindow;
+                __threadfence();
+                if (known && t >= 0) total = (unsigned int)__ldcg(f.ranges + 2 * t + 1);
+            }
+            if (order && known) {
+                const unsigned int tiles = __ballot_sync(0xffffffffu, t >= 0);
+                const int cls = length_class(total);
+                if (t >= 0) {
                     const unsigned int same = __match_any_sync(tiles, cls);
                     if (lane == __ffs(same) - 1) atomicAdd(&ctrl->class_total[cls], (unsigned int)__popc(same));
                 }
@@ -361,10 +420,11 @@ list_scan_kernel(ViewTable* vt, int* __restrict__ ranges, Control* ctrl, Room ro
 __global__ void __launch_bounds__(kWriteThreads, kWriteCtas)
 list_write_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, Room scratch) {
     chain_begin();
-    const SegmentRoom room = segment_room(scratch, vt);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const SortedPairs in = sorted_pairs(f, ctrl, vt);
+    const SegmentRoom room = segment_room(scratch, vt, in.n);
     const bool noted = has_room(room, vt, in.n);
+    const unsigned int id_mask = in.packed ? (unsigned int)(kPackedCells - 1) : 0xFFFFFFFFu;
     const unsigned int out = ctrl->list_buffer;
     unsigned int* __restrict__ kout = out ? f.keys[1] : f.keys[0];
     unsigned int* __restrict__ vout = out ? f.vals[1] : f.vals[0];
@@ -377,17 +437,26 @@ list_write_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ct
         if (noted) {
             const int4 seg = *reinterpret_cast<const int4*>(room.p + w);
             i0 = seg.x;
-            end = seg.x + seg.y;
+            end = seg.x + (seg.y & 1023);
             tile0 = (unsigned int)seg.z;
             tiles_x = seg.w;
             if (lane < kCellTiles) before = room.p[w].before[lane];
+            if (const int part = (int)((unsigned int)seg.y >> 10)) {
+                /* the parts of the cell before, two at a time */
+                const long long cell = min((long long)(in.keys[i0] & id_mask), vt->hdr.total_cells - 1);
+                const long long window = vt->hdr.total_cells + i0 / kWindow;   /* the part's own item */
+                unsigned int sum = 0u;
+#pragma unroll 4
+                for (int k = lane / kCellTiles; k < part; k += 2)
+                    sum += room.total[k ? window - part + k : cell][lane % kCellTiles];
+                before += sum + __shfl_down_sync(0xffffffffu, sum, kCellTiles);
+            }
             if (!in.packed) {
                 const ViewDesc& vd = vt->view[find_view_by_tile(vt, vt->hdr.n_views, tile0)];
                 cx = (int)((tile0 - vd.tile_begin) % tiles_x);
                 cy = (int)((tile0 - vd.tile_begin) / tiles_x);
             }
         } else {
-            const unsigned int id_mask = in.packed ? (unsigned int)(kPackedCells - 1) : 0xFFFFFFFFu;
             i0 = first_of_cell(in.keys, in.n, id_mask, (unsigned int)w);
             end = first_of_cell(in.keys, in.n, id_mask, (unsigned int)w + 1u);
             const Cell c = find_cell(vt, vt->hdr.n_views, w);
@@ -458,11 +527,11 @@ void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned
      * 4K, 32400 tiles: 288 -> 301). */
     const long long line = (long long)kCompositeBlocksPerSm * num_sms;
     const Room room{scratch + room_offset, room_bytes, room_offset, line + line / 2, 10 * line};
-    launch_chained(list_count_kernel, dim3(grid_of(n_cells, 64ll * num_sms)), dim3(kCountThreads), 0, st,
-                   (const ViewTable*)vt, f, ctrl, room);
+    launch_chained(list_count_kernel, dim3(grid_of(n_cells + f.instance_capacity / kWindow, 64ll * num_sms)),
+                   dim3(kCountThreads), 0, st, (const ViewTable*)vt, f, ctrl, room);
     launch_chained(list_scan_kernel, dim3(grid_of((n_tiles + kScanThreads - 1) / kScanThreads, 2ll * num_sms)),
                    dim3(kScanThreads), 0, st, vt, f.ranges, ctrl, room);
-    const long long most = f.instance_capacity / kSegment + n_cells;   /* segments, or cells */
+    const long long most = f.instance_capacity / kSegment + n_cells + f.instance_capacity / kWindow;   /* segments, or cells */
     launch_chained(list_write_kernel, dim3(grid_of((most + kWriteWarps - 1) / kWriteWarps, kWriteCtas * num_sms)),
                    dim3(kWriteThreads), 0, st, (const ViewTable*)vt, f, ctrl, room);
 }

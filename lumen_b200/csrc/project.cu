@@ -305,7 +305,8 @@ constexpr unsigned int kEmitLaneCells = 16;
  * cell ids it writes (per CTA in shared memory, added to the sort's histogram
  * once all its tickets are done) and clears the sort's look-back descriptors of
  * the 256 * sort_items-key tiles that start among its pairs. It also fills the
- * cells' ranges with (-1, -1) for the sort's last pass.
+ * cells' ranges with (-1, -1) for the sort's last pass and the tiles' with zeros
+ * for the lists' counts.
  *
  * Instances (the tiles of the rectangles) are only counted here; those
  * beyond the capacity are left out of the pairs, so that the lists hold the
@@ -343,6 +344,9 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
         const long long nthreads = (long long)gridDim.x * blockDim.x;
         for (long long j = (long long)blockIdx.x * blockDim.x + tid; j < 2 * n_cells; j += nthreads) ranges[j] = -1;
     }
+    for (long long j = (long long)blockIdx.x * blockDim.x + tid; j < 2 * vt->hdr.total_tiles;
+         j += (long long)gridDim.x * blockDim.x)
+        f.ranges[j] = 0;
     unsigned int kor = 0u, knot = 0u;
     unsigned long long tile_sum = 0ull;
     for (;;) {
