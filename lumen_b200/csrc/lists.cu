@@ -35,6 +35,9 @@ namespace {
 
 constexpr int kCountThreads = 256;
 constexpr int kCountWarps = kCountThreads / 32;
+/* At most so many CTAs per SM, whatever the cells: a persistent launch, sized for
+ * the most cells that its buffers hold, spent 8 us on starting 64 per SM. */
+constexpr int kCountCtas = 16;
 constexpr int kScanThreads = 1024;
 constexpr int kWriteThreads = 128;
 constexpr int kWriteWarps = kWriteThreads / 32;
@@ -527,7 +530,7 @@ void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned
      * 4K, 32400 tiles: 288 -> 301). */
     const long long line = (long long)kCompositeBlocksPerSm * num_sms;
     const Room room{scratch + room_offset, room_bytes, room_offset, line + line / 2, 10 * line};
-    launch_chained(list_count_kernel, dim3(grid_of(n_cells + f.instance_capacity / kWindow, 64ll * num_sms)),
+    launch_chained(list_count_kernel, dim3(grid_of(n_cells + f.instance_capacity / kWindow, (long long)kCountCtas * num_sms)),
                    dim3(kCountThreads), 0, st, (const ViewTable*)vt, f, ctrl, room);
     launch_chained(list_scan_kernel, dim3(grid_of((n_tiles + kScanThreads - 1) / kScanThreads, 2ll * num_sms)),
                    dim3(kScanThreads), 0, st, vt, f.ranges, ctrl, room);

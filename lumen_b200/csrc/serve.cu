@@ -13,7 +13,7 @@
  * control block and view table (out), and one captured graph per launch
  * variant. The graph holds: table upload, frame init and the persistent
  * pipeline up to the tiles' lists (grids fixed; sizes read from the table).
- * The compositor, whose grid is the batch's tiles, the counter read-back and
+ * The compositor, whose grids are the batch's tiles, the counter read-back and
  * the per-request byte copies follow the graph.
  */
 #include <algorithm>
@@ -21,6 +21,7 @@
 #include <chrono>
 #include <cmath>
 #include <condition_variable>
+#include <cstddef>
 #include <cstring>
 #include <deque>
 #include <map>
@@ -66,9 +67,12 @@ int variant_of(int chunk, int items) {
  * against 15.2 to 17.9, and the first images wait longer. */
 constexpr int64_t kBatchTileIds = 1ll << 16;
 
-/* Bands of rows of a view that is alone in its batch, each a wave of tiles. */
+/* The least tiles of a part of a batch (composite_and_copy), about a wave, and
+ * the bands of rows of a view that is alone in its batch. */
+constexpr long long kPartTiles = 1024;
 constexpr int kBands = 4;
-constexpr long long kBandTiles = 1024;
+
+constexpr size_t kControlHead = offsetof(Control, proj_ticket);   /* the counters that the host reads back */
 
 /* FIFO admission: the longest prefix of the queue whose sums fit. */
 int admit_prefix(const int64_t* slots, const int64_t* tiles, const int64_t* inst, const int64_t* pix, int n,
@@ -294,28 +298,31 @@ void enqueue_batch_work(LumenServer* srv, Slot* s, const LaunchConfig& lc, bool 
 }
 
 /* The images: the compositor, the counter read-back and the copies to the
- * host. The batch is composited view by view, a view alone in four bands of
- * rows, and each part leaves for the host while the next is composited: copied
- * after the whole batch, the last batches of a burst left the GPU idle for
- * 0.12 ms per view. A burst of 16 views of 1 M Gaussians at 1080p takes 5.1 ms
- * instead of 5.4 in batches of four, 4.7 instead of 5.5 in batches of eight. */
+ * host. A batch of two waves of tiles or more is composited in parts, runs of
+ * views or, for a view alone, bands of rows, and each part leaves for the host
+ * while the next is composited: copied after the whole batch, the last batches
+ * of a burst left the GPU idle for 0.12 ms per view. A burst of 16 views of 1 M
+ * Gaussians at 1080p takes 5.1 ms instead of 5.4 in batches of four, 4.7 instead
+ * of 5.5 in batches of eight. A part has a wave of tiles at least: the next one
+ * starts when its last tile ends, so smaller ones leave SMs idle (64 views of
+ * 64x64 pixels and 200 k Gaussians, one by one 37 ms, at once 7). */
 cudaError_t composite_and_copy(LumenServer* srv, Slot* s, const LaunchConfig& lc, long long n_tiles,
                                size_t table_bytes) {
-    struct Part {
-        long long tile, n_tiles;       /* of the batch */
-        uint8_t* to;
-        const uint8_t* from;
-        size_t bytes;
-    };
     unsigned char* base = (unsigned char*)s->frame.scratch;
     Control* ctrl = (Control*)(base + s->layout.control_off);
     const ViewTable* vt = (const ViewTable*)(base + s->layout.table_off);
     const ViewTable* host = (const ViewTable*)s->h_table;
     const int nv = (int)s->batch.size(), sms = device_sm_count();
-    const int bands = nv == 1 && n_tiles >= kBands * kBandTiles ? kBands : 1;
-    const bool split = nv > 1 || bands > 1;
-    std::vector<Part> parts;
-    long long pix = 0;
+    const int bands = nv == 1 && n_tiles >= kBands * kPartTiles ? kBands : 1;
+    struct Copy {
+        uint8_t* to;
+        const uint8_t* from;
+        size_t bytes;
+        int part;                       /* the part that completes it */
+    };
+    std::vector<Copy> copies;
+    std::vector<long long> part_tiles(1, 0);
+    long long pix = 0, left = n_tiles;   /* tiles after the parts so far */
     for (int v = 0; v < nv; ++v) {
         const Request& r = *s->batch[(size_t)v];
         const ViewDesc& d = host->view[v];
@@ -323,34 +330,34 @@ cudaError_t composite_and_copy(LumenServer* srv, Slot* s, const LaunchConfig& lc
         for (int b = 0; b < bands; ++b) {
             const long long r0 = rows * b / bands, r1 = rows * (b + 1) / bands;
             const long long y0 = r0 * kTile, y1 = std::min<long long>(r1 * kTile, r.cam.height);
-            parts.push_back({d.tile_begin + r0 * d.tiles_x, (r1 - r0) * d.tiles_x,
-                             r.out ? (uint8_t*)r.out + y0 * row_bytes : nullptr, s->d_rgb8 + pix * 3 + y0 * row_bytes,
-                             (size_t)((y1 - y0) * row_bytes)});
+            if (part_tiles.back() >= kPartTiles && left - part_tiles.back() >= kPartTiles) {
+                left -= part_tiles.back();
+                part_tiles.push_back(0);
+            }
+            part_tiles.back() += (r1 - r0) * d.tiles_x;
+            copies.push_back({(uint8_t*)r.out + y0 * row_bytes, s->d_rgb8 + pix * 3 + y0 * row_bytes,
+                              (size_t)((y1 - y0) * row_bytes), (int)part_tiles.size() - 1});
         }
         pix += r.pixels;
     }
-    auto composite = [&](long long first, long long n) {
-        launch_composite(vt, nv, s->frame, ctrl, srv->cfg.options, first, n, !split, lc.composite_chunk, lc.track != 0,
-                         sms, s->stream);
-    };
+    const bool split = part_tiles.size() > 1;
     cudaError_t e = cudaSuccess;
-    if (!split) {
-        composite(0, n_tiles);
-    } else {
-        for (size_t i = 0; i < parts.size() && e == cudaSuccess; ++i) {
-            composite(parts[i].tile, parts[i].n_tiles);
-            e = cudaEventRecord(s->ev_parts[i], s->stream);
-        }
+    long long first = 0;
+    for (size_t i = 0; i < part_tiles.size() && e == cudaSuccess; ++i) {
+        launch_composite(vt, nv, s->frame, ctrl, srv->cfg.options, first, part_tiles[i], !split, lc.composite_chunk,
+                         lc.track != 0, sms, s->stream);
+        first += part_tiles[i];
+        if (split) e = cudaEventRecord(s->ev_parts[i], s->stream);
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(s->h_back, ctrl, sizeof(Control), cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(s->h_back, ctrl, kControlHead, cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(s->h_back + sizeof(Control), vt, table_bytes, cudaMemcpyDeviceToHost, s->stream);
     const cudaStream_t to = split ? s->copies : s->stream;
-    for (size_t i = 0; i < parts.size() && e == cudaSuccess; ++i) {
-        if (!parts[i].to) continue;
-        if (split) e = cudaStreamWaitEvent(to, s->ev_parts[i], 0);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(parts[i].to, parts[i].from, parts[i].bytes, cudaMemcpyDeviceToHost, to);
+    int waited = -1;
+    for (size_t i = 0; i < copies.size() && e == cudaSuccess; ++i) {
+        const Copy& c = copies[i];
+        if (split && c.part != waited) e = cudaStreamWaitEvent(to, s->ev_parts[(size_t)(waited = c.part)], 0);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(c.to, c.from, c.bytes, cudaMemcpyDeviceToHost, to);
     }
     if (split) {   /* the slot's stream goes on when the images have left */
         if (e == cudaSuccess) e = cudaEventRecord(s->ev_copied, s->copies);
@@ -527,8 +534,8 @@ void completer_main(LumenServer* srv, Slot* s) {
         if (e == cudaSuccess) e = cudaEventSynchronize(s->ev_end);
         float ms = 0.0f;
         if (e == cudaSuccess) cudaEventElapsedTime(&ms, s->ev_start, s->ev_end);
-        Control c;
-        std::memcpy(&c, s->h_back, sizeof(Control));
+        Control c;   /* its counters */
+        std::memcpy(&c, s->h_back, kControlHead);
         const ViewTable* vt = (const ViewTable*)(s->h_back + sizeof(Control));
         lk.lock();
         const int nv = (int)s->batch.size();
