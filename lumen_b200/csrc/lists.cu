@@ -43,7 +43,7 @@ constexpr int kWriteThreads = 128;
 constexpr int kWriteWarps = kWriteThreads / 32;
 constexpr int kWriteCtas = 6;                   /* per SM */
 constexpr int kSegment = 256;                   /* pairs of a cell that a warp counts and writes at a time */
-constexpr int kLongCell = 8192;                 /* cells of more pairs are counted in parts, */
+constexpr int kLongCell = 24576;                /* cells of more pairs are counted in parts, */
 constexpr int kWindow = 16384;                  /* cut at multiples of so many sorted pairs */
 constexpr int kCellTiles = kCellSide * kCellSide;
 
@@ -115,12 +115,15 @@ __device__ __forceinline__ unsigned int pair_mask(const SortedPairs& in, unsigne
     return v + 1u == in.cut_splat ? cut_mask(rect, x, y, mask, in.cut_tiles) : mask;
 }
 
+/* kPacked: the cells are known to be few enough for packed keys (kernels that
+ * may have to form masks take 40 more registers). */
+template <bool kPacked>
 __device__ __forceinline__ SortedPairs sorted_pairs(const LumenGpuFrame& f, const Control* ctrl,
                                                     const ViewTable* vt) {
     const unsigned int b = ctrl->cell_sort.sorted_buffer;
     const long long n = (long long)ctrl->cell_sort.n;
     return {b ? f.keys[1] : f.keys[0], b ? f.vals[1] : f.vals[0],
-            (int)(n < f.instance_capacity ? n : f.instance_capacity), vt->hdr.total_cells <= kPackedCells,
+            (int)(n < f.instance_capacity ? n : f.instance_capacity), kPacked || vt->hdr.total_cells <= kPackedCells,
             ctrl->cut_splat, ctrl->cut_tiles};
 }
 
@@ -201,11 +204,14 @@ __device__ __forceinline__ void find_bounds(int* bounds, const SortedPairs& in, 
 /* One CTA per item, eight segments at a time (a warp each, all its keys'
  * reads in flight, the next eight's before these are counted). Bound by the
  * latency of those reads (4 B per pair, once), about 0.6 us per step of 2048
- * pairs: a cell of 2 M pairs alone took 590 us (2 M splats in a 64x64 image: the
- * frame 1.81 ms, against 1.22 with the instances sorted by tile), so long cells
- * are counted in parts by as many CTAs. A part's counts start at 0 (the write
+ * pairs, so long cells are counted in parts by as many CTAs: a cell of 2 M pairs
+ * by one CTA took 590 us (2 M splats in a 64x64 image: the frame 1.81 ms, in
+ * parts 1.26, and 1.22 with the instances sorted by tile; 1 M in 128x72 0.70,
+ * 0.52 and 0.54). With cells of 8192 pairs already in parts, 2 M splats at 4K
+ * counted 31 us instead of 23. A part's counts start at 0 (the write
  * kernel adds the totals of the parts before); the tiles' totals are added up by
  * atomics, and the last part to arrive knows them. */
+template <bool kPacked>
 __global__ void __launch_bounds__(kCountThreads)
 list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, Room scratch) {
     chain_begin();
@@ -215,7 +221,7 @@ list_count_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ct
     __shared__ unsigned int slot_s;
     __shared__ unsigned int count[2][kCountWarps][kCellTiles];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const SortedPairs in = sorted_pairs(f, ctrl, vt);
+    const SortedPairs in = sorted_pairs<kPacked>(f, ctrl, vt);
     const SegmentRoom room = segment_room(scratch, vt, in.n);
     const bool noted = has_room(room, vt, in.n);
     const int* cells = ctrl->cells_by_sort ? cell_ranges(f, ctrl, vt) : nullptr;
@@ -420,11 +426,12 @@ list_scan_kernel(ViewTable* vt, int* __restrict__ ranges, Control* ctrl, Room ro
  * kernels 464 us, with 32 warps 480, with 48 and segments of 128 pairs 769); a
  * transpose and a gather in shared memory took half as many instructions again
  * (2 M at 4K: 98 against 71 us). */
+template <bool kPacked>
 __global__ void __launch_bounds__(kWriteThreads, kWriteCtas)
 list_write_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, Room scratch) {
     chain_begin();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const SortedPairs in = sorted_pairs(f, ctrl, vt);
+    const SortedPairs in = sorted_pairs<kPacked>(f, ctrl, vt);
     const SegmentRoom room = segment_room(scratch, vt, in.n);
     const bool noted = has_room(room, vt, in.n);
     const unsigned int id_mask = in.packed ? (unsigned int)(kPackedCells - 1) : 0xFFFFFFFFu;
@@ -530,13 +537,17 @@ void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned
      * 4K, 32400 tiles: 288 -> 301). */
     const long long line = (long long)kCompositeBlocksPerSm * num_sms;
     const Room room{scratch + room_offset, room_bytes, room_offset, line + line / 2, 10 * line};
-    launch_chained(list_count_kernel, dim3(grid_of(n_cells + f.instance_capacity / kWindow, (long long)kCountCtas * num_sms)),
-                   dim3(kCountThreads), 0, st, (const ViewTable*)vt, f, ctrl, room);
+    const bool packed = n_cells <= kPackedCells;
+    const long long windows = f.instance_capacity / kWindow;
+    launch_chained(packed ? list_count_kernel<true> : list_count_kernel<false>,
+                   dim3(grid_of(n_cells + windows, (long long)kCountCtas * num_sms)), dim3(kCountThreads), 0, st,
+                   (const ViewTable*)vt, f, ctrl, room);
     launch_chained(list_scan_kernel, dim3(grid_of((n_tiles + kScanThreads - 1) / kScanThreads, 2ll * num_sms)),
                    dim3(kScanThreads), 0, st, vt, f.ranges, ctrl, room);
-    const long long most = f.instance_capacity / kSegment + n_cells + f.instance_capacity / kWindow;   /* segments, or cells */
-    launch_chained(list_write_kernel, dim3(grid_of((most + kWriteWarps - 1) / kWriteWarps, kWriteCtas * num_sms)),
-                   dim3(kWriteThreads), 0, st, (const ViewTable*)vt, f, ctrl, room);
+    const long long most = f.instance_capacity / kSegment + n_cells + windows;   /* segments, or cells */
+    launch_chained(packed ? list_write_kernel<true> : list_write_kernel<false>,
+                   dim3(grid_of((most + kWriteWarps - 1) / kWriteWarps, kWriteCtas * num_sms)), dim3(kWriteThreads), 0,
+                   st, (const ViewTable*)vt, f, ctrl, room);
 }
 
 }  // namespace lumen
