@@ -467,8 +467,7 @@ static float stop_transmittance(const LumenRenderOptions& opt) {
 
 template <int kChunk, bool kTrack>
 static void launch_composite_chunk(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
-                                   const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
-                                   int num_sms, cudaStream_t st) {
+                                   const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole, cudaStream_t st) {
     launch_chained(composite_kernel<kChunk, kTrack>, dim3((unsigned int)n_tiles), dim3(kCompositeThreads), 0, st, vt,
                    n_views, (const LumenSplatRecord*)f.records, f, (long long)f.instance_capacity, ctrl, opt,
                    tile_offset, whole, stop_transmittance(opt), -1.0f);
@@ -477,11 +476,11 @@ static void launch_composite_chunk(const ViewTable* vt, int n_views, const Lumen
 template <int kChunk>
 static void launch_composite_track(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
                                    const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
-                                   bool track, int num_sms, cudaStream_t st) {
+                                   bool track, cudaStream_t st) {
     if (track)
-        launch_composite_chunk<kChunk, true>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, num_sms, st);
+        launch_composite_chunk<kChunk, true>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, st);
     else
-        launch_composite_chunk<kChunk, false>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, num_sms, st);
+        launch_composite_chunk<kChunk, false>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, st);
 }
 
 /* Shades tiles [tile_offset, tile_offset + n_tiles) of the batch. whole: these
@@ -490,7 +489,7 @@ static void launch_composite_track(const ViewTable* vt, int n_views, const Lumen
  * contributor counts or last-visited offsets. */
 void launch_composite(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
                       const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
-                      int chunk, bool track, int num_sms, cudaStream_t st) {
+                      int chunk, bool track, cudaStream_t st) {
     if (n_tiles <= 0) return;
     /* Not chained: blocks that are resident before the list kernel ends are
      * placed where that leaves room, so the first (longest) tiles crowd on a
@@ -500,16 +499,13 @@ void launch_composite(const ViewTable* vt, int n_views, const LumenGpuFrame& f, 
     ChainedLaunches chained(false);
     switch (chunk) {
         case 128:
-            launch_composite_track<128>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, track, num_sms,
-                                        st);
+            launch_composite_track<128>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, track, st);
             break;
         case 512:
-            launch_composite_track<512>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, track, num_sms,
-                                        st);
+            launch_composite_track<512>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, track, st);
             break;
         default:
-            launch_composite_track<256>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, track, num_sms,
-                                        st);
+            launch_composite_track<256>(vt, n_views, f, ctrl, opt, tile_offset, n_tiles, whole, track, st);
             break;
     }
 }

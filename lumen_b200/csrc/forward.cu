@@ -44,7 +44,8 @@ void launch_cell_sort(const LumenGpuFrame& f, Control* ctrl, const ViewTable* vt
                       long long lb_tiles_cap, int items, CellDigits digits, bool wide, bool persistent, int num_sms,
                       cudaStream_t st);
 void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned char* scratch, long long room_offset,
-                  long long room_bytes, long long n_cells, long long n_tiles, int num_sms, cudaStream_t st);
+                  long long room_bytes, long long n_cells, long long n_tiles, long long order_most, int num_sms,
+                  cudaStream_t st);
 void launch_sort64(unsigned long long* k0, unsigned int* v0, unsigned long long* k1, unsigned int* v1,
                    long long capacity, SortControl* sc, unsigned int* lb, long long lb_tiles_cap, unsigned int* err,
                    int num_sms, cudaStream_t st);
@@ -53,7 +54,7 @@ void launch_sorted_keys64(const LumenGpuFrame& f, const Control* ctrl, int key_m
                           int num_sms, cudaStream_t st);
 void launch_composite(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
                       const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole,
-                      int chunk, bool track, int num_sms, cudaStream_t st);
+                      int chunk, bool track, cudaStream_t st);
 void configure_sort_kernels();
 
 int device_sm_count() {
@@ -184,11 +185,12 @@ constexpr long long kOnePassBlocks = 1024;
  * the projection units (plain launches). Projection is a visibility count,
  * an offset scan and the projection proper, Gaussian-major (each distinct
  * scene read once); a single view of few Gaussians runs one kernel with its
- * compacting scan fused in (project_kernel). */
+ * compacting scan fused in (project_kernel). order_most, without the
+ * compositor: the most tiles that the caller's own launch may take in line. */
 void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRenderOptions& opt,
                      const LumenGpuFrame& f, long long n_slots, long long n_tiles, long long n_cells, int n_views,
                      bool persistent, const LaunchConfig& lc, cudaEvent_t* ev, cudaStream_t s, bool with_composite,
-                     long long n_units) {
+                     long long n_units, long long order_most) {
     Control* ctrl = (Control*)(base + L.control_off);
     ViewTable* vt = (ViewTable*)(base + L.table_off);
     unsigned long long* proj_lb = (unsigned long long*)(base + L.proj_lb_off);
@@ -224,10 +226,10 @@ void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRen
     }
     if (ev) cudaEventRecord(ev[2], s);
     launch_lists(vt, f, ctrl, base, (long long)L.tile_lb_off, (long long)(L.total - L.tile_lb_off),
-                 n_cells, n_tiles, sms, s);
+                 n_cells, n_tiles, with_composite ? n_tiles : order_most, sms, s);
     if (ev) cudaEventRecord(ev[3], s);
     if (!with_composite) return;
-    launch_composite(vt, n_views, f, ctrl, opt, 0, n_tiles, true, lc.composite_chunk, lc.track != 0, sms, s);
+    launch_composite(vt, n_views, f, ctrl, opt, 0, n_tiles, true, lc.composite_chunk, lc.track != 0, s);
     if (ev) cudaEventRecord(ev[4], s);
 }
 
@@ -307,7 +309,7 @@ static LumenStatus forward_impl(const LumenGpuGaussians* g, const LumenViewCamer
     single_view_table(g, cam, img, L, tiles, &hdr, &v);
     if (ev) cudaEventRecord(ev[0], s);
     launch_init(L, base, &hdr, &v, s);
-    launch_pipeline(L, base, *opt, *f, g->count, tiles, hdr.total_cells, 1, false, lc, ev, s, true, hdr.total_units);
+    launch_pipeline(L, base, *opt, *f, g->count, tiles, hdr.total_cells, 1, false, lc, ev, s, true, hdr.total_units, 0);
     return map_cuda(cudaGetLastError());
 }
 
@@ -335,15 +337,14 @@ LumenStatus forward_banded(const LumenGpuGaussians* g, const LumenViewCamera* ca
     launch_init(L, base, &hdr, &v, s);
     const LaunchConfig lc = default_launch(g->count);
     launch_pipeline(L, base, *opt, *f, g->count, tiles, hdr.total_cells, 1, false, lc, nullptr, s, false,
-                    hdr.total_units);
+                    hdr.total_units, 0);
     Control* ctrl = (Control*)(base + L.control_off);
     const ViewTable* vt = (const ViewTable*)(base + L.table_off);
-    const int sms = device_sm_count();
     if (n_bands > tiles_y) n_bands = tiles_y;
     for (int b = 0; b < n_bands; ++b) {
         const int r0 = (int)((long long)tiles_y * b / n_bands), r1 = (int)((long long)tiles_y * (b + 1) / n_bands);
         launch_composite(vt, 1, *f, ctrl, *opt, (long long)r0 * tiles_x, (long long)(r1 - r0) * tiles_x, false,
-                         lc.composite_chunk, img->n_contrib || img->last_idx, sms, s);
+                         lc.composite_chunk, img->n_contrib || img->last_idx, s);
         const int y0 = r0 * kTile, y1 = r1 * kTile < cam->height ? r1 * kTile : cam->height;
         if (after_band) after_band(ctx, y0, y1, s);
     }
@@ -421,7 +422,7 @@ static LumenStatus batch_impl(const LumenGpuBatchView* views, int n_views, const
     for (int v = 0; v < n_views; ++v)
         if (views[v].image.n_contrib || views[v].image.last_idx) lc.track = 1;
     launch_pipeline(L, base, *opt, *f, slots, hdr.total_tiles, hdr.total_cells, n_views, false, lc, ev, s, true,
-                    hdr.total_units);
+                    hdr.total_units, 0);
     return map_cuda(cudaGetLastError());
 }
 

@@ -524,9 +524,12 @@ int grid_of(long long n, long long cap) { return (int)(n < 1 ? 1 : n < cap ? n :
 }  // namespace
 
 /* n_cells, n_tiles: the batch's, or upper bounds for a persistent launch
- * (the kernels read the batch's from the table; grids are strided). */
+ * (the kernels read the batch's from the table; grids are strided). order_most:
+ * the most tiles of a batch that may be composited in one launch, which goes by
+ * the tiles' order. */
 void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned char* scratch, long long room_offset,
-                  long long room_bytes, long long n_cells, long long n_tiles, int num_sms, cudaStream_t st) {
+                  long long room_bytes, long long n_cells, long long n_tiles, long long order_most, int num_sms,
+                  cudaStream_t st) {
     /* Longest lists first: a tile with a long list that starts late runs on
      * alone. Of use from one and a half to ten tiles per resident CTA of the
      * compositor. Compositor, in tile order and longest first: 100 k splats at
@@ -536,7 +539,8 @@ void launch_lists(ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, unsigned
      * more, neighbouring tiles no longer share their splats in the L2 (2 M at
      * 4K, 32400 tiles: 288 -> 301). */
     const long long line = (long long)kCompositeBlocksPerSm * num_sms;
-    const Room room{scratch + room_offset, room_bytes, room_offset, line + line / 2, 10 * line};
+    const Room room{scratch + room_offset, room_bytes, room_offset, line + line / 2,
+                    order_most < 10 * line ? order_most : 10 * line};
     const bool packed = n_cells <= kPackedCells;
     const long long windows = f.instance_capacity / kWindow;
     launch_chained(packed ? list_count_kernel<true> : list_count_kernel<false>,

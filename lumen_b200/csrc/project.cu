@@ -450,6 +450,7 @@ emit_kernel(const ViewTable* __restrict__ vt, LumenGpuFrame f, Control* ctrl, un
             auto count = [&](unsigned int cell) {
                 kor |= cell;
                 knot |= ~cell;
+                if (nd == 0) return;   /* one cell: nothing to sort */
                 atomicAdd(&s.hist[0][0] + (cell & digit_mask), 1u);
                 for (int d = 1; d < nd; ++d) atomicAdd(&s.hist[d][(cell >> (bits * d)) & digit_mask], 1u);
             };

@@ -44,10 +44,10 @@ void launch_init(const ScratchLayout& L, unsigned char* base, const BatchHeader*
 void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRenderOptions& opt,
                      const LumenGpuFrame& f, long long n_slots, long long n_tiles, long long n_cells, int n_views,
                      bool persistent, const LaunchConfig& lc, cudaEvent_t* ev, cudaStream_t s, bool with_composite,
-                     long long n_units);
+                     long long n_units, long long order_most);
 void launch_composite(const ViewTable* vt, int n_views, const LumenGpuFrame& f, Control* ctrl,
                       const LumenRenderOptions& opt, long long tile_offset, long long n_tiles, bool whole, int chunk,
-                      bool track, int num_sms, cudaStream_t st);
+                      bool track, cudaStream_t st);
 
 namespace {
 
@@ -293,7 +293,7 @@ void enqueue_batch_work(LumenServer* srv, Slot* s, const LaunchConfig& lc, bool 
         ChainedLaunches plain(false);
         launch_init(s->layout, base, nullptr, nullptr, s->stream);
         launch_pipeline(s->layout, base, srv->cfg.options, s->frame, n_slots, n_tiles, n_cells, n_views, persistent, lc,
-                        nullptr, s->stream, false, n_units);
+                        nullptr, s->stream, false, n_units, kBands * kPartTiles - 1);   /* more leave in parts */
     }
 }
 
@@ -312,7 +312,7 @@ cudaError_t composite_and_copy(LumenServer* srv, Slot* s, const LaunchConfig& lc
     Control* ctrl = (Control*)(base + s->layout.control_off);
     const ViewTable* vt = (const ViewTable*)(base + s->layout.table_off);
     const ViewTable* host = (const ViewTable*)s->h_table;
-    const int nv = (int)s->batch.size(), sms = device_sm_count();
+    const int nv = (int)s->batch.size();
     const int bands = nv == 1 && n_tiles >= kBands * kPartTiles ? kBands : 1;
     struct Copy {
         uint8_t* to;
@@ -345,7 +345,7 @@ cudaError_t composite_and_copy(LumenServer* srv, Slot* s, const LaunchConfig& lc
     long long first = 0;
     for (size_t i = 0; i < part_tiles.size() && e == cudaSuccess; ++i) {
         launch_composite(vt, nv, s->frame, ctrl, srv->cfg.options, first, part_tiles[i], !split, lc.composite_chunk,
-                         lc.track != 0, sms, s->stream);
+                         lc.track != 0, s->stream);
         first += part_tiles[i];
         if (split) e = cudaEventRecord(s->ev_parts[i], s->stream);
     }
