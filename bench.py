@@ -40,8 +40,12 @@ UNIT = "frames/s"
 N_GAUSSIANS = 1_000_000
 WIDTH, HEIGHT = 1920, 1080
 # DRAM bytes (read + write) of one composite_kernel launch at the 1 M-Gaussian
-# 1080p workload, from an ncu capture (profiles/forward_config1_kernels.md)
+# 1080p workload, from an ncu capture
 COMPOSITE_DRAM_BYTES = 51.7e6
+
+STAGES = ["project", "sort", "lists", "composite"]
+
+
 def cells_of(width: int, height: int) -> int:
     """Cells of 4x4 tiles (64x64 pixels) of a view."""
     return ((width + 63) // 64) * ((height + 63) // 64)
@@ -54,9 +58,34 @@ def kernels_per_frame(slots: int, cells: int, views: int = 1) -> int:
     digit passes); the emission (which also counts the cell sort's digits); one
     cell-sort digit pass per byte a cell id can vary in, or one nine-bit pass
     for 257 to 512 cells; the lists' count, scan and write; composite."""
-    cell_passes = 1 if 256 < cells <= 512 else ((cells - 1).bit_length() + 7) // 8
     small = slots <= 131072
-    return 1 + (1 if small and views == 1 else 3) + (1 if small else 5) + 1 + cell_passes + 3 + 1
+    return 1 + (1 if small and views == 1 else 3) + (1 if small else 5) + 1 + cell_passes(cells) + 3 + 1
+
+
+def cell_passes(cells: int) -> int:
+    return 1 if 256 < cells <= 512 else ((cells - 1).bit_length() + 7) // 8
+
+
+def cell_pairs(rects) -> int:
+    """(cell, splat) pairs of visible splats' tile rectangles."""
+    f = [(rects >> s) & 0xFFF for s in (0, 12, 24, 36)]
+    return int((((f[2] >> 2) - (f[0] >> 2) + 1) * ((f[3] >> 2) - (f[1] >> 2) + 1)).sum())
+
+
+def forward_bytes(n: int, V: int, K: int, pairs: int, depth_passes: int, passes: int, T: int, P: int, one_view_small=False):
+    """What each stage of a forward pass has to move between its kernels: per
+    Gaussian its parameters (236 B; the visibility count reads 44 B of them
+    once more, unless one kernel projects) and radius; per visible splat its
+    record, index, rectangle, depth key and order; per executed depth pass key
+    and order in and out, and one read by the histogram; per pair 8 B out of
+    the emission, in and out of every executed pass over the cells (`passes`),
+    and its key into the lists' count and both words into their write; per
+    instance its tile and splat out; per instance in the compositor its splat
+    and the 36 B of its record that are used."""
+    return {"project": (236 if one_view_small else 280) * n + 4 * n + 68 * V,
+            "sort": 4 * V + 16 * V * depth_passes + 12 * V + 8 * pairs + 16 * pairs * passes,
+            "lists": 12 * pairs + 8 * K + 16 * T,
+            "composite": 40 * K + 16 * P}
 
 
 def parse():
@@ -353,7 +382,8 @@ def fwd_bwd_leg(dev, steps, warmup, hbm_peak):
                       cam, opt).rgb.contiguous()
     first = R.render(*params, cam, opt)
     V, K, T, P = first.n_visible, first.n_instances, cam.n_tiles, WIDTH * HEIGHT
-    passes = bin(first.varying_digits & 0xFFFF).count("1")
+    b_stage = forward_bytes(n, V, K, cell_pairs(first.frame.rects[:V]), bin(first.varying_digits >> 8 & 0xFF).count("1"),
+                            cell_passes(cells_of(WIDTH, HEIGHT)), T, P)
     lib = L.load()
     g = R.gaussians_struct(*params)
     ccam, copt = L.view_camera(cam), L.render_options(opt)
@@ -431,16 +461,15 @@ def fwd_bwd_leg(dev, steps, warmup, hbm_peak):
         A.l1_loss(r, target).backward()
     torch.cuda.synchronize(dev)
     api_ms = (time.perf_counter() - t0) * 1e3 / ta_steps
-    b_fwd = 244 * n + 64 * V + (60 + 24 * passes) * K + 16 * T + 16 * P
+    b_fwd = sum(b_stage.values())
     b_bwd = 80 * K + 12 * P + 88 * V + 472 * n
     total = b_fwd + 24 * P + b_bwd
-    stages = {"project": fst[0] / reps, "sort": fst[1] / reps, "tile_ranges": fst[2] / reps,
-              "composite": fst[3] / reps, "composite_backward": bst[0] / reps, "project_backward": bst[1] / reps}
+    stages = {**{k: v / reps for k, v in zip(STAGES, fst)}, "composite_backward": bst[0] / reps, "project_backward": bst[1] / reps}
     return {"workload": "config 3: 500k Gaussians, 1920x1080, L1 to the perturbed-scene render",
             "steps_per_s": 1000.0 / ms, "ms_per_step": ms, "backward_ms": bwd_ms,
             "stages_ms": {k: round(v, 4) for k, v in stages.items()},
             "stages_timing": "a second, event-instrumented run of the forward and of the backward",
-            "sizes": {"n": n, "visible": V, "instances": K, "pixels": P, "tiles": T, "digit_passes": passes},
+            "sizes": {"n": n, "visible": V, "instances": K, "pixels": P, "tiles": T}, "stage_bytes": b_stage,
             "autograd_api_steps_per_s": 1000.0 / api_ms, "visible": V, "instances": K,
             "roofline": {"bytes": total, "achieved": total / (ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                          "frac": total / (ms * 1e-3) / 1e9 / hbm_peak}}
@@ -681,17 +710,16 @@ def multiview_leg(dev, steps, warmup, hbm_peak):
     V, K = first.n_visible, first.n_instances
     T = sum(c.n_tiles for c in cams)
     P = n_views * W * H
-    tile_bits = max(T - 1, 1).bit_length()
     depth_keys = [r.varying_digits >> 8 for r in singles]
-    depth_bytes = bin(int(np.bitwise_or.reduce(np.array(depth_keys))) & 0xFF).count("1")
-    p = (tile_bits + 7) // 8 + depth_bytes
-    b = 236 * n + 8 * n * n_views + 64 * V + (60 + 24 * p) * K + 16 * T + 16 * P
+    depth_passes = bin(int(np.bitwise_or.reduce(np.array(depth_keys))) & 0xFF).count("1")
+    p = cell_passes(n_views * cells_of(W, H))
+    b = sum(forward_bytes(n, V, K, cell_pairs(first.frame.frame.rects[:V]), depth_passes, p, T, P).values())
     return {"workload": "config 2: 300k Gaussians, 64 orbit views at 1280x720, one batch per step",
             "views_per_s": n_views * 1000.0 / ms, "ms_per_batch": ms,
             "per_call_views_per_s": n_views * 1000.0 / ms_single, "per_call_ms_for_64": ms_single,
-            "stages_ms": {k: round(v / steps, 4) for k, v in zip(["project", "sort", "tile_ranges", "composite"],
-                                                                 stage)},
-            "visible": V, "instances": K, "tiles": T, "digit_passes": p, "gpu_launches_per_batch": kernels_per_frame(n * n_views, n_views * cells_of(W, H), n_views),
+            "stages_ms": {k: round(v / steps, 4) for k, v in zip(STAGES, stage)},
+            "visible": V, "instances": K, "tiles": T, "digit_passes": p + depth_passes,
+            "gpu_launches_per_batch": kernels_per_frame(n * n_views, n_views * cells_of(W, H), n_views),
             "roofline": {"bytes": b, "achieved": b / (ms * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                          "frac": b / (ms * 1e-3) / 1e9 / hbm_peak}}
 
@@ -789,7 +817,7 @@ def _batch_ceiling(dev, dscene, lib, opt, n_views):
     nfr = C.c_int(0)
     L.check(lib.lumen_gpu_stage_timer_read(timer, stage, C.byref(total), C.byref(nfr)), "timer")
     lib.lumen_gpu_stage_timer_destroy(timer)
-    per_view = {k: v / reps / n_views for k, v in zip(["project", "sort", "tile_ranges", "composite"], stage)}
+    per_view = {k: v / reps / n_views for k, v in zip(STAGES, stage)}
     per_view["total"] = total.value / reps / n_views
     return per_view
 
@@ -913,12 +941,12 @@ def serving_leg(dev, n_requests, hbm_budget):
     # the bound: what a batch of 1080p views of the 1M scene costs per view, by stage, at the
     # server's largest batch of such views (8: 65 280 tiles)
     ceil = _batch_ceiling(dev, dscenes[sizes.index(1_000_000)], lib, opt, 8)
-    per_view_unshared = ceil["sort"] + ceil["tile_ranges"] + ceil["composite"]
+    per_view_unshared = ceil["sort"] + ceil["lists"] + ceil["composite"]
     out["ceiling_1080p_1M"] = {
         "per_view_stage_ms_in_8_view_batch": {k: round(v, 4) for k, v in ceil.items()},
         "frames_per_s_if_projection_were_free": 1000.0 / per_view_unshared,
         "frames_per_s_at_measured_batch_cost": 1000.0 / ceil["total"],
-        "note": "sorts, tile ranges and compositing read and write per-view data; only projection reads the "
+        "note": "sorts, tile lists and compositing read and write per-view data; only projection reads the "
                 "shared scene, so no batching can serve more than frames_per_s_if_projection_were_free"}
     out["workload"] = ("config 4: 8 resident scenes {50k..2M} (6.4M Gaussians), random scene, orbit camera and "
                        "resolution in {640x480, 1280x720, 1920x1080, 3840x2160}; and a 1080p stream of the 1M "
@@ -982,21 +1010,14 @@ def kernels_table(line, hbm_peak, sm_mhz=1965.0):
 
     c = line.get("counts", {})
     st = line.get("stages_ms", {})
-    N, V, K, T, p = N_GAUSSIANS, c.get("visible", 0), c.get("instances", 0), c.get("tiles", 0), c.get("digit_passes", 0)
-    P = WIDTH * HEIGHT
-    if st:
-        add("project", "config 1", st["project"], 236 * N + 48 * V + 4 * N)
-        add("sort", "config 1", st["sort"], 8 * N + 16 * V + 12 * K + 8 * K + 24 * K * p + 8 * T)
-        add("tile_ranges", "config 1", st["tile_ranges"], 8 * T)
-        add("composite", "config 1", st["composite"], 40 * K + 16 * P)
+    for k in STAGES if st else ():
+        add(k, "config 1", st[k], c["stage_bytes"][k])
     fb = line.get("fwd_bwd")
     if fb and "stages_ms" in fb:
         z, s3 = fb["sizes"], fb["stages_ms"]
-        n3, V3, K3, P3, T3, p3 = z["n"], z["visible"], z["instances"], z["pixels"], z["tiles"], z["digit_passes"]
-        add("project", "config 3", s3["project"], 236 * n3 + 48 * V3 + 4 * n3)
-        add("sort", "config 3", s3["sort"], 8 * n3 + 16 * V3 + 12 * K3 + 8 * K3 + 24 * K3 * p3 + 8 * T3)
-        add("tile_ranges", "config 3", s3["tile_ranges"], 8 * T3)
-        add("composite", "config 3", s3["composite"], 40 * K3 + 16 * P3)
+        n3, V3, K3, P3 = z["n"], z["visible"], z["instances"], z["pixels"]
+        for k in STAGES:
+            add(k, "config 3", s3[k], fb["stage_bytes"][k])
         add("composite_backward", "config 3", s3["composite_backward"], 80 * K3 + 12 * P3)
         add("project_backward", "config 3", s3["project_backward"], 88 * V3 + 472 * n3)
     return rows
@@ -1044,9 +1065,8 @@ def main():
     first = R.render(means, sc_t, quats, op_t, sh, cam, opt)
     frame = first.frame
     V, K, T = first.n_visible, first.n_instances, cam.n_tiles
-    # bytes of the reference's 64-bit key that vary: tile-id bytes (low 8 bits of the mask,
-    # key bytes 4..7) and depth-key bytes (next 8 bits, key bytes 0..3)
-    passes = bin(first.varying_digits & 0xFFFF).count("1")
+    depth_passes, passes = bin(first.varying_digits >> 8 & 0xFF).count("1"), cell_passes(cells_of(WIDTH, HEIGHT))
+    pairs = cell_pairs(frame.rects[:V])
     lib = L.load()
     g = R.gaussians_struct(means, sc_t, quats, op_t, sh)
     ccam, copt = L.view_camera(cam), L.render_options(opt)
@@ -1099,22 +1119,14 @@ def main():
     ms_max, value = replica_throughput(ms, world, pg, dev)
 
     stage_ms = [x / steps for x in stage]
-    names = ["project", "sort", "tile_ranges", "composite"]
-    # algorithmic bytes per launch; p = digit passes of the
-    # reference's 64-bit key sort that vary (its 8-pass sort with constant digits skipped)
-    P = WIDTH * HEIGHT
-    p = passes
-    alg = {"project": 236 * N_GAUSSIANS + 48 * V + 4 * N_GAUSSIANS,
-           "sort": 8 * N_GAUSSIANS + 16 * V + 12 * K + 8 * K + 24 * K * p + 8 * T,
-           "tile_ranges": 8 * T,
-           "composite": 40 * K + 16 * P}
-    # the dominant kernel: composite_kernel, the largest share of the frame's
-    # launch list (profiles/forward_config1_launches.md); the sort stage is
-    # seven kernels, none above a tenth of the frame
+    names = STAGES
+    alg = forward_bytes(N_GAUSSIANS, V, K, pairs, depth_passes, passes, T, WIDTH * HEIGHT)
+    # the dominant kernel: composite_kernel, the largest share of the frame; the
+    # sort stage is seven kernels, none above a tenth of the frame
     dom = names.index("composite")
     dname = names[dom]
     achieved = alg[dname] / (stage_ms[dom] * 1e-3) / 1e9
-    b_fwd = 244 * N_GAUSSIANS + 64 * V + (60 + 24 * passes) * K + 16 * T + 16 * P
+    b_fwd = sum(alg.values())
     frame_gbs = b_fwd / (ms_max * 1e-3) / 1e9
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": steps, "warmup": args.warmup,
@@ -1125,12 +1137,13 @@ def main():
             "clocks": clk.summary(),
             "stages_ms": {n: round(v, 4) for n, v in zip(names, stage_ms)},
             "stages_timing": "a second run of the K frames with CUDA events between the stages",
-            "counts": {"visible": V, "instances": K, "tiles": T, "digit_passes": passes},
+            "counts": {"visible": V, "instances": K, "tiles": T, "cell_pairs": pairs, "digit_passes": depth_passes + passes,
+                       "stage_bytes": alg},
             "roofline": {"bound": "hbm", "kernel": dname, "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                          "frac": achieved / hbm_peak, "traffic": COMPOSITE_DRAM_BYTES, "peak_source": peak_src,
                          "algorithmic_bytes": alg[dname],
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one composite_kernel "
-                                           "launch at this workload (profiles/forward_config1_kernels.md)"},
+                                           "launch at this workload"},
             "frame_roofline": {"bytes": b_fwd, "achieved": frame_gbs, "peak": hbm_peak, "unit": "GB/s",
                                "frac": frame_gbs / hbm_peak}}
     if not args.no_multiview:
