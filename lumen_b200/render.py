@@ -26,9 +26,12 @@ def _p(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)   # not part of torch's public interface
+
+
 def _stream_handle(device: torch.device) -> int:
-    if device.type == "cuda" and device.index is not None:
-        return torch._C._cuda_getCurrentRawStream(device.index)   # no Stream object is made
+    if _raw_stream is not None and device.type == "cuda" and device.index is not None:
+        return _raw_stream(device.index)   # no Stream object is made
     return torch.cuda.current_stream(device).cuda_stream
 
 
