@@ -158,7 +158,8 @@ __device__ __forceinline__ bool has_order(const Room& room, const ViewTable* vt)
 /* The work items of the count: a cell, or (from n_cells on) a window of
  * sorted pairs that lies in a long cell which starts before it. Part 0 of a
  * cell is the cell's item; part k the window k after the one that the cell starts
- * in. total: per item and tile, the part's instances. */
+ * in. total: per item and tile, the part's instances. Without more pairs than a
+ * long cell has, there are no windows and no totals. */
 struct SegmentRoom {
     unsigned int (*total)[kCellTiles];
     Segment* p;
@@ -166,12 +167,13 @@ struct SegmentRoom {
 };
 
 __device__ __forceinline__ long long count_items(const ViewTable* vt, int n_pairs) {
-    return vt->hdr.total_cells + (n_pairs + kWindow - 1) / kWindow;
+    return vt->hdr.total_cells + (n_pairs > kLongCell ? (n_pairs + kWindow - 1) / kWindow : 0);
 }
 
 __device__ __forceinline__ SegmentRoom segment_room(const Room& room, const ViewTable* vt, int n_pairs) {
     const long long order = has_order(room, vt) ? (vt->hdr.total_tiles * 4 + 15) / 16 * 16 : 0;
-    const long long totals = count_items(vt, n_pairs) * (long long)sizeof(unsigned int[kCellTiles]);
+    const long long totals =
+        n_pairs > kLongCell ? count_items(vt, n_pairs) * (long long)sizeof(unsigned int[kCellTiles]) : 0;
     return {reinterpret_cast<unsigned int(*)[kCellTiles]>(room.p + order),
             reinterpret_cast<Segment*>(room.p + order + totals),
             max(room.bytes - order - totals, 0ll) / (long long)sizeof(Segment)};
