@@ -11,7 +11,8 @@
  *    batch while the batch fits a slot's work buffers (projection slots,
  *    tiles, an instance estimate learned per scene and resolution, output
  *    pixels) and max_views_per_batch, and while its tiles number at most
- *    65 536 (unless one view alone has more);
+ *    65 536 (unless one view alone has more; larger batches serve a burst a
+ *    little faster, but every image waits for its batch);
  *  - up to max_batches_in_flight batches are on the device at once, each on
  *    its own stream with its own buffers, so a batch admitted while others
  *    run overlaps with them; a slot is reused as soon as its batch is done;

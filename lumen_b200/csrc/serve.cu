@@ -62,15 +62,19 @@ int variant_of(int chunk, int items) {
 }
 
 /* Tiles a batch holds unless one view alone has more: eight 1080p views. Views
- * share the projection's reads and the launches, and eight of them fill the
- * GPU; with up to sixteen a burst of 64 views of 1 M Gaussians took 16.3 ms
- * against 15.2 to 17.9, and the first images wait longer. */
-constexpr int64_t kBatchTileIds = 1ll << 16;
+ * share the projection's reads and the launches, so larger batches end a burst
+ * sooner, but an image waits for its whole batch. 64 views of 1 M Gaussians at
+ * 1080p in batches of up to 4, 8, 16 and 22 views (2^15, 2^16, 2^17 and 2^20
+ * tiles): all after 18.4, 17.6, 17.1 and 17.0 ms, on average after 9.9, 10.5,
+ * 11.8 and 12.6; 64 of 300 k at 720p: 7.6, 7.1, 6.5 and 7.3 ms, 4.4, 4.7, 5.3 and
+ * 6.2. */
+constexpr int64_t kBatchTiles = 1ll << 16;
 
 /* The least tiles of a part of a batch (composite_and_copy), about a wave, and
  * the bands of rows of a view that is alone in its batch. */
 constexpr long long kPartTiles = 1024;
 constexpr int kBands = 4;
+constexpr int kMaxParts = (int)(kBatchTiles / kPartTiles) + kBands;
 
 constexpr size_t kControlHead = offsetof(Control, proj_ticket);   /* the counters that the host reads back */
 
@@ -250,7 +254,7 @@ cudaError_t alloc_slot(LumenServer* srv, Slot* s) {
     if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess) return e;
     if ((e = cudaStreamCreateWithFlags(&s->copies, cudaStreamNonBlocking)) != cudaSuccess) return e;
     if ((e = cudaEventCreateWithFlags(&s->ev_copied, cudaEventDisableTiming)) != cudaSuccess) return e;
-    for (int i = 0; i < std::max<int>(srv->cfg.max_views_per_batch, kBands); ++i) {
+    for (int i = 0; i < kMaxParts; ++i) {
         cudaEvent_t ev;
         if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return e;
         s->ev_parts.push_back(ev);
@@ -469,9 +473,9 @@ void scheduler_main(LumenServer* srv) {
             sl[i] = r.slots; ti[i] = r.tiles; in[i] = r.inst_est; px[i] = r.pixels;
         }
         int k = admit_prefix(sl.data(), ti.data(), in.data(), px.data(), n, srv->cfg.max_views_per_batch,
-                             srv->max_slots, std::min<int64_t>(srv->max_tiles, kBatchTileIds), srv->max_inst,
+                             srv->max_slots, std::min<int64_t>(srv->max_tiles, kBatchTiles), srv->max_inst,
                              srv->max_pix);
-        if (k == 0 && ti[0] > kBatchTileIds)   /* a view of more tiles than that goes alone */
+        if (k == 0 && ti[0] > kBatchTiles)   /* a view of more tiles than that goes alone */
             k = admit_prefix(sl.data(), ti.data(), in.data(), px.data(), 1, 1, srv->max_slots, srv->max_tiles,
                              srv->max_inst, srv->max_pix);
         if (k == 0) {

@@ -30,3 +30,15 @@ def test_images_of_a_split_batch(sizes):
             assert alone.result(timeout_ms=60_000).status == 0 and max(r.batch_views for r in res) > 1
             for r, c in zip(res, cams):
                 assert r.status == 0 and torch.equal(r.image, alone_u8(ds, c))
+
+
+def test_a_server_for_many_views_per_batch():
+    """One event per part a batch can have, not per view."""
+    from lumen_b200 import serve
+    ds = device_scene(scenes.box_scene(500, seed=18))
+    cam = ViewCamera.from_fov(65, 33, 50.0)
+    with serve.Server(work_budget_bytes=1 << 30, max_views_per_batch=65535, autotune=False) as srv:
+        sid = srv.add_scene(ds)
+        for h in [srv.submit(sid, cam) for _ in range(300)]:
+            r = h.result(timeout_ms=60_000)
+            assert r.status == 0 and torch.equal(r.image, alone_u8(ds, cam))
