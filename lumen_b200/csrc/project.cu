@@ -796,14 +796,15 @@ static int resident_ctas(const void* kernel, int threads, size_t smem) {
     return per_sm;
 }
 
-static int g_emit_per_sm = 0, g_batch_count_per_sm = 0, g_batch_project_per_sm = 0;
+static int g_emit_per_sm[2] = {0, 0}, g_batch_count_per_sm = 0, g_batch_project_per_sm = 0;   /* emit: one and four rounds */
 constexpr size_t kProjStageBytes = (size_t)kProjThreads * 48 * sizeof(float);
 
 /* Kernel attributes and the occupancy of the persistent kernels, set and
  * queried once (before any capture). */
 void prime_persistent_launches() {
     cudaFuncSetAttribute(project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kProjStageBytes);
-    g_emit_per_sm = resident_ctas((const void*)emit_kernel<1>, kEmitThreads, 0);
+    g_emit_per_sm[0] = resident_ctas((const void*)emit_kernel<1>, kEmitThreads, 0);
+    g_emit_per_sm[1] = resident_ctas((const void*)emit_kernel<kEmitMaxRounds>, kEmitThreads, 0);
     cudaFuncSetAttribute(batch_project_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kProjStageBytes);
     cudaFuncSetAttribute(batch_project_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -851,8 +852,9 @@ void launch_emit(const ViewTable* vt, const LumenGpuFrame& f, Control* ctrl, uns
                  unsigned int* sort_lb, long long sort_lb_tiles, int sort_tile_keys, bool wide, long long n_blocks,
                  bool persistent, int num_sms, cudaStream_t st) {
     if (n_blocks <= 0) return;
-    const long long resident = (long long)(g_emit_per_sm > 0 ? g_emit_per_sm : 1) * num_sms;
     auto run = [&](auto kernel, int rounds) {
+        const int per_sm = g_emit_per_sm[rounds > 1];
+        const long long resident = (long long)(per_sm > 0 ? per_sm : 1) * num_sms;
         const long long blocks = (n_blocks * kProjThreads + rounds * kEmitThreads - 1) / (rounds * kEmitThreads);
         launch_chained(kernel, dim3((unsigned int)(persistent || blocks > resident ? resident : blocks)),
                        dim3(kEmitThreads), 0, st, vt, f, ctrl, lb, sort_lb, sort_lb_tiles, sort_tile_keys, wide);
