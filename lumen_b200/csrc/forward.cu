@@ -5,15 +5,19 @@
  *
  * Launch sequence of a frame (all on the caller's stream, no host sync):
  *   frame_init         control block and look-back descriptors zeroed, view table
+ *   project            K1, for one view of up to 131072 Gaussians: projection, cull, SH,
+ *                      records and depth keys; otherwise
  *   batch_count        K1a: each block's visible count (geometry only)
  *   batch_offsets      K1b: the counts scanned into each block's first visible index
  *   batch_project      K1c: projection, cull, SH, records and depth keys at those offsets
+ *   cluster_sort       stable sort of up to 131072 splats by depth key; otherwise
  *   histogram<u32>     depth-key digits of the visible splats
  *   onesweep_pass x4   stable sort of visible splats by depth key
  *   emit               K2: (cell and tile mask, visible index) per touched cell of 4x4
  *                      tiles, in depth order; also the cell sort's digit counts and
  *                      look-back tiles
- *   onesweep_pass xb   stable sort of the pairs by cell (b: the bytes a cell id can vary in)
+ *   onesweep_pass xb   stable sort of the pairs by cell (b: the digits of a cell id
+ *                      (CellDigits), or one of nine bits for 257 to 512 cells)
  *   list_count, list_scan, list_write   K4: each cell's list split over its tiles: counts,
  *                      ranges with touched tiles and each view's first instance, lists
  *   composite          K5
@@ -175,7 +179,9 @@ __global__ void frame_init_kernel(unsigned long long* zero, long long n_words, V
  * kernel. Projection, one kernel and three: 512 Gaussians 13.3 and 19.9 us
  * (and two launches fewer to issue), 50 k 20.8 and 22.2, 100 k 13.5 and 18.4
  * (without the launch before); 250 k 43 and 39.6, where the look-back is the
- * longer way. */
+ * longer way. Whole frames on both sides of the line, where the depth sort
+ * changes its form as well: 131072 Gaussians 182, 198 and 248 us at 640x480,
+ * 1279x719 and 1080p, 131073 192, 214 and 250. */
 constexpr long long kOnePassBlocks = 1024;
 
 /* The frame's kernels after the view table is in place. n_slots, n_tiles and
@@ -351,7 +357,7 @@ LumenStatus forward_banded(const LumenGpuGaussians* g, const LumenViewCamera* ca
     return map_cuda(cudaGetLastError());
 }
 
-/* Offsets of a batch's views: blocks (256 Gaussians each) and tiles. */
+/* Offsets of a batch's views: blocks (kProjThreads Gaussians each), tiles and cells. */
 static LumenStatus plan_batch(const LumenGpuBatchView* views, int n_views, const LumenRenderOptions* opt,
                               std::vector<ViewDesc>* out, BatchHeader* hdr) {
     if (!views || n_views <= 0 || n_views > kMaxViews) return LUMEN_ERROR_INVALID_ARGUMENT;

@@ -7,7 +7,7 @@
  * B200 design (onesweep, Adinets & Merrill 2022), for 32- or 64-bit keys:
  *  - one histogram pass reads the keys once and counts every digit that
  *    varies (the frame's cell sort needs none: the emission that writes the
- *    cell ids counts them). A digit is constant when no two keys differ in
+ *    pairs counts their digits). A digit is constant when no two keys differ in
  *    that byte (the OR of all keys and the OR of all complemented keys,
  *    gathered by the kernel that produced them, tell which); a pass over a
  *    constant digit leaves a stable sort unchanged, so it is skipped on the
@@ -44,9 +44,9 @@ __device__ __forceinline__ long long sort_count(const SortControl* c, long long 
  *
  * Each thread counts runs of kRun consecutive keys: equal digits in a row
  * are summed in a register and added to the warp's shared histogram once
- * per run. Tile ids in emission order form long runs in their high byte
- * (the instances of one splat row), so those collapse to a few atomics;
- * random digits cost one shared atomic per key, with no warp-wide match. */
+ * per run: keys that come in runs (sorted before, or equal in a high byte)
+ * cost a few atomics, random digits one shared atomic per key, with no
+ * warp-wide match. */
 template <typename KeyT>
 __global__ void __launch_bounds__(256)
 histogram_kernel(const KeyT* __restrict__ keys, long long capacity, SortControl* sc, unsigned int* lb,
