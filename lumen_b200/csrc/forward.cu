@@ -216,7 +216,10 @@ void launch_pipeline(const ScratchLayout& L, unsigned char* base, const LumenRen
                       s);
         /* 257 to 512 cells (1080p has 510): one pass over nine bits instead of
          * two over eight and one. 1 M splats at 1080p: the emission and both
-         * passes 87 us, with one pass 74. A persistent launch knows only a
+         * passes 87 us, with one pass 74. Frames of 2 k, 50 k, 250 k and 1 M
+         * splats with two passes and with one: 260 cells 77.2, 115.0, 208 and
+         * 332.8 -> 72.7, 108.1, 196 and 332.2 us, 512 cells 87.2, 129.2, 236 and
+         * 368.7 -> 83.1, 123.4, 230 and 364. A persistent launch knows only a
          * bound of the cells. */
         const bool wide = !persistent && n_cells > 256 && n_cells <= kWideCells;
         launch_emit(vt, f, ctrl, emit_lb, cell_lb, 2 * L.sort_tiles,
@@ -257,12 +260,16 @@ void launch_init(const ScratchLayout& L, unsigned char* base, const BatchHeader*
  * smaller tiles where tiles of 4096 keys would leave SMs idle. The depth sort,
  * up to three of those per SM: 250 k splats 227 -> 220 us per frame, 1 M 392.4
  * -> 390.8, 2 M (beyond) 731.5 -> 732. The cell sort, whose pairs the host does
- * not know, up to the slots of a one-kernel projection: 50 k splats 96.2 ->
- * 93.4, 250 k (beyond) 220 -> 222. */
+ * not know (about two per splat), up to kSmallCellSortSlots: at 640x480 and 4K
+ * 2 k splats 60.4 and 157.4 -> 57.1 and 155.2, 130 k 135 and 385 -> 131.5 and
+ * 381, 200 k 152.8 and 443.7 -> 151.5 and 440.7; 500 k 214.5 and 554.5 -> 215.4
+ * and 558, 250 k at 1279x719 220 -> 222. */
+constexpr long long kSmallCellSortSlots = 200 * 1024;
+
 static LaunchConfig default_launch(long long n_slots) {
     LaunchConfig lc = kDefaultLaunch;
     if (n_slots <= 3ll * device_sm_count() * kSortTile) lc.depth_sort_items = 8;
-    if (n_slots <= kOnePassBlocks * kProjThreads) lc.tile_sort_items = 8;
+    if (n_slots <= kSmallCellSortSlots) lc.tile_sort_items = 8;
     return lc;
 }
 
